@@ -38,8 +38,8 @@ struct qs_register {
     // differ from zval is an exact zero, so later measurements visit only the live subspace.
     uint64_t zmask = 0;
     uint64_t zval = 0;
-    // Scratch of the compact measurement sequences (half the state), allocated by the first one and
-    // kept until the register is destroyed.
+    // Scratch of the compact measurement sequences and of the squares of reference-order sums (half
+    // the state), allocated by the first one and kept until the register is destroyed.
     void* mscratch = nullptr;
 };
 
@@ -208,6 +208,21 @@ bool exact_quotient(const qs_register* reg) { return reg->prec == QS_PREC_C128 &
 
 bool sequential_sums(const qs_register* reg) {
     return reg->prec == QS_PREC_C128 && reg->arith == QS_ARITH_EXACT && reg->n <= kSequentialMaxQubits;
+}
+
+// The register's half-state scratch, null when it cannot be had.
+void* measure_scratch(qs_register* reg) {
+    if (!reg->mscratch && cudaMalloc(&reg->mscratch, (size_t(1) << (reg->n - 1)) * amp_bytes(reg->prec)) != cudaSuccess) {
+        cudaGetLastError();
+        reg->mscratch = nullptr;
+    }
+    return reg->mscratch;
+}
+
+// Room for the squares of reference-order sums: registers that the one-block kernel serves as well
+// (13 qubits and fewer) do without it.
+double* seq_squares(qs_register* reg) {
+    return sequential_sums(reg) && reg->n > 13 ? static_cast<double*>(measure_scratch(reg)) : nullptr;
 }
 
 void record_outcome(qs_register* reg, size_t target, int res) {
@@ -387,7 +402,8 @@ int qs_try_measure(qs_register* reg, size_t target, double draw, int* outcome, d
         return set_err(QS_INVALID_TARGET, "InvalidTarget(" + std::to_string(target) + ")");
     }
     QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(target), reg->partials, kMaxPartials,
-                                     reg->dres, reg->stream, reg->sms, reg->zmask, reg->zval, sequential_sums(reg)),
+                                     reg->dres, reg->stream, reg->sms, reg->zmask, reg->zval, sequential_sums(reg),
+                                     seq_squares(reg)),
             "measure_probs");
     QS_CUDA(cudaMemcpyAsync(reg->hres, reg->dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, reg->stream),
             "measure readback");
@@ -427,12 +443,8 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
                              double* prob0s, double* prob1s) {
     const int n = reg->n;
     const size_t amp = amp_bytes(reg->prec);
-    if (!reg->mscratch && cudaMalloc(&reg->mscratch, (size_t(1) << (n - 1)) * amp) != cudaSuccess) {
-        cudaGetLastError();
-        reg->mscratch = nullptr;
-        return 1;
-    }
-    void* scratch = reg->mscratch;
+    void* scratch = measure_scratch(reg);
+    if (!scratch) return 1;
     const bool exactq = exact_quotient(reg);
     QS_CUDA(qs::launch_measure_probs(reg->state, n, reg->prec, int(targets[0]), reg->partials, kMaxPartials,
                                      reg->dres, reg->stream, reg->sms),
@@ -517,7 +529,7 @@ int qs_measure_sequence(qs_register* reg, const size_t* targets, size_t m, const
         if (rc != 1) return rc;
     }
     QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(targets[0]), reg->partials, kMaxPartials,
-                                     reg->dres, reg->stream, reg->sms, reg->zmask, reg->zval, seq),
+                                     reg->dres, reg->stream, reg->sms, reg->zmask, reg->zval, seq, seq_squares(reg)),
             "measure_probs");
     for (size_t k = 0; k < m; k++) {
         QS_CUDA(cudaMemcpyAsync(reg->hres, reg->dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, reg->stream),
@@ -543,7 +555,7 @@ int qs_measure_sequence(qs_register* reg, const size_t* targets, size_t m, const
             if (k + 1 < m)
                 QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(targets[k + 1]), reg->partials,
                                                  kMaxPartials, reg->dres, reg->stream, reg->sms, reg->zmask,
-                                                 reg->zval, seq),
+                                                 reg->zval, seq, seq_squares(reg)),
                         "measure_probs");
         }
         outcomes[k] = res;

@@ -71,10 +71,11 @@ cudaError_t launch_init_basis(void* state, int n, int prec, uint64_t index, cuda
 cudaError_t launch_init_product(void* state, int n, int prec, const double* qubits, cudaStream_t s, int sms);
 // FP64 probability sums of target bit 0 / 1 into out[0], out[1] (device), via per-block partials,
 // over the live subspace (amplitudes whose zmask bits equal zval; the others must be zero).
-// sequential (complex128 only): one block adds the squares in index order, as the reference does.
+// sequential (complex128 only): the sums are those of adding the squares in index order, as the
+// reference does; `squares` (null, or room for one double per amplitude) lets the whole chip do it.
 cudaError_t launch_measure_probs(const void* state, int n, int prec, int target, double* partials,
                                  int max_partials, double* out, cudaStream_t s, int sms, uint64_t zmask = 0,
-                                 uint64_t zval = 0, bool sequential = false);
+                                 uint64_t zval = 0, bool sequential = false, double* squares = nullptr);
 // Zero amplitudes whose target bit != outcome and divide the rest by d (rinv = 1/d), within the
 // live subspace: complex128 with exact_quotient as the correctly rounded quotient (Rust's `/`),
 // otherwise within one ulp of it (a multiply by rinv).

@@ -207,55 +207,307 @@ __global__ void __launch_bounds__(kT) k_prob_final(const double* __restrict__ pa
 }
 
 // The probability sums in the reference's order (src/register.rs:306-315): norm_sqr = re*re + im*im
-// rounded per operation, added to prob_0 or prob_1 one amplitude after another in index order. One
-// block stages chunks of amplitudes in shared memory; the bit-0 and bit-1 chains are independent
-// sums and run on two threads. Amplitudes outside the live subspace are exact zeros, which leave a
-// running sum unchanged, so only the subspace is read.
-constexpr int kSeqChunk = 2048;
-__global__ void __launch_bounds__(kT) k_prob_sequential(const double2* __restrict__ st, uint64_t count, int target,
-                                                        const __grid_constant__ IndexMap map,
-                                                        double* __restrict__ out) {
-    __shared__ double pr[kSeqChunk];
-    __shared__ uint8_t bit[kSeqChunk];
-    double acc = 0.0;  // thread 0: prob_0, thread 32: prob_1
-    for (uint64_t base = 0; base < count; base += kSeqChunk) {
-        const int len = int(count - base < uint64_t(kSeqChunk) ? count - base : uint64_t(kSeqChunk));
-        for (int j = threadIdx.x; j < len; j += kT) {
-            const uint64_t i = expand_index(base + uint64_t(j), map);
-            const double2 a = st[i];
-            pr[j] = __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y));
-            bit[j] = uint8_t((i >> target) & 1ull);
+// rounded per operation, added to prob_0 or prob_1 one amplitude after another in index order, so
+// acc = RN(acc + t) for every t of a chain (the squares with target bit 0, or 1). Taken literally
+// that is a chain of FP64 additions, and sm_103a needs 64 cycles for each (8.6 ms for 2^18 squares).
+// The same values come from integers: while acc stays in one binade, with ulp u, acc = A u for an
+// integer A and RN(acc + t) = (A + d) u, where d is t / u rounded to nearest, ties to the even A + d.
+// Only a tie looks at A, and only at its parity, so a run of squares is a pair of integers (what it
+// adds to an even and to an odd A), and runs compose associatively. Because the squares are not
+// negative, a run is right whenever it ends at A <= 2^53, the end of the binade; the one square that
+// crosses it is added in FP64, and the next run starts in the next binade.
+struct SeqRun {
+    long long d0, d1;  // added to an even / odd A
+};
+
+constexpr long long kSeqTop = 1ll << 53;
+constexpr long long kSeqHuge = 1ll << 55;  // a run that cannot end in the binade (saturated)
+
+__device__ __forceinline__ SeqRun seq_compose(SeqRun a, SeqRun b) {  // a, then b
+    SeqRun r;
+    r.d0 = a.d0 + ((a.d0 & 1) ? b.d1 : b.d0);
+    r.d1 = a.d1 + ((a.d1 & 1) ? b.d0 : b.d1);
+    if (r.d0 > kSeqHuge) r.d0 = kSeqHuge;
+    if (r.d1 > kSeqHuge) r.d1 = kSeqHuge;
+    return r;
+}
+
+// One square t >= 0 (or an infinity or NaN: huge) against a binade with exponent field e >= 1.
+__device__ __forceinline__ SeqRun seq_square(double t, int e) {
+    const long long bits = __double_as_longlong(t);
+    const int et = int(bits >> 52) & 0x7ff;
+    long long m = bits & 0xfffffffffffffll;
+    if (et) m |= 1ll << 52;
+    const int sh = e - (et ? et : 1);
+    SeqRun r;
+    if (sh < 0 || et == 0x7ff) {  // above the binade
+        r.d0 = r.d1 = m ? kSeqHuge : 0;
+        return r;
+    }
+    if (sh > 53) {  // below half an ulp
+        r.d0 = r.d1 = 0;
+        return r;
+    }
+    const long long q = m >> sh, rem = m - (q << sh), half = sh ? 1ll << (sh - 1) : 1ll;
+    const long long up = q + (rem > half ? 1 : 0);
+    const bool tie = rem == half && sh;
+    r.d0 = up + ((tie && (q & 1)) ? 1 : 0);
+    r.d1 = up + ((tie && !(q & 1)) ? 1 : 0);
+    return r;
+}
+
+// acc's binade as its exponent field, 0 when the integer form does not apply (zero, subnormal,
+// infinite, NaN).
+__device__ __forceinline__ int seq_binade(double acc) {
+    const int e = int(__double_as_longlong(acc) >> 52) & 0x7ff;
+    return e == 0x7ff ? 0 : e;
+}
+__device__ __forceinline__ long long seq_integer(double acc) {
+    return (__double_as_longlong(acc) & 0xfffffffffffffll) | (1ll << 52);
+}
+__device__ __forceinline__ double seq_double(long long A, int e) {  // 2^52 <= A <= 2^53
+    // A = 2^53 carries into the exponent field
+    return __longlong_as_double((static_cast<long long>(e - 1) << 52) + A);
+}
+
+// acc after the squares t[0, len) (shared or global memory), by one warp; every lane returns it. A
+// step takes 32 x kSeqLane squares; the step that leaves the binade keeps its squares up to the
+// crossing one, adds that one in FP64 and continues behind it.
+constexpr int kSeqLane = 8;
+__device__ double seq_warp(double acc, const double* t, int len) {
+    const int lane = threadIdx.x & 31;
+    int at = 0;
+    while (at < len) {
+        const int e = seq_binade(acc);
+        const int first = at + lane * kSeqLane;
+        double v[kSeqLane];
+#pragma unroll
+        for (int j = 0; j < kSeqLane; j++) v[j] = first + j < len ? t[first + j] : 0.0;
+        if (e == 0) {
+            if (!(acc < __longlong_as_double(0x7ffll << 52))) {  // infinite or NaN: only a NaN changes it
+                bool nan = false;
+#pragma unroll
+                for (int j = 0; j < kSeqLane; j++) nan |= v[j] != v[j];
+                if (__ballot_sync(0xffffffffu, nan)) acc = __longlong_as_double(0x7ff8ll << 48);
+                at += 32 * kSeqLane;
+                continue;
+            }
+            int mine = kSeqLane;  // up to the first square that is not zero, which is added in FP64
+#pragma unroll
+            for (int j = kSeqLane - 1; j >= 0; j--)
+                if (v[j] != 0.0) mine = j;
+            const unsigned any = __ballot_sync(0xffffffffu, mine < kSeqLane);
+            if (!any) {
+                at += 32 * kSeqLane;
+                continue;
+            }
+            const int l = __ffs(any) - 1;
+            const int idx = at + l * kSeqLane + __shfl_sync(0xffffffffu, mine, l);
+            acc = __dadd_rn(acc, t[idx]);
+            at = idx + 1;
+            continue;
+        }
+        SeqRun run = seq_square(v[0], e);
+#pragma unroll
+        for (int j = 1; j < kSeqLane; j++) run = seq_compose(run, seq_square(v[j], e));
+        SeqRun incl = run;  // the runs of lanes 0..lane
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            SeqRun p;
+            p.d0 = __shfl_up_sync(0xffffffffu, incl.d0, o);
+            p.d1 = __shfl_up_sync(0xffffffffu, incl.d1, o);
+            if (lane >= o) incl = seq_compose(p, incl);
+        }
+        const long long A = seq_integer(acc);
+        const long long after = A + ((A & 1) ? incl.d1 : incl.d0);
+        const unsigned over = __ballot_sync(0xffffffffu, after > kSeqTop);
+        if (!over) {
+            acc = seq_double(__shfl_sync(0xffffffffu, after, 31), e);
+            at += 32 * kSeqLane;
+            continue;
+        }
+        const int l = __ffs(over) - 1;  // the first lane whose squares leave the binade
+        long long B = __shfl_sync(0xffffffffu, after, l ? l - 1 : 0);
+        if (l == 0) B = A;
+        int cross = kSeqLane;
+        if (lane == l) {
+            cross = 0;
+#pragma unroll
+            for (int j = 0; j < kSeqLane; j++) {
+                const SeqRun q = seq_square(v[j], e);
+                const long long C = B + ((B & 1) ? q.d1 : q.d0);
+                if (cross == j && C <= kSeqTop) {
+                    B = C;
+                    cross = j + 1;
+                }
+            }
+        }
+        cross = __shfl_sync(0xffffffffu, cross, l);
+        B = __shfl_sync(0xffffffffu, B, l);
+        const int idx = at + l * kSeqLane + cross;
+        acc = __dadd_rn(seq_double(B, e), t[idx]);
+        at = idx + 1;
+    }
+    return acc;
+}
+
+// One block for both chains, chunk after chunk of squares in shared memory: what registers of up to
+// 13 qubits take (4096 squares: 5 us against 28 us for the additions one by one), and larger ones
+// when the scratch of the three-kernel form below cannot be had.
+constexpr int kSeqChunk = 2048;  // pairs per chunk
+__global__ void __launch_bounds__(1024) k_prob_seq_block(const double2* __restrict__ st, uint64_t npairs, uint64_t tb,
+                                                         const __grid_constant__ IndexMap map,
+                                                         double* __restrict__ out) {
+    __shared__ double sq[2][kSeqChunk];
+    double acc = 0.0;  // warp 0: prob_0, warp 1: prob_1
+    for (uint64_t base = 0; base < npairs; base += kSeqChunk) {
+        const int len = int(npairs - base < uint64_t(kSeqChunk) ? npairs - base : uint64_t(kSeqChunk));
+        for (int j = threadIdx.x; j < 2 * len; j += blockDim.x) {
+            const int c = j >= len, k = c ? j - len : j;
+            const double2 a = st[expand_index(base + uint64_t(k), map) | (c ? tb : 0ull)];
+            sq[c][k] = __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y));
         }
         __syncthreads();
-        if (threadIdx.x == 0 || threadIdx.x == 32) {
-            const uint8_t want = threadIdx.x == 32 ? 1 : 0;
-            for (int j = 0; j < len; j++)
-                if (bit[j] == want) acc = __dadd_rn(acc, pr[j]);
-        }
+        if (threadIdx.x < 64) acc = seq_warp(acc, sq[threadIdx.x >> 5], len);
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[0] = acc;
-    if (threadIdx.x == 32) out[1] = acc;
+    if (threadIdx.x < 64 && (threadIdx.x & 31) == 0) out[threadIdx.x >> 5] = acc;
 }
+
+// The same on the whole chip, for larger registers: (1) every square, and the sum of every group of
+// kSeqGroup of them; (2) each group's run in the binade that the sums before it predict; (3) one warp
+// per chain composes the groups, 32 at a time, and goes through a group square by square (seq_warp)
+// only where the binade changes or was not the predicted one. A wrong prediction costs time, not
+// the result. 2^18 pairs take 20 us (single SM: its FP64 pipe takes 200 us for the squares alone).
+constexpr int kSeqGroup = 512;
+struct SeqGroup {
+    SeqRun run;
+    long long e;  // the binade's exponent field, 0: none, -1: every square is zero (any acc)
+};
+
+__global__ void __launch_bounds__(kT) k_seq_squares(const double2* __restrict__ st, uint64_t npairs, uint64_t tb,
+                                                    const __grid_constant__ IndexMap map, double* __restrict__ sq,
+                                                    float* __restrict__ sums) {
+    const uint64_t groups = npairs / kSeqGroup;  // per chain
+    const uint64_t w = uint64_t(blockIdx.x) * (kT / 32) + (threadIdx.x >> 5);
+    if (w >= 2 * groups) return;
+    const int lane = threadIdx.x & 31;
+    const bool one = w >= groups;
+    const uint64_t p0 = (one ? w - groups : w) * kSeqGroup;
+    float s = 0.0f;
+    bool any = false;
+#pragma unroll 4
+    for (int j = lane; j < kSeqGroup; j += 32) {
+        const double2 a = st[expand_index(p0 + uint64_t(j), map) | (one ? tb : 0ull)];
+        const double v = __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y));
+        sq[w * kSeqGroup + j] = v;
+        s += float(v);
+        any |= v != 0.0;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    any = __ballot_sync(0xffffffffu, any) != 0u;
+    if (lane == 0) sums[w] = any ? s : -0.0f;  // -0: a group of zeros
+}
+
+__global__ void __launch_bounds__(kT) k_seq_groups(const double* __restrict__ sq, uint64_t groups,
+                                                   const float* __restrict__ sums, SeqGroup* __restrict__ out) {
+    const uint64_t w = uint64_t(blockIdx.x) * (kT / 32) + (threadIdx.x >> 5);
+    if (w >= 2 * groups) return;
+    const int lane = threadIdx.x & 31;
+    if (__float_as_uint(sums[w]) == 0x80000000u) {
+        if (lane == 0) out[w] = SeqGroup{{0, 0}, -1};
+        return;
+    }
+    float s = 0.0f;  // the sum of the chain before this group
+    for (uint64_t g = (w >= groups ? groups : 0) + lane; g < w; g += 32) s += sums[g];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    const uint32_t fe = (__float_as_uint(s) >> 23) & 0xffu;
+    const int e = (fe == 0u || fe == 255u) ? 0 : int(fe) + 896;
+    SeqRun run{0, 0};
+    if (e) {
+        constexpr int per = kSeqGroup / 32;
+        const double2* t = reinterpret_cast<const double2*>(sq + w * kSeqGroup + lane * per);
+#pragma unroll
+        for (int j = 0; j < per / 2; j++) {
+            const double2 v = t[j];
+            run = seq_compose(run, seq_compose(seq_square(v.x, e), seq_square(v.y, e)));
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            SeqRun p;
+            p.d0 = __shfl_down_sync(0xffffffffu, run.d0, o);
+            p.d1 = __shfl_down_sync(0xffffffffu, run.d1, o);
+            if (lane + o < 32) run = seq_compose(run, p);
+        }
+    }
+    if (lane == 0) out[w] = SeqGroup{run, e};
+}
+
+__global__ void __launch_bounds__(64) k_seq_resolve(const double* __restrict__ sq, uint64_t groups,
+                                                    const SeqGroup* __restrict__ runs, double* __restrict__ out) {
+    const int lane = threadIdx.x & 31, chain = threadIdx.x >> 5;
+    sq += uint64_t(chain) * groups * kSeqGroup;
+    runs += uint64_t(chain) * groups;
+    double acc = 0.0;
+    uint64_t g = 0;
+    while (g < groups) {
+        const int e = seq_binade(acc);
+        SeqGroup mine{{0, 0}, 0};
+        if (g + lane < groups) mine = runs[g + lane];
+        bool ok = mine.e == -1 || (e != 0 && mine.e == e);
+        SeqRun incl = mine.run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            SeqRun p;
+            p.d0 = __shfl_up_sync(0xffffffffu, incl.d0, o);
+            p.d1 = __shfl_up_sync(0xffffffffu, incl.d1, o);
+            if (lane >= o) incl = seq_compose(p, incl);
+        }
+        const long long A = seq_integer(acc);
+        const long long after = A + ((A & 1) ? incl.d1 : incl.d0);
+        ok = ok && (e == 0 || after <= kSeqTop);
+        const unsigned bad = ~__ballot_sync(0xffffffffu, ok);
+        const int n = bad ? __ffs(bad) - 1 : 32;  // groups taken as they are
+        if (n > 0 && e != 0) acc = seq_double(__shfl_sync(0xffffffffu, after, n - 1), e);
+        g += n;
+        if (n < 32 && g < groups) {
+            acc = seq_warp(acc, sq + g * kSeqGroup, kSeqGroup);
+            g++;
+        }
+    }
+    if (lane == 0) out[chain] = acc;
+}
+
+// The three kernels take whole groups; smaller subspaces take the one-block kernel.
+constexpr uint64_t kSeqGridPairs = 4096;
+static_assert(kSeqGridPairs % kSeqGroup == 0, "whole groups");
+static_assert((sizeof(float) + sizeof(SeqGroup)) * 2 * ((1u << 19) / kSeqGroup) <= 2 * 4096 * sizeof(double),
+              "the group tables of a 20-qubit register fit the partials");
 
 cudaError_t launch_measure_probs(const void* state, int n, int prec, int target, double* partials,
                                  int max_partials, double* out, cudaStream_t s, int sms, uint64_t zmask,
-                                 uint64_t zval, bool sequential) {
+                                 uint64_t zval, bool sequential, double* squares) {
     const IndexMap map = subspace_map(target, zmask, zval);
     const uint64_t npairs = subspace_pairs(n, target, zmask);
     const uint64_t tb = 1ull << target;
     if (sequential && prec == QS_PREC_C128) {
-        // every amplitude of the subspace in index order: the free bits are all bits but the
-        // collapsed ones (the target's bit is free here)
-        IndexMap all;
-        std::memset(&all, 0, sizeof(all));
-        int k = 0;
-        const uint64_t fixed = zmask & ~tb;
-        for (int b = 0; b < 64; b++)
-            if (fixed >> b & 1ull) all.pos[k++] = uint8_t(b);
-        all.npos = k;
-        all.fixval = zval & fixed;
-        k_prob_sequential<<<1, kT, 0, s>>>((const double2*)state, 2 * npairs, target, all, out);
+        const double2* st = static_cast<const double2*>(state);
+        const uint64_t groups = npairs / kSeqGroup;
+        const size_t table = 2 * groups * sizeof(SeqGroup);
+        if (squares && npairs >= kSeqGridPairs &&
+            table + 2 * groups * sizeof(float) <= 2 * size_t(max_partials) * sizeof(double)) {
+            SeqGroup* runs = reinterpret_cast<SeqGroup*>(partials);
+            float* sums = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(partials) + table);
+            const int grid = int((2 * groups + kT / 32 - 1) / (kT / 32));
+            k_seq_squares<<<grid, kT, 0, s>>>(st, npairs, tb, map, squares, sums);
+            k_seq_groups<<<grid, kT, 0, s>>>(squares, groups, sums, runs);
+            k_seq_resolve<<<1, 64, 0, s>>>(squares, groups, runs, out);
+            return counted(cudaGetLastError(), 3);
+        }
+        const int threads = int(std::min<uint64_t>(1024, std::max<uint64_t>(64, 2 * npairs)));
+        k_prob_seq_block<<<1, (threads + 31) / 32 * 32, 0, s>>>(st, npairs, tb, map, out);
         return counted(cudaGetLastError());
     }
     int grid = grid_cap(npairs, sms, 4);
