@@ -328,3 +328,88 @@ __device__ __forceinline__ double fx_dot(const int32_t* vh, const int32_t* vl, c
 }
 
 }  // namespace qs
+
+namespace qs {
+
+// ---- correctly rounded FP64 products on the integer pipes ------------------------------------
+// sm_103a issues about 2 FP64 operations per clock and SM but 64 integer ones, so a kernel bound by
+// its FP64 operations forms its products here and leaves the additions to the FP64 pipe. The product
+// of a gate's coefficient and an amplitude component: both significands at bit 63 of a 64-bit word,
+// the 128-bit product by four wide multiply-adds, one bit of normalisation, round to nearest even:
+// the bits of __dmul_rn in about 23 instructions.
+//
+// Valid for coefficients im_coef accepts (zero, or 2^-100 <= |c| < 2^100) and components im_in_range
+// accepts (zero, or 2^-800 <= |x| < 2^800): then every product is zero or normal. A zero factor gives
+// +0, whatever the signs.
+struct ImCoef {
+    uint32_t h, l;  // significand << 11
+    uint32_t k;     // sign << 31 | (exponent field - 1023 - 1) << 20, added to the component's exponent
+    uint32_t nz;    // 0: the coefficient is zero
+};
+struct ImVal {
+    uint32_t h, l;  // significand << 11
+    uint32_t se;    // sign and exponent field as in the double's high word, significand bits cleared
+    bool nz;
+};
+
+inline bool im_coef(double c, ImCoef* o) {
+    union {
+        double d;
+        uint64_t u;
+    } v;
+    v.d = c;
+    const uint32_t e = uint32_t(v.u >> 52) & 0x7ffu;
+    o->h = o->l = o->k = o->nz = 0;
+    if (c == 0.0) return true;
+    if (e < 1023u - 100u || e >= 1023u + 100u) return false;
+    const uint64_t m = ((v.u & 0xfffffffffffffull) | (1ull << 52)) << 11;
+    o->h = uint32_t(m >> 32);
+    o->l = uint32_t(m);
+    o->k = (uint32_t(v.u >> 63) << 31) + ((e - 1024u) << 20);
+    o->nz = 1;
+    return true;
+}
+
+__device__ __forceinline__ bool im_in_range(double x) {
+    const uint32_t hi = uint32_t(__double2hiint(x)), lo = uint32_t(__double2loint(x));
+    const uint32_t mag = hi & 0x7fffffffu;
+    return (mag - (223u << 20) < (1600u << 20)) || (mag | lo) == 0u;
+}
+
+__device__ __forceinline__ ImVal im_unpack(double x) {
+    const uint32_t hi = uint32_t(__double2hiint(x)), lo = uint32_t(__double2loint(x));
+    ImVal v;
+    v.h = __funnelshift_l(lo, hi, 11) | 0x80000000u;
+    v.l = lo << 11;
+    v.se = hi & 0xfff00000u;
+    v.nz = (hi & 0x7fffffffu) != 0u;  // in range: a zero high word is a zero
+    return v;
+}
+
+__device__ __forceinline__ uint64_t im_madw(uint32_t a, uint32_t b, uint64_t c) {
+    uint64_t d;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
+}
+
+__device__ __forceinline__ double im_mul(const ImCoef& c, const ImVal& x) {
+    const uint64_t t = im_madw(x.l, c.l, 0ull);
+    const uint64_t u = im_madw(x.h, c.l, t >> 32);
+    const uint64_t v = im_madw(x.l, c.h, u & 0xffffffffull);
+    const uint64_t H = im_madw(x.h, c.h, u >> 32) + (v >> 32);  // bits 127..64 of the product
+    const uint32_t rest = uint32_t(v) | uint32_t(t);             // bits 63..0, as far as they are zero or not
+    uint32_t hh = uint32_t(H >> 32), hl = uint32_t(H);
+    const uint32_t top = hh >> 31, sh = top ^ 1u;  // the leading one at bit 63 or 62
+    hh = __funnelshift_l(hl, hh, sh);
+    hl = hl << sh;
+    const uint32_t qh = hh >> 11, ql = __funnelshift_r(hl, hh, 11);  // 53 bits, then 11 to round
+    const uint32_t odd = (ql & 1u) | (rest != 0u ? 1u : 0u);
+    const uint32_t up = ((hl & 0x7ffu) + odd > 0x400u) ? 1u : 0u;
+    const uint64_t q = ((uint64_t(qh) << 32) | ql) + up;
+    // the implicit bit (and a carry out of the significand) adds to the exponent field
+    const uint32_t hi = uint32_t(q >> 32) + x.se + c.k + (top << 20);
+    const bool nz = x.nz && c.nz != 0u;
+    return __hiloint2double(nz ? int(hi) : 0, nz ? int(uint32_t(q)) : 0);
+}
+
+}  // namespace qs
