@@ -22,6 +22,8 @@
 #include "qs_pass.cuh"
 #include "qs_rot.cuh"
 #include "qs_reduce.cuh"
+#include "qs_sweep.cuh"
+#include "qs_sweep.h"
 #include "qs_tile.h"
 
 namespace qs {
@@ -132,80 +134,78 @@ __global__ void __launch_bounds__(kAT) k_pauli_sum(const T* __restrict__ psi, T*
     }
 }
 
-template <typename T, int AXIS>
-__global__ void __launch_bounds__(kAT) k_rot(T* __restrict__ psi, uint64_t npairs, int q,
-                                             const double2* __restrict__ cs, int slot, int inverse) {
-    using R = decltype(psi[0].x);
-    const double2 t = cs[slot];
-    const R c = R(t.x), s = R(inverse ? -t.y : t.y);
-    const uint64_t lo = (1ull << q) - 1ull, tb = 1ull << q;
-    for (uint64_t p = uint64_t(blockIdx.x) * kAT + threadIdx.x; p < npairs; p += uint64_t(gridDim.x) * kAT) {
-        const uint64_t i0 = ((p & ~lo) << 1) | (p & lo);
-        T a = psi[i0], b = psi[i0 | tb];
-        rot_pair<AXIS>(c, s, a.x, a.y, b.x, b.y);
-        psi[i0] = a;
-        psi[i0 | tb] = b;
-    }
-}
-
-template <typename T, int AXIS>
-__global__ void __launch_bounds__(kAT) k_adj_rot(T* __restrict__ psi, T* __restrict__ lam, uint64_t npairs, int q,
-                                                 const double2* __restrict__ cs, int slot,
-                                                 double* __restrict__ partials) {
-    using R = decltype(psi[0].x);
-    const double2 t = cs[slot];
-    const R c = R(t.x), s = R(-t.y);
-    const uint64_t lo = (1ull << q) - 1ull, tb = 1ull << q;
-    double acc = 0.0;
-    DfAcc facc;
-    for (uint64_t p = uint64_t(blockIdx.x) * kAT + threadIdx.x; p < npairs; p += uint64_t(gridDim.x) * kAT) {
-        const uint64_t i0 = ((p & ~lo) << 1) | (p & lo);
-        T a = psi[i0], b = psi[i0 | tb], l0 = lam[i0], l1 = lam[i0 | tb];
-        if constexpr (sizeof(R) == 8) {
-            acc += im_term<AXIS>(l0, l1, a, b);
-        } else {
-            im_term_acc<AXIS>(facc, l0, l1, a, b);
-        }
-        rot_pair<AXIS>(c, s, a.x, a.y, b.x, b.y);
-        rot_pair<AXIS>(c, s, l0.x, l0.y, l1.x, l1.y);
-        psi[i0] = a;
-        psi[i0 | tb] = b;
-        lam[i0] = l0;
-        lam[i0 | tb] = l1;
-    }
-    if constexpr (sizeof(R) == 4) acc = __dadd_rn(df_f2d(facc.s), df_f2d(facc.c));
-    double dummy = 0.0;
-    rd_block_sum2<kAT>(acc, dummy);
-    if (threadIdx.x == 0) partials[blockIdx.x] = acc;
-}
-
-// Block g sums partials[g * nblocks .. (g+1) * nblocks) into out[g].
+// Block g sums partials[g * nblocks .. (g+1) * nblocks) into out[g], times weights[at[g]] (at[g] < 0: 1).
 __global__ void __launch_bounds__(kAT) k_grad_final(const double* __restrict__ partials, int nblocks,
+                                                    const double* __restrict__ weights, const int* __restrict__ at,
                                                     double* __restrict__ out) {
     const double* p = partials + size_t(blockIdx.x) * nblocks;
     double a = 0.0, b = 0.0;
     for (int i = threadIdx.x; i < nblocks; i += kAT) a += p[i];
     rd_block_sum2<kAT>(a, b);
-    if (threadIdx.x == 0) out[blockIdx.x] = a;
+    if (threadIdx.x == 0) out[blockIdx.x] = at[blockIdx.x] < 0 ? a : a * weights[at[blockIdx.x]];
 }
 
-// ---------------------------------------------------------------- tiled reverse sweep
-// One stage of the reverse sweep over tiles of 2^T amplitudes: psi and lambda tiles side by side in
-// shared memory, the stage's gates taken in reverse order. A rotation adds Im<lambda|A|psi> over the
-// tile's pairs to its slot (FP64, per warp, in shared memory) and is un-applied from both tiles; a
-// fixed gate (its inverse) is applied to both. Gates were reordered only past gates on disjoint
-// qubits, with which they commute, so every inner product equals the one of the gate-by-gate sweep.
-constexpr int kAdjT = 11;           // tile qubits of the reverse sweep (largest; see adj_tile_qubits)
+// ---------------------------------------------------------------- tiled sweeps
+// The forward run and the reverse walk as launches of stage programs (qs_sweep.h): a block takes its
+// tiles of 2^T amplitudes (psi; in the reverse walk psi and lambda side by side) through the program's
+// passes in shared memory. The reverse walk takes the gates backwards, a rotation adding
+// Im<lambda|A|psi> over the tile to its slot before it is un-applied from both vectors. Gates were
+// reordered only past gates on disjoint qubits, with which they commute, so every inner product equals
+// the one of the gate-by-gate walk.
+struct SweepArgs {
+    int RH, pass0, coef0, prog;   // 2^RH tile rows; first pass, first coefficient and index of the program
+    SweepTile t;
+    IndexMap outer;
+    uint8_t rhigh[kTileMaxHigh];
+    int slot[kSwMaxRot];          // global slot of each program-local rotation
+};
+
+// src: psi as the launch finds it (the register's own state in the first launch, which is not written).
+template <int RB>
+constexpr int sweep_threads() {
+    return RB == 3 ? 256 : 128;  // the largest tile that takes RB register bits
+}
+// Blocks per SM: two complex128 tile pairs fill the shared memory; complex64 tiles gain more from a third
+// block's warps (80 registers) than from free registers (20-qubit gradient 1.81 against 1.89 ms).
+template <typename T, int RB, bool REV>
+__global__ void __launch_bounds__(sweep_threads<RB>(), RB < 3 ? 4 : sizeof(T) == 16 ? 2 : REV ? 3 : 4)
+    k_sweep(const typename Sw<T>::Glob* __restrict__ src, typename Sw<T>::Glob* __restrict__ psi,
+            typename Sw<T>::Glob* __restrict__ lam, uint64_t ntiles, const __grid_constant__ SweepArgs a,
+            const SweepPass* __restrict__ passes, const TileOp* __restrict__ fixed,
+            const SweepCoef* __restrict__ coef, const double* __restrict__ sigmas, double* __restrict__ partials) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int nt = blockDim.x;
+    SweepTile t = a.t;
+    t.sigma = sigmas[a.prog];
+    T* sp = reinterpret_cast<T*>(smem_raw);
+    T* sl = sp + (REV ? 1u << t.T : 0u);
+    const SweepSide<T> side(reinterpret_cast<unsigned char*>(sl + (1u << t.T)), t.npass, t.nrot, t.ndiag, REV);
+    for (int r = threadIdx.x; r < (1 << a.RH); r += nt) {
+        uint64_t o = 0;
+        for (int b = 0; b < a.RH; b++)
+            if (r >> b & 1) o |= 1ull << a.rhigh[b];
+        side.rowoff[r] = o;
+    }
+    sw_begin<T>(side, passes + a.pass0, t.npass, coef + a.coef0, t.nrot, t.T, REV, t.sigma, nt);
+    for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
+        sw_tile<T, RB, REV, false>(src, psi, lam, expand_index(tile, a.outer), t, sp, sl, side, fixed, nt);
+    if (REV)
+        for (int r = threadIdx.x; r < t.nrot; r += nt)
+            partials[size_t(a.slot[r]) * gridDim.x + blockIdx.x] = sw_total<T>(side, r, nt);
+}
+
+// ---------------------------------------------------------------- double-float reverse sweep
+// Stages of rotations and pure moves on complex128 registers in QS_ARITH_DF64: psi and lambda tiles as
+// double-float values, one gate after another.
+constexpr int kAdjT = 11;           // tile qubits of the sweeps (largest; see adj_tile_qubits)
 constexpr int kAdjThreads = 256;
 constexpr int kAdjMaxOps = 32;      // gates per stage: the op table is staged in shared memory
-constexpr int kAdjMaxRot = kAdjMaxOps;  // rotations per launch
 
 struct AdjOpDev {
-    TileOp t;      // tile-local form (target bit, tuple expansion, controls, matrix of a fixed gate)
+    TileOp t;      // tile-local form (target bit, tuple expansion, controls)
     int rot;       // stage-local rotation slot, or -1 for a fixed gate
     int axis;      // QS_GATE_RX / RY / RZ
     double c, s;   // cos(theta/2), -sin(theta/2): the inverse rotation
-    float cf, sf;  // the same rounded to float (complex64 tiles)
 };
 
 static_assert(sizeof(AdjOpDev) % 16 == 0, "the op table is copied to shared memory in 16-byte words");
@@ -215,100 +215,8 @@ struct AdjStageArgs {
     int nops, nrot;
     IndexMap outer;
     uint8_t rhigh[kTileMaxHigh];
-    int slot[kAdjMaxRot];  // global rotation slot of each stage-local slot
+    int slot[kAdjMaxOps];  // global rotation slot of each stage-local slot
 };
-
-template <typename T>
-__device__ __forceinline__ void adj_fixed(T* s, const TileOp& op, uint32_t tsize) {
-    using R = decltype(T().x);
-    const uint32_t ntup = tsize >> op.npos;
-    uint32_t seg[5];
-#pragma unroll
-    for (int j = 0; j < 5; j++) seg[j] = op.seg[j];
-    if (op.kind == OP_DENSE || op.kind == OP_DENSE_REAL) {
-        const uint32_t tb = op.off[1];
-        // complex64 tiles read the host-rounded float copy (no FP64-pipe conversions per thread)
-        const auto* mm = [&] {
-            if constexpr (sizeof(R) == 4)
-                return op.mf;
-            else
-                return op.m;
-        }();
-        const R m0 = mm[0], m1 = mm[1], m2 = mm[2], m3 = mm[3], m4 = mm[4], m5 = mm[5], m6 = mm[6], m7 = mm[7];
-        for (uint32_t p = threadIdx.x; p < ntup; p += kAdjThreads) {
-            const uint32_t i0 = tuple_index(p, op.npos, seg, op.pos, op.lfixval);
-            const T a = s[i0], b = s[i0 | tb];
-            T y0 = cfma(m2, m3, b, czero<T>());
-            y0 = cfma(m0, m1, a, y0);
-            T y1 = cfma(m6, m7, b, czero<T>());
-            y1 = cfma(m4, m5, a, y1);
-            s[i0] = y0;
-            s[i0 | tb] = y1;
-        }
-        return;
-    }
-    const int D = 1 << op.k;  // monomial: permutation with factors
-    for (uint32_t p = threadIdx.x; p < ntup; p += kAdjThreads) {
-        const uint32_t i0 = tuple_index(p, op.npos, seg, op.pos, op.lfixval);
-        T y[8];
-#pragma unroll
-        for (int r = 0; r < 8; r++)
-            if (r < D && op.pf[r] != PF_SKIP_DEV) y[r] = s[i0 + op.offsrc[r]];
-#pragma unroll
-        for (int r = 0; r < 8; r++) {
-            if (r >= D || op.pf[r] == PF_SKIP_DEV) continue;
-            T v = y[r];
-            if (op.pf[r] == 255) {
-                R pr, pi;
-                if constexpr (sizeof(R) == 4)
-                    pr = op.mf[2 * r], pi = op.mf[2 * r + 1];
-                else
-                    pr = op.m[2 * r], pi = op.m[2 * r + 1];
-                v = cfma(pr, pi, y[r], czero<T>());
-            } else {
-                v = apply_pf(y[r], op.pf[r]);
-            }
-            s[i0 + op.off[r]] = v;
-        }
-    }
-}
-
-// The rotation un-applied from both tiles; returns this thread's share of Im<lambda|A|psi> (complex128:
-// an FP64 sum; complex64: a compensated float pair).
-template <typename T, int AXIS>
-__device__ __forceinline__ auto adj_rot_tile(T* sp, T* sl, const AdjOpDev& op, uint32_t tsize) {
-    using R = decltype(T().x);
-    const TileOp& t = op.t;
-    uint32_t seg[5];
-#pragma unroll
-    for (int j = 0; j < 5; j++) seg[j] = t.seg[j];
-    const uint32_t tb = 1u << t.tb[0];
-    R c, sn;
-    if constexpr (sizeof(R) == 4)
-        c = op.cf, sn = op.sf;
-    else
-        c = op.c, sn = op.s;
-    double acc = 0.0;
-    DfAcc facc;
-    for (uint32_t p = threadIdx.x; p < (tsize >> 1); p += kAdjThreads) {
-        const uint32_t i0 = tuple_index(p, t.npos, seg, t.pos, 0u), i1 = i0 | tb;
-        T a = sp[i0], b = sp[i1], l0 = sl[i0], l1 = sl[i1];
-        if constexpr (sizeof(R) == 8)
-            acc += im_term<AXIS>(l0, l1, a, b);
-        else
-            im_term_acc<AXIS>(facc, l0, l1, a, b);
-        rot_pair<AXIS>(c, sn, a.x, a.y, b.x, b.y);
-        rot_pair<AXIS>(c, sn, l0.x, l0.y, l1.x, l1.y);
-        sp[i0] = a;
-        sp[i1] = b;
-        sl[i0] = l0;
-        sl[i1] = l1;
-    }
-    if constexpr (sizeof(R) == 4)
-        return facc;
-    else
-        return acc;
-}
 
 template <int AXIS>
 __device__ __forceinline__ DfAcc adj_rot_tile_df(float4* sp, float4* sl, const AdjOpDev& op, uint32_t tsize) {
@@ -361,19 +269,15 @@ __device__ __forceinline__ void adj_move_df(float4* s, const TileOp& op, uint32_
     }
 }
 
-template <typename T, bool DF>
-__global__ void __launch_bounds__(kAdjThreads) k_adj_stage(T* __restrict__ psi, T* __restrict__ lam, uint64_t ntiles,
-                                                           const __grid_constant__ AdjStageArgs a,
-                                                           const AdjOpDev* __restrict__ ops,
-                                                           double* __restrict__ partials) {
-    static_assert(!DF || sizeof(T) == 16, "double-float tiles hold complex128 registers");
+__global__ void __launch_bounds__(kAdjThreads) k_adj_stage_df(double2* __restrict__ psi, double2* __restrict__ lam,
+                                                              uint64_t ntiles, const __grid_constant__ AdjStageArgs a,
+                                                              const AdjOpDev* __restrict__ ops,
+                                                              double* __restrict__ partials) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const uint32_t tsize = 1u << a.T;
-    T* sp = reinterpret_cast<T*>(smem_raw);
-    T* sl = sp + tsize;
-    float4* fp = reinterpret_cast<float4*>(sp);  // the same buffers as double-float amplitudes
-    float4* fl = reinterpret_cast<float4*>(sl);
-    double* sacc = reinterpret_cast<double*>(sl + tsize);  // [nrot][8 warps]
+    float4* fp = reinterpret_cast<float4*>(smem_raw);
+    float4* fl = fp + tsize;
+    double* sacc = reinterpret_cast<double*>(fl + tsize);  // [nrot][8 warps]
     AdjOpDev* sops = reinterpret_cast<AdjOpDev*>(sacc + size_t(a.nrot) * (kAdjThreads / 32));
     uint64_t* rowoff = reinterpret_cast<uint64_t*>(sops + a.nops);
     const int nrows = 1 << a.RH, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -396,79 +300,41 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_stage(T* __restrict__ psi, 
         const uint64_t base = expand_index(tile, a.outer);
         for (uint32_t i = threadIdx.x; i < tsize; i += kAdjThreads) {
             const uint64_t g = base + rowoff[i >> a.RL] + (i & rmask);
-            if constexpr (DF) {
-                const double2 v = reinterpret_cast<const double2*>(psi)[g], w = reinterpret_cast<const double2*>(lam)[g];
-                float4 f;
-                df_split(v.x, f.x, f.y);
-                df_split(v.y, f.z, f.w);
-                fp[i] = f;
-                df_split(w.x, f.x, f.y);
-                df_split(w.y, f.z, f.w);
-                fl[i] = f;
-            } else {
-                sp[i] = psi[g];
-                sl[i] = lam[g];
-            }
+            const double2 v = psi[g], w = lam[g];
+            float4 f;
+            df_split(v.x, f.x, f.y);
+            df_split(v.y, f.z, f.w);
+            fp[i] = f;
+            df_split(w.x, f.x, f.y);
+            df_split(w.y, f.z, f.w);
+            fl[i] = f;
         }
         __syncthreads();
         for (int o = 0; o < a.nops; o++) {
             const AdjOpDev& op = sops[o];
             if ((base & op.t.omask) != op.t.oval) continue;  // the same for the whole block
-            if (op.rot >= 0) {
-                double v;
-                if constexpr (DF) {  // the warp's float pairs reduced on the FP32 pipe, one FP64 rejoin
-                    DfAcc f;
-                    if (op.axis == QS_GATE_RX)
-                        f = adj_rot_tile_df<QS_GATE_RX>(fp, fl, op, tsize);
-                    else if (op.axis == QS_GATE_RY)
-                        f = adj_rot_tile_df<QS_GATE_RY>(fp, fl, op, tsize);
-                    else
-                        f = adj_rot_tile_df<QS_GATE_RZ>(fp, fl, op, tsize);
-                    f.warp_reduce();
-                    v = __dadd_rn(df_f2d(f.s), df_f2d(f.c));
-                } else if constexpr (sizeof(T) == 8) {
-                    // complex64: the warp's compensated float pairs reduced on the FP32 pipe, one
-                    // FP64 rejoin per warp
-                    DfAcc f;
-                    if (op.axis == QS_GATE_RX)
-                        f = adj_rot_tile<T, QS_GATE_RX>(sp, sl, op, tsize);
-                    else if (op.axis == QS_GATE_RY)
-                        f = adj_rot_tile<T, QS_GATE_RY>(sp, sl, op, tsize);
-                    else
-                        f = adj_rot_tile<T, QS_GATE_RZ>(sp, sl, op, tsize);
-                    f.warp_reduce();
-                    v = __dadd_rn(df_f2d(f.s), df_f2d(f.c));
-                } else {
-                    if (op.axis == QS_GATE_RX)
-                        v = adj_rot_tile<T, QS_GATE_RX>(sp, sl, op, tsize);
-                    else if (op.axis == QS_GATE_RY)
-                        v = adj_rot_tile<T, QS_GATE_RY>(sp, sl, op, tsize);
-                    else
-                        v = adj_rot_tile<T, QS_GATE_RZ>(sp, sl, op, tsize);
-                    v = rd_warp_sum(v);
-                }
+            if (op.rot >= 0) {  // the warp's float pairs reduced on the FP32 pipe, one FP64 rejoin
+                DfAcc f;
+                if (op.axis == QS_GATE_RX)
+                    f = adj_rot_tile_df<QS_GATE_RX>(fp, fl, op, tsize);
+                else if (op.axis == QS_GATE_RY)
+                    f = adj_rot_tile_df<QS_GATE_RY>(fp, fl, op, tsize);
+                else
+                    f = adj_rot_tile_df<QS_GATE_RZ>(fp, fl, op, tsize);
+                f.warp_reduce();
+                const double v = __dadd_rn(df_f2d(f.s), df_f2d(f.c));
                 if (lane == 0) sacc[op.rot * (kAdjThreads / 32) + warp] += v;
-            } else if constexpr (DF) {
+            } else {
                 adj_move_df(fp, op.t, tsize);
                 adj_move_df(fl, op.t, tsize);
-            } else {
-                adj_fixed(sp, op.t, tsize);
-                adj_fixed(sl, op.t, tsize);
             }
             __syncthreads();
         }
         for (uint32_t i = threadIdx.x; i < tsize; i += kAdjThreads) {
             const uint64_t g = base + rowoff[i >> a.RL] + (i & rmask);
-            if constexpr (DF) {
-                const float4 f = fp[i], h = fl[i];
-                reinterpret_cast<double2*>(psi)[g] =
-                    make_double2(__dadd_rn(df_f2d(f.x), df_f2d(f.y)), __dadd_rn(df_f2d(f.z), df_f2d(f.w)));
-                reinterpret_cast<double2*>(lam)[g] =
-                    make_double2(__dadd_rn(df_f2d(h.x), df_f2d(h.y)), __dadd_rn(df_f2d(h.z), df_f2d(h.w)));
-            } else {
-                psi[g] = sp[i];
-                lam[g] = sl[i];
-            }
+            const float4 f = fp[i], h = fl[i];
+            psi[g] = make_double2(__dadd_rn(df_f2d(f.x), df_f2d(f.y)), __dadd_rn(df_f2d(f.z), df_f2d(f.w)));
+            lam[g] = make_double2(__dadd_rn(df_f2d(h.x), df_f2d(h.y)), __dadd_rn(df_f2d(h.z), df_f2d(h.w)));
         }
         __syncthreads();
     }
@@ -573,34 +439,7 @@ done:
     return rc;
 }
 
-template <typename T>
-static void launch_rot(int kind, void* psi, int n, int q, const double2* cs, int slot, int inverse, cudaStream_t s,
-                       int sms) {
-    const uint64_t np = 1ull << (n - 1);
-    const int grid = grid_for_pairs(np, sms);
-    if (kind == QS_GATE_RX)
-        k_rot<T, QS_GATE_RX><<<grid, kAT, 0, s>>>((T*)psi, np, q, cs, slot, inverse);
-    else if (kind == QS_GATE_RY)
-        k_rot<T, QS_GATE_RY><<<grid, kAT, 0, s>>>((T*)psi, np, q, cs, slot, inverse);
-    else
-        k_rot<T, QS_GATE_RZ><<<grid, kAT, 0, s>>>((T*)psi, np, q, cs, slot, inverse);
-    note_launches(1);
-}
-
-template <typename T>
-static void launch_adj_rot(int kind, void* psi, void* lam, int n, int q, const double2* cs, int slot,
-                           double* partials, int grid, cudaStream_t s) {
-    const uint64_t np = 1ull << (n - 1);
-    if (kind == QS_GATE_RX)
-        k_adj_rot<T, QS_GATE_RX><<<grid, kAT, 0, s>>>((T*)psi, (T*)lam, np, q, cs, slot, partials);
-    else if (kind == QS_GATE_RY)
-        k_adj_rot<T, QS_GATE_RY><<<grid, kAT, 0, s>>>((T*)psi, (T*)lam, np, q, cs, slot, partials);
-    else
-        k_adj_rot<T, QS_GATE_RZ><<<grid, kAT, 0, s>>>((T*)psi, (T*)lam, np, q, cs, slot, partials);
-    note_launches(1);
-}
-
-// R_A(theta) as a row-major interleaved 2x2 matrix (the convention of rot_pair).
+// R_A(theta) as a row-major interleaved 2x2 matrix.
 static std::vector<double> rotation_matrix(int axis, double c, double s) {
     if (axis == QS_GATE_RX) return {c, 0, 0, -s, 0, -s, c, 0};
     if (axis == QS_GATE_RY) return {c, 0, -s, 0, s, 0, c, 0};
@@ -612,149 +451,329 @@ static std::vector<double> rotation_matrix(int axis, double c, double s) {
 // and the whole state in one tile up to 8 qubits (one block runs every gate without a launch each).
 static int adj_tile_qubits(int n, int cap) { return std::min(n, std::max(8, std::min(cap, n - 7))); }
 
-constexpr int kAdjTiledMin = 6;  // from this many qubits the gradient runs as tiled stages
+constexpr int kAdjDfMin = 6;  // from this many qubits QS_ARITH_DF64 runs double-float tiles
 
-// Grid of the tiled reverse sweep for n qubits in tiles of tq qubits (the same for every stage, so
-// partials line up).
-template <typename T>
-static int adj_grid(int n, int tq, int sms) {
-    const size_t smem = 2 * (sizeof(T) << kAdjT) + size_t(kAdjMaxRot) * (kAdjThreads / 32) * 8 +
-                        size_t(kAdjMaxOps) * sizeof(AdjOpDev) + (8u << 6);
-    int per_sm = 1;  // the smaller of the two variants' occupancies (each variant's limit raised to smem)
-    resident_blocks(reinterpret_cast<const void*>(k_adj_stage<T, false>), kAdjThreads, smem, &per_sm);
-    if (sizeof(T) == 16) {
-        int df = 1;
-        resident_blocks(reinterpret_cast<const void*>(k_adj_stage<T, sizeof(T) == 16>), kAdjThreads, smem, &df);
-        per_sm = std::min(per_sm, df);
-    }
-    const uint64_t ntiles = 1ull << (n - tq);
-    return int(std::min<uint64_t>(ntiles, uint64_t(sms) * uint64_t(std::max(1, per_sm))));
+// The tile types of qs_sweep.cuh.
+enum SweepType { SW_C64, SW_FX, SW_F64 };
+
+template <typename T, int RB>
+static int sweep_per_sm(int tq) {
+    const size_t smem = 2 * (sizeof(T) << tq) + SweepSide<T>::bytes(kSwMaxPass, kSwMaxRot, kSwMaxDiag, true, kTileMaxHigh);
+    int per_sm = 1;
+    resident_blocks(reinterpret_cast<const void*>(k_sweep<T, RB, false>), sweep_threads<RB>(), smem, &per_sm);  // raises its limit
+    resident_blocks(reinterpret_cast<const void*>(k_sweep<T, RB, true>), sweep_threads<RB>(), smem, &per_sm);
+    return std::max(1, per_sm);
 }
 
-// The reverse sweep as tiled stages: gates m-1 .. 0, rotations with their inner products, fixed
-// gates as their inverses (inv, whose entries are moved out). Partials of rotation slot r land in
-// part[r * grid .. + grid).
-template <typename T>
-static int reverse_tiled(void* state, void* lam, int n, int prec, int arith, const qs_param_gate* gates, size_t m,
-                         const double* params, const std::vector<int>& rot_slot, std::vector<OpDesc>& inv,
-                         double* part, int grid, cudaStream_t s, int sms, std::string* msg) {
-    std::vector<OpDesc> rops;
-    std::vector<int> src;
-    rops.reserve(m);
-    src.reserve(m);
-    for (size_t gg = m; gg-- > 0;) {
-        if (rot_slot[gg] >= 0) {  // planning form: a dense 1-qubit gate on the rotation's target
+// Calls F<T, RB>() for a tile type and tile size.
+#define QS_SWEEP(type, tq, F)                                  \
+    [&] {                                                      \
+        const int rb_ = sw_register_bits(tq);                  \
+        if ((type) == SW_C64) {                                \
+            if (rb_ == 3) return F(float2, 3);                 \
+            if (rb_ == 2) return F(float2, 2);                 \
+            return F(float2, 1);                               \
+        }                                                      \
+        if ((type) == SW_FX) {                                 \
+            if (rb_ == 3) return F(FxC, 3);                    \
+            if (rb_ == 2) return F(FxC, 2);                    \
+            return F(FxC, 1);                                  \
+        }                                                      \
+        if (rb_ == 3) return F(double2, 3);                    \
+        if (rb_ == 2) return F(double2, 2);                    \
+        return F(double2, 1);                                  \
+    }()
+
+// Blocks of a launch over 2^n amplitudes in tiles of tq qubits (the same for every launch of a gradient,
+// so that partials line up).
+static int sweep_grid(int n, int tq, SweepType type, bool df, int sms) {
+#define QS_F(T, RB) sweep_per_sm<T, RB>(tq)
+    int per_sm = QS_SWEEP(type, tq, QS_F);
+#undef QS_F
+    if (df) {
+        int k = 1;
+        const size_t smem = 2 * (sizeof(float4) << kAdjT) + size_t(kAdjMaxOps) * (kAdjThreads / 32) * 8 +
+                            size_t(kAdjMaxOps) * sizeof(AdjOpDev) + (8u << kTileMaxHigh);
+        resident_blocks(reinterpret_cast<const void*>(k_adj_stage_df), kAdjThreads, smem, &k);
+        per_sm = std::max(1, std::min(per_sm, k));
+    }
+    return int(std::min<uint64_t>(1ull << (n - tq), uint64_t(sms) * uint64_t(per_sm)));
+}
+
+// The circuit as sweeps: the gates in order of execution, their stages, and the launches with their
+// tables. A launch is a program, a double-float stage (df) or a gate no tile holds (single).
+struct SweepPlan {
+    struct Launch {
+        int stage = 0, single = -1, prog = -1;
+        bool df = false;
+        int first = 0, count = 0;            // df: entries of df_ops
+        SweepProgram program;
+        std::vector<int> slots;              // df: global slots
+    };
+    SweepType type = SW_F64;
+    std::vector<OpDesc> ops;                 // planning form, in order of execution
+    std::vector<int> src;                    // gate index of each op
+    std::vector<TileStage> stages;
+    std::vector<Launch> launches;
+    std::vector<SweepRange> ranges;          // per program
+    std::vector<SweepPass> passes;
+    std::vector<SweepRot> rots;
+    std::vector<TileOp> fixed;
+    std::vector<AdjOpDev> df_ops;
+    std::vector<int> weight_at;              // per rotation slot: its coefficient, -1: none
+};
+
+// gates in order (reverse: backwards), fixed gates as `fixed` classifies them (moved out).
+static void plan_sweep(const qs_param_gate* gates, size_t m, const double2* angles, const std::vector<int>& rot_slot,
+                       int nrot, std::vector<OpDesc>& fixed, int n, int tq, bool reverse, SweepType type, bool df,
+                       bool ordered, SweepPlan* P) {
+    P->type = type;
+    P->ops.reserve(m);
+    P->src.reserve(m);
+    for (size_t k = 0; k < m; k++) {
+        const size_t g = reverse ? m - 1 - k : k;
+        if (rot_slot[g] >= 0) {  // planning form: a dense 1-qubit gate on the rotation's target
             OpDesc d;
             d.kind = OP_DENSE;
             d.k = d.orig_k = 1;
-            d.tq[0] = int(gates[gg].targets[0]);
+            d.tq[0] = int(gates[g].targets[0]);
             d.m.assign(8, 0.0);
             d.touched_rows = 2;
-            rops.push_back(std::move(d));
+            P->ops.push_back(std::move(d));
         } else {
-            rops.push_back(std::move(inv[gg]));  // consumed: the caller reads inv no further
+            P->ops.push_back(std::move(fixed[g]));
         }
-        src.push_back(int(gg));
+        P->src.push_back(int(g));
     }
-    const int tq = adj_tile_qubits(n, kAdjT);
-    const std::vector<TileStage> stages = plan_tiles(rops, n, tq, 5, false, kAdjMaxOps);
-    // device tables: every stage's ops (split so a launch holds at most kAdjMaxRot rotations)
-    std::vector<AdjOpDev> host;
-    struct Launch {
-        int stage, first, count, nrot;
-        int slot[kAdjMaxRot];
-        bool moves_only;  // every fixed gate a pure move (double-float tiles can take the launch)
-    };
-    std::vector<Launch> launches;
-    for (size_t si = 0; si < stages.size(); si++) {
-        const TileStage& st = stages[si];
+    P->weight_at.assign(std::max(1, nrot), -1);
+    // rows of 128 bytes: more of the tile's qubits are free to choose
+    const int low = df || ordered ? 5 : type == SW_C64 ? 4 : 3;
+    P->stages = plan_tiles(P->ops, n, tq, std::min(low, tq), false, df || ordered ? kAdjMaxOps : kSwMaxRot);
+    for (size_t si = 0; si < P->stages.size(); si++) {
+        const TileStage& st = P->stages[si];
+        SweepPlan::Launch L;
+        L.stage = int(si);
         if (!st.tiled) {
-            launches.push_back(Launch{int(si), -1, 0, 0, {}, false});
+            L.single = st.single;
+            P->launches.push_back(L);
             continue;
         }
-        Launch cur{int(si), int(host.size()), 0, 0, {}, true};
+        bool moves_only = true;  // double-float tiles take rotations and pure moves
+        for (int idx : st.ops)
+            if (rot_slot[P->src[idx]] < 0 && P->ops[idx].kind != OP_MONO_PF) moves_only = false;
+        if (df && moves_only) {
+            L.df = true;
+            L.first = int(P->df_ops.size());
+            for (int idx : st.ops) {
+                const int g = P->src[idx];
+                AdjOpDev e;
+                std::memset(&e, 0, sizeof(e));
+                e.t = make_tile_op(P->ops[idx], st);
+                e.rot = -1;
+                if (rot_slot[g] >= 0) {
+                    e.rot = int(L.slots.size());
+                    L.slots.push_back(rot_slot[g]);
+                    e.axis = gates[g].kind;
+                    e.c = angles[g].x;
+                    e.s = -angles[g].y;
+                }
+                P->df_ops.push_back(e);
+            }
+            L.count = int(P->df_ops.size()) - L.first;
+            P->launches.push_back(L);
+            continue;
+        }
+        std::vector<SweepGate> sg;
         for (int idx : st.ops) {
-            const int g = src[idx];
-            if (rot_slot[g] >= 0 && cur.nrot == kAdjMaxRot) {
-                launches.push_back(cur);
-                cur = Launch{int(si), int(host.size()), 0, 0, {}, true};
-            }
-            AdjOpDev e;
-            std::memset(&e, 0, sizeof(e));
-            e.t = make_tile_op(rops[idx], st);
-            e.rot = -1;
-            if (rot_slot[g] < 0 && rops[idx].kind != OP_MONO_PF) cur.moves_only = false;
+            const int g = P->src[idx];
+            SweepGate e;
+            e.gate = g;
             if (rot_slot[g] >= 0) {
-                const double th = params[gates[g].param];
-                e.rot = cur.nrot;
-                cur.slot[cur.nrot++] = rot_slot[g];
                 e.axis = gates[g].kind;
-                e.c = std::cos(0.5 * th);
-                e.s = -std::sin(0.5 * th);
-                e.cf = float(e.c);
-                e.sf = float(e.s);
+                e.target = int(gates[g].targets[0]);
+            } else {
+                e.fixed = &P->ops[idx];
             }
-            host.push_back(e);
-            cur.count++;
+            sg.push_back(e);
         }
-        launches.push_back(cur);
+        for (SweepProgram& prog : build_sweep(sg, st, type == SW_FX, reverse, ordered, &P->fixed)) {
+            L.prog = int(P->ranges.size());
+            P->ranges.push_back(SweepRange{int(P->passes.size()), int(prog.passes.size()), int(P->rots.size()),
+                                           int(prog.rots.size()), prog.ndiag, type != SW_FX, type == SW_C64, 0});
+            for (int g : prog.rots) {
+                P->weight_at[rot_slot[g]] = int(P->rots.size());
+                P->rots.push_back(SweepRot{g, gates[g].kind});
+            }
+            P->passes.insert(P->passes.end(), prog.passes.begin(), prog.passes.end());
+            L.program = std::move(prog);
+            P->launches.push_back(L);
+        }
     }
-    AdjOpDev* dops = nullptr;
-    if (!host.empty()) {
-        const size_t bytes = host.size() * sizeof(AdjOpDev);
-        cudaError_t e = cudaMallocAsync((void**)&dops, bytes, s);
-        if (e == cudaSuccess) {  // page-locked: the upload does not wait for the forward pass queued before it
-            void* stage = pinned_staging(1, bytes);
-            if (stage) std::memcpy(stage, host.data(), bytes);
-            e = cudaMemcpyAsync(dops, stage ? stage : host.data(), bytes, cudaMemcpyHostToDevice, s);
-        }
-        if (e != cudaSuccess) return fail(e, "reverse-sweep tables", msg);
+}
+
+// Copy rows and tuple expansion of a stage's tiles.
+template <typename A>
+static void tile_geometry(const TileStage& st, A* a, int* T, int* RL) {
+    *T = st.T;
+    const int H = int(st.high.size());
+    int run = 0;
+    while (run < H && st.high[run] == st.L + run) run++;
+    *RL = st.L + run;
+    a->RH = H - run;
+    for (int b = 0; b < a->RH; b++) a->rhigh[b] = uint8_t(st.high[run + b]);
+    std::vector<int> qpos;
+    for (int q = 0; q < st.L; q++) qpos.push_back(q);
+    for (int q : st.high) qpos.push_back(q);
+    std::sort(qpos.begin(), qpos.end());
+    a->outer.npos = int(qpos.size());
+    for (size_t i = 0; i < qpos.size(); i++) a->outer.pos[i] = uint8_t(qpos[i]);
+}
+
+// A plan's tables on the device.
+struct SweepTables {
+    unsigned char* dev = nullptr;
+    const SweepRange* ranges = nullptr;
+    const SweepPass* passes = nullptr;
+    const SweepRot* rots = nullptr;
+    const TileOp* fixed = nullptr;
+    const AdjOpDev* df_ops = nullptr;
+    const int* weight_at = nullptr;
+    const double2* angles = nullptr;
+    SweepCoef* coefs = nullptr;
+    double* weights = nullptr;
+    double* sigmas = nullptr;
+};
+
+template <typename T, int RB>
+static void launch_sweep(bool reverse, const void* src, void* psi, void* lam, uint64_t ntiles, const SweepArgs& a,
+                         const SweepTables& tb, double* part, int grid, cudaStream_t s) {
+    using G = typename Sw<T>::Glob;
+    const size_t smem = size_t(reverse ? 2 : 1) * (sizeof(T) << a.t.T) +
+                        SweepSide<T>::bytes(a.t.npass, a.t.nrot, a.t.ndiag, reverse, a.RH);
+    const int threads = std::max(32, (1 << a.t.T) >> RB);
+    if (reverse)
+        k_sweep<T, RB, true><<<grid, threads, smem, s>>>((const G*)src, (G*)psi, (G*)lam, ntiles, a, tb.passes, tb.fixed,
+                                                         tb.coefs, tb.sigmas, part);
+    else
+        k_sweep<T, RB, false><<<grid, threads, smem, s>>>((const G*)src, (G*)psi, (G*)lam, ntiles, a, tb.passes,
+                                                          tb.fixed, tb.coefs, tb.sigmas, part);
+}
+
+// Uploads a plan's tables (through page-locked staging buffer `staging`, so that the upload does not wait
+// for work queued before it) and forms its coefficients. tb->dev is the caller's to free.
+static int upload_sweep(const SweepPlan& P, const std::vector<double2>& angles, int staging, cudaStream_t s,
+                        SweepTables* tb, std::string* msg) {
+    auto al = [](size_t x) { return ((x + 255) / 256) * 256; };
+    const size_t o_range = 0, o_pass = o_range + al(P.ranges.size() * sizeof(SweepRange)),
+                 o_rot = o_pass + al(P.passes.size() * sizeof(SweepPass)), o_fix = o_rot + al(P.rots.size() * sizeof(SweepRot)),
+                 o_df = o_fix + al(P.fixed.size() * sizeof(TileOp)), o_at = o_df + al(P.df_ops.size() * sizeof(AdjOpDev)),
+                 o_ang = o_at + al(P.weight_at.size() * sizeof(int)), up = o_ang + al(angles.size() * sizeof(double2)),
+                 o_coef = up, o_wt = o_coef + al(P.rots.size() * sizeof(SweepCoef)), o_sig = o_wt + al(P.rots.size() * 8 + 8),
+                 total = o_sig + al(P.ranges.size() * 8 + 8);
+    cudaError_t e = cudaMallocAsync((void**)&tb->dev, total, s);
+    if (e != cudaSuccess) {
+        tb->dev = nullptr;
+        return fail(e, "sweep tables", msg);
     }
-    int rc = QS_OK;
-    const uint64_t ntiles = 1ull << (n - tq);
-    for (const Launch& L : launches) {
-        const TileStage& st = stages[L.stage];
-        if (L.first < 0) {  // a gate no tile holds: its inverse on psi and lambda, one sweep each
-            const OpDesc& op = rops[st.single];
-            if ((rc = apply_op(state, n, prec, arith, op, s, sms, msg)) != QS_OK) break;
-            if ((rc = apply_op(lam, n, prec, arith, op, s, sms, msg)) != QS_OK) break;
-            continue;
-        }
-        AdjStageArgs a;
-        std::memset(&a, 0, sizeof(a));
-        a.T = st.T;
-        const int H = int(st.high.size());
-        int run = 0;
-        while (run < H && st.high[run] == st.L + run) run++;
-        a.RL = st.L + run;
-        a.RH = H - run;
-        for (int b = 0; b < a.RH; b++) a.rhigh[b] = uint8_t(st.high[run + b]);
-        std::vector<int> qpos;
-        for (int q = 0; q < st.L; q++) qpos.push_back(q);
-        for (int q : st.high) qpos.push_back(q);
-        std::sort(qpos.begin(), qpos.end());
-        a.outer.npos = int(qpos.size());
-        for (size_t i = 0; i < qpos.size(); i++) a.outer.pos[i] = uint8_t(qpos[i]);
-        a.nops = L.count;
-        a.nrot = L.nrot;
-        for (int r = 0; r < L.nrot; r++) a.slot[r] = L.slot[r];
-        const size_t smem = 2 * (sizeof(T) << st.T) + size_t(a.nrot) * (kAdjThreads / 32) * 8 +
-                            size_t(a.nops) * sizeof(AdjOpDev) + (8u << a.RH);
-        if (sizeof(T) == 16 && L.moves_only && arith == QS_ARITH_DF64)
-            k_adj_stage<T, sizeof(T) == 16><<<grid, kAdjThreads, smem, s>>>((T*)state, (T*)lam, ntiles, a,
-                                                                           dops + L.first, part);
-        else
-            k_adj_stage<T, false><<<grid, kAdjThreads, smem, s>>>((T*)state, (T*)lam, ntiles, a, dops + L.first,
-                                                                  part);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) {
-            rc = fail(e, "reverse-sweep stage", msg);
-            break;
-        }
+    std::vector<unsigned char> pageable;
+    unsigned char* host = static_cast<unsigned char*>(pinned_staging(staging, up));
+    if (!host) {
+        pageable.resize(up);
+        host = pageable.data();
+    }
+    auto put = [&](size_t at, const void* p, size_t bytes) {
+        if (bytes) std::memcpy(host + at, p, bytes);
+    };
+    put(o_range, P.ranges.data(), P.ranges.size() * sizeof(SweepRange));
+    put(o_pass, P.passes.data(), P.passes.size() * sizeof(SweepPass));
+    put(o_rot, P.rots.data(), P.rots.size() * sizeof(SweepRot));
+    put(o_fix, P.fixed.data(), P.fixed.size() * sizeof(TileOp));
+    put(o_df, P.df_ops.data(), P.df_ops.size() * sizeof(AdjOpDev));
+    put(o_at, P.weight_at.data(), P.weight_at.size() * sizeof(int));
+    put(o_ang, angles.data(), angles.size() * sizeof(double2));
+    e = cudaMemcpyAsync(tb->dev, host, up, cudaMemcpyHostToDevice, s);
+    if (e != cudaSuccess) return fail(e, "sweep tables", msg);
+    tb->ranges = reinterpret_cast<const SweepRange*>(tb->dev + o_range);
+    tb->passes = reinterpret_cast<const SweepPass*>(tb->dev + o_pass);
+    tb->rots = reinterpret_cast<const SweepRot*>(tb->dev + o_rot);
+    tb->fixed = reinterpret_cast<const TileOp*>(tb->dev + o_fix);
+    tb->df_ops = reinterpret_cast<const AdjOpDev*>(tb->dev + o_df);
+    tb->weight_at = reinterpret_cast<const int*>(tb->dev + o_at);
+    tb->angles = reinterpret_cast<const double2*>(tb->dev + o_ang);
+    tb->coefs = reinterpret_cast<SweepCoef*>(tb->dev + o_coef);
+    tb->weights = reinterpret_cast<double*>(tb->dev + o_wt);
+    tb->sigmas = reinterpret_cast<double*>(tb->dev + o_sig);
+    if (!P.ranges.empty()) {
+        k_sweep_coefs<<<int(P.ranges.size()), 64, 0, s>>>(tb->ranges, tb->passes, tb->rots, tb->angles, tb->coefs,
+                                                         tb->weights, tb->sigmas);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return fail(e, "sweep coefficients", msg);
         note_launches(1);
     }
-    if (dops) cudaFreeAsync(dops, s);
-    return rc;
+    return QS_OK;
+}
+
+// Runs a plan: psi (and lam in the reverse walk) hold the vectors; src, when not null, is where the
+// first launch finds psi. Partials of rotation slot r land in part[r * grid .. + grid).
+static int run_sweep(const SweepPlan& P, const SweepTables& tb, const void* src, void* psi, void* lam, int n, int prec,
+                     int arith, bool reverse, const std::vector<int>& rot_slot, double* part, int grid, cudaStream_t s,
+                     int sms, std::string* msg) {
+    const size_t amp = prec == QS_PREC_C64 ? 8 : 16;
+    cudaError_t e = cudaSuccess;
+    for (size_t li = 0; li < P.launches.size(); li++) {
+        const SweepPlan::Launch& L = P.launches[li];
+        const TileStage& st = P.stages[L.stage];
+        if (src && (L.single >= 0 || L.df)) {  // works in place
+            e = cudaMemcpyAsync(psi, src, (size_t(1) << n) * amp, cudaMemcpyDeviceToDevice, s);
+            if (e != cudaSuccess) return fail(e, "state copy", msg);
+            src = nullptr;
+        }
+        if (L.single >= 0) {  // a gate no tile holds: one sweep each
+            int rc = apply_op(psi, n, prec, arith, P.ops[L.single], s, sms, msg);
+            if (rc == QS_OK && reverse) rc = apply_op(lam, n, prec, arith, P.ops[L.single], s, sms, msg);
+            if (rc != QS_OK) return rc;
+            continue;
+        }
+        const uint64_t ntiles = 1ull << (n - st.T);
+        if (L.df) {
+            AdjStageArgs a;
+            std::memset(&a, 0, sizeof(a));
+            tile_geometry(st, &a, &a.T, &a.RL);
+            a.nops = L.count;
+            a.nrot = int(L.slots.size());
+            for (int r = 0; r < a.nrot; r++) a.slot[r] = L.slots[r];
+            const size_t smem = 2 * (sizeof(float4) << st.T) + size_t(a.nrot) * (kAdjThreads / 32) * 8 +
+                                size_t(a.nops) * sizeof(AdjOpDev) + (8u << a.RH);
+            k_adj_stage_df<<<grid, kAdjThreads, smem, s>>>((double2*)psi, (double2*)lam, ntiles, a, tb.df_ops + L.first,
+                                                           part);
+        } else {
+            SweepArgs a;
+            std::memset(&a, 0, sizeof(a));
+            tile_geometry(st, &a, &a.t.T, &a.t.RL);
+            const SweepRange& R = P.ranges[L.prog];
+            a.t.npass = R.npass;
+            a.t.nrot = R.nrot;
+            a.t.ndiag = R.ndiag;
+            a.t.store = !reverse || li + 1 < P.launches.size();
+            a.pass0 = R.pass0;
+            a.coef0 = R.coef0;
+            a.prog = L.prog;
+            for (int r = 0; r < R.nrot; r++) a.slot[r] = rot_slot[L.program.rots[r]];
+            const void* from = src ? src : psi;
+#define QS_F(T, RB) launch_sweep<T, RB>(reverse, from, psi, lam, ntiles, a, tb, part, grid, s)
+            QS_SWEEP(P.type, st.T, QS_F);
+#undef QS_F
+        }
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return fail(e, "sweep", msg);
+        note_launches(1);
+        src = nullptr;
+    }
+    if (src) {  // no launch took the state over
+        e = cudaMemcpyAsync(psi, src, (size_t(1) << n) * amp, cudaMemcpyDeviceToDevice, s);
+        if (e != cudaSuccess) return fail(e, "state copy", msg);
+    }
+    return QS_OK;
 }
 
 int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gate* gates, size_t m,
@@ -806,55 +825,59 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
         }
     }
     // ---- tables
-    std::vector<double2> cs(std::max<size_t>(m, 1));
-    for (size_t g = 0; g < m; g++)
-        if (rot_slot[g] >= 0) {
-            const double th = params[gates[g].param];
-            cs[g] = make_double2(std::cos(0.5 * th), std::sin(0.5 * th));
-        }
     std::vector<PauliDev> ht = pauli_table(terms, nt);
     const size_t amp = prec == QS_PREC_C64 ? 8 : 16;
     const uint64_t N = 1ull << n;
-    const bool tiled = n >= kAdjTiledMin;  // forward as fused stages, reverse sweep as tiled stages
+    const bool df = prec == QS_PREC_C128 && arith == QS_ARITH_DF64 && n >= kAdjDfMin;
     const int tq = adj_tile_qubits(n, kAdjT);
-    const int pgrid = tiled ? (prec == QS_PREC_C64 ? adj_grid<float2>(n, tq, sms) : adj_grid<double2>(n, tq, sms))
-                            : grid_for_pairs(N >> 1, sms);
+    bool unitary = true;
+    for (size_t g = 0; g < m && unitary; g++)
+        if (gates[g].kind == QS_GATE_FIXED) unitary = is_unitary(gates[g].matrix, gates[g].k);
+    const SweepType type = prec == QS_PREC_C64 ? SW_C64 : unitary ? SW_FX : SW_F64;
+    const int pgrid = sweep_grid(n, tq, type, df, sms);
     auto al = [](size_t x) { return ((x + 255) / 256) * 256; };
-    const size_t o_cs = 0, o_terms = o_cs + al(cs.size() * 16), o_part = o_terms + al(nt * sizeof(PauliDev) + 1),
+    const size_t o_terms = 0, o_part = o_terms + al(nt * sizeof(PauliDev) + 1),
                  o_res = o_part + al(size_t(std::max(nrot, 1)) * pgrid * 8 + 4096 * 16),
                  o_err = o_res + al((2 + size_t(nrot)) * 8), o_lam = o_err + al(sizeof(int)),
-                 o_save = o_lam + al(N * amp), total = o_save + N * amp;
+                 o_psi = o_lam + al(N * amp), total = o_psi + N * amp;
     unsigned char* blob = nullptr;
     std::vector<double> res(2 + nrot, 0.0);
+    std::vector<double2> angles(std::max<size_t>(m, 1), make_double2(1.0, 0.0));  // per gate: cos, sin of theta / 2
+    for (size_t g = 0; g < m; g++)
+        if (rot_slot[g] >= 0) {
+            const double th = params[gates[g].param];
+            angles[g] = make_double2(std::cos(0.5 * th), std::sin(0.5 * th));
+        }
+    SweepPlan fplan, rplan;
+    SweepTables ftab, rtab;
     int rc = QS_OK;
     AJ_CHECK(cudaMallocAsync((void**)&blob, total, s), "adjoint buffers");
     {
-        const double2* dcs = (const double2*)(blob + o_cs);
         void* lam = blob + o_lam;
+        void* psi = blob + o_psi;  // the register's own state is only read
         double* part = (double*)(blob + o_part);
         double* dres = (double*)(blob + o_res);
-        AJ_CHECK(cudaMemcpyAsync(blob + o_cs, cs.data(), cs.size() * 16, cudaMemcpyHostToDevice, s), "cs upload");
         if (nt)
             AJ_CHECK(cudaMemcpyAsync(blob + o_terms, ht.data(), nt * sizeof(PauliDev), cudaMemcpyHostToDevice, s),
                      "terms upload");
-        AJ_CHECK(cudaMemcpyAsync(blob + o_save, state, N * amp, cudaMemcpyDeviceToDevice, s), "save state");
         int* derr = reinterpret_cast<int*>(blob + o_err);  // raised by a forward tile kernel's bounded wait
         AJ_CHECK(cudaMemsetAsync(derr, 0, sizeof(int), s), "status flag");
         int herr = 0;
         // forward
-        if (tiled) {
+        if (df) {
+            AJ_CHECK(cudaMemcpyAsync(psi, state, N * amp, cudaMemcpyDeviceToDevice, s), "state copy");
             std::vector<OpDesc> fops(m);
             std::vector<double> rmat(8 * m);  // the rotations' matrices, in gate order
             for (size_t g = 0; g < m; g++) {
                 if (rot_slot[g] >= 0) {
-                    const std::vector<double> R = rotation_matrix(gates[g].kind, cs[g].x, cs[g].y);
+                    const std::vector<double> R = rotation_matrix(gates[g].kind, angles[g].x, angles[g].y);
                     std::copy(R.begin(), R.end(), rmat.begin() + 8 * g);
                     classify_gate(R.data(), 1, gates[g].targets, &fops[g]);
                 } else {
-                    fops[g] = std::move(fwd[g]);  // the tiled path reads fwd no further
+                    fops[g] = std::move(fwd[g]);
                 }
             }
-            if (prec == QS_PREC_C128 && arith == QS_ARITH_DF64 && n >= 18) {
+            if (n >= 18) {
                 // double-float dense blocks (3 qubits, the automatic width): the fastest complex128
                 // double-float form of a circuit of 1-qubit rotations and CNOTs at 11-qubit tiles (1.85x
                 // the stages at 20 qubits; below 18 qubits the smaller stage tiles win); the blocks are
@@ -864,69 +887,44 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
                     qg[g] = rot_slot[g] >= 0 ? qs_gate{1, gates[g].targets, rmat.data() + 8 * g}
                                              : qs_gate{gates[g].k, gates[g].targets, gates[g].matrix};
                 const qs_circuit_options fo{2, 0, 0, 0};
-                if ((rc = run_circuit(state, n, prec, arith, fops, qg.data(), fo, s, sms, msg, derr)) != QS_OK)
+                if ((rc = run_circuit(psi, n, prec, arith, fops, qg.data(), fo, s, sms, msg, derr)) != QS_OK)
                     goto done;
             } else {
-                // tiles as in the reverse sweep: below 18 (complex128) or 19 (complex64) qubits smaller
-                // than the default so that smaller states still spread over many blocks
-                const qs_circuit_options fo{1, 5, adj_tile_qubits(n, prec == QS_PREC_C64 ? 12 : 11), 0};
+                // tiles as in the reverse sweep: below 18 qubits smaller than the default so that smaller
+                // states still spread over many blocks
+                const qs_circuit_options fo{1, 5, adj_tile_qubits(n, 11), 0};
                 // queued without waiting: the reverse sweep is planned while the forward runs
-                if ((rc = run_circuit(state, n, prec, arith, fops, nullptr, fo, s, sms, msg, derr)) != QS_OK)
+                if ((rc = run_circuit(psi, n, prec, arith, fops, nullptr, fo, s, sms, msg, derr)) != QS_OK)
                     goto done;
             }
-        }
-        for (size_t g = 0; g < m && !tiled; g++) {
-            if (rot_slot[g] >= 0) {
-                if (prec == QS_PREC_C64)
-                    launch_rot<float2>(gates[g].kind, state, n, int(gates[g].targets[0]), dcs, int(g), 0, s, sms);
-                else
-                    launch_rot<double2>(gates[g].kind, state, n, int(gates[g].targets[0]), dcs, int(g), 0, s, sms);
-                AJ_CHECK(cudaGetLastError(), "rotation");
-            } else if ((rc = apply_op(state, n, prec, arith, fwd[g], s, sms, msg)) != QS_OK) {
+        } else {
+            plan_sweep(gates, m, angles.data(), rot_slot, nrot, fwd, n, tq, false, type, false, !unitary, &fplan);
+            if ((rc = upload_sweep(fplan, angles, 0, s, &ftab, msg)) != QS_OK) goto done;
+            if ((rc = run_sweep(fplan, ftab, state, psi, nullptr, n, prec, arith, false, rot_slot, part, pgrid, s, sms,
+                                msg)) != QS_OK)
                 goto done;
-            }
         }
         // lambda = H psi, E = Re<psi|lambda>
         if (prec == QS_PREC_C64)
-            launch_pauli_sum<float2>(state, lam, n, (const PauliDev*)(blob + o_terms), int(nt), pauli_df_ok(ht), s,
-                                     sms);
+            launch_pauli_sum<float2>(psi, lam, n, (const PauliDev*)(blob + o_terms), int(nt), pauli_df_ok(ht), s, sms);
         else
-            launch_pauli_sum<double2>(state, lam, n, (const PauliDev*)(blob + o_terms), int(nt), false, s, sms);
+            launch_pauli_sum<double2>(psi, lam, n, (const PauliDev*)(blob + o_terms), int(nt), false, s, sms);
         AJ_CHECK(cudaGetLastError(), "pauli sum");
-        if (inner_product(state, prec, lam, prec, n, s, sms, part + size_t(std::max(nrot, 1)) * pgrid, dres))
+        if (inner_product(psi, prec, lam, prec, n, s, sms, part + size_t(std::max(nrot, 1)) * pgrid, dres))
             AJ_CHECK(cudaGetLastError(), "energy");
         // reverse
-        if (tiled) {
-            rc = prec == QS_PREC_C64
-                     ? reverse_tiled<float2>(state, lam, n, prec, arith, gates, m, params, rot_slot, inv, part, pgrid,
-                                             s, sms, msg)
-                     : reverse_tiled<double2>(state, lam, n, prec, arith, gates, m, params, rot_slot, inv, part,
-                                              pgrid, s, sms, msg);
-            if (rc != QS_OK) goto done;
-        }
-        for (size_t gg = m; gg-- > 0 && !tiled;) {
-            if (rot_slot[gg] >= 0) {
-                double* p = part + size_t(rot_slot[gg]) * pgrid;
-                if (prec == QS_PREC_C64)
-                    launch_adj_rot<float2>(gates[gg].kind, state, lam, n, int(gates[gg].targets[0]), dcs, int(gg), p,
-                                           pgrid, s);
-                else
-                    launch_adj_rot<double2>(gates[gg].kind, state, lam, n, int(gates[gg].targets[0]), dcs, int(gg), p,
-                                            pgrid, s);
-                AJ_CHECK(cudaGetLastError(), "adjoint rotation");
-            } else {
-                if ((rc = apply_op(state, n, prec, arith, inv[gg], s, sms, msg)) != QS_OK) goto done;
-                if ((rc = apply_op(lam, n, prec, arith, inv[gg], s, sms, msg)) != QS_OK) goto done;
-            }
-        }
+        plan_sweep(gates, m, angles.data(), rot_slot, nrot, inv, n, tq, true, type, df, !unitary, &rplan);
+        if ((rc = upload_sweep(rplan, angles, 1, s, &rtab, msg)) != QS_OK) goto done;
+        if ((rc = run_sweep(rplan, rtab, nullptr, psi, lam, n, prec, arith, true, rot_slot, part, pgrid, s, sms, msg)) !=
+            QS_OK)
+            goto done;
         if (nrot) {
-            k_grad_final<<<nrot, kAT, 0, s>>>(part, pgrid, dres + 2);
+            k_grad_final<<<nrot, kAT, 0, s>>>(part, pgrid, rtab.weights, rtab.weight_at, dres + 2);
             note_launches(1);
             AJ_CHECK(cudaGetLastError(), "gradient reduction");
         }
         AJ_CHECK(cudaMemcpyAsync(res.data(), dres, res.size() * 8, cudaMemcpyDeviceToHost, s), "readback");
         AJ_CHECK(cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, s), "status readback");
-        AJ_CHECK(cudaMemcpyAsync(state, blob + o_save, N * amp, cudaMemcpyDeviceToDevice, s), "restore state");
         AJ_CHECK(cudaStreamSynchronize(s), "adjoint sync");
         if (herr) {
             *msg = "a tile kernel's bounded wait for its bulk copies gave up";
@@ -941,6 +939,9 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
         }
     }
 done:
+    if (rc != QS_OK) cudaStreamSynchronize(s);  // the staging buffers are free again
+    if (ftab.dev) cudaFreeAsync(ftab.dev, s);
+    if (rtab.dev) cudaFreeAsync(rtab.dev, s);
     if (blob) cudaFreeAsync(blob, s);
     return rc;
 }

@@ -13,8 +13,10 @@
 //
 // The whole pass (parameter upload, state reset, persistent kernel, partial reduction, result
 // download) is captured once in a CUDA graph; a run writes new parameters into pinned memory and
-// replays it. Complex128 batches with QS_ARITH_DF64 hold the tiles of stages made of rotations and
-// CNOTs as double-float values (FP32 pipe), with the inner products accumulated in FP64.
+// replays it. A stage runs as a pass program of qs_sweep.cuh (complex64 tiles, or complex128 ones in
+// fixed point; in FP64 where a fixed gate is not unitary). Complex128 batches with QS_ARITH_DF64 hold the
+// tiles of stages made of rotations and CNOTs as double-float values (FP32 pipe), one gate after another,
+// with the inner products accumulated in FP64.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,6 +34,8 @@
 #include "qs_kernels.h"
 #include "qs_reduce.cuh"
 #include "qs_rot.cuh"
+#include "qs_sweep.cuh"
+#include "qs_sweep.h"
 #include "qs_tile.h"
 #include "qs_tma.cuh"
 
@@ -39,7 +43,6 @@ namespace qs {
 namespace {
 
 constexpr int kBT = 256;
-constexpr int kFix1 = 16;  // fixed dense 1-qubit gate
 constexpr int kCnot = 17;  // CNOT
 constexpr int kBTileMax = 11;  // tile qubits
 constexpr int kBMaxRot = kMaxStageOps;  // rotations per stage
@@ -54,14 +57,14 @@ struct BCirc {
 };
 
 struct BStage {
-    int op_off, nops, nrot, df;  // df: double-float tiles
-    int L, H, pad0, pad1;
+    int op_off, nops, nrot, df;  // df: double-float tiles, gates op_off .. op_off + nops
+    int L, H, prog, pad;         // prog: the stage's program otherwise
     uint8_t pos[16];   // the tile's qubits, sorted (its base index skips them)
     uint8_t high[8];   // qubit of local bit L + b
 };
 
 struct BOp {
-    int kind;   // QS_GATE_RX / RY / RZ, kFix1, kCnot
+    int kind;   // QS_GATE_RX / RY / RZ, kCnot
     int tb;     // local target bit
     int cb;     // CNOT: local control bit, or -1
     int cglob;  // CNOT: control qubit outside the tile, or -1
@@ -69,7 +72,6 @@ struct BOp {
     int rslot;  // rotation: circuit-level slot
     int lrot;   // rotation: stage-local slot
     int pad;
-    double m[8];  // kFix1: the 2x2 matrix (forward); its adjoint is formed on the fly
 };
 
 struct BPauli {
@@ -98,21 +100,6 @@ struct St<float2> {
     static __device__ __forceinline__ float2 from(double2 v) { return make_float2(float(v.x), float(v.y)); }
 };
 
-// y = M x for a 2x2 complex matrix (adjoint: M^H).
-__device__ __forceinline__ void mat2(const double* m, bool adj, double2& a, double2& b) {
-    double u[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) u[i] = m[i];
-    if (adj) {  // (M^H)_{rc} = conj(M_{cr})
-        const double t[8] = {u[0], -u[1], u[4], -u[5], u[2], -u[3], u[6], -u[7]};
-#pragma unroll
-        for (int i = 0; i < 8; i++) u[i] = t[i];
-    }
-    const double2 x = a, y = b;
-    a = make_double2(u[0] * x.x - u[1] * x.y + u[2] * y.x - u[3] * y.y, u[0] * x.y + u[1] * x.x + u[2] * y.y + u[3] * y.x);
-    b = make_double2(u[4] * x.x - u[5] * x.y + u[6] * y.x - u[7] * y.y, u[4] * x.y + u[5] * x.x + u[6] * y.y + u[7] * y.x);
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kBT) k_batch_reset(const BCirc* __restrict__ circs) {
     const BCirc C = circs[blockIdx.y];
@@ -126,36 +113,8 @@ __device__ __forceinline__ uint32_t pair_index(uint32_t p, int tb) {
     return ((p >> tb) << (tb + 1)) | (p & ((1u << tb) - 1u));
 }
 
-// One gate of a stage on the tile(s) in shared memory. fwd: psi only; reverse: psi and lambda, with
-// a rotation's inner-product term accumulated (before it is un-applied) into acc.
-template <typename T, int AXIS, typename R = decltype(T().x)>
-__device__ __forceinline__ auto tile_rot(T* sp, T* sl, uint32_t half, int tb, R c, R sn, bool fwd) {
-    const R cc = c, ss = fwd ? sn : -sn;
-    double acc = 0.0;
-    DfAcc facc;  // complex64: compensated pair sums, reduced over the warp as a float pair
-    for (uint32_t p = threadIdx.x; p < half; p += kBT) {
-        const uint32_t i0 = pair_index(p, tb), i1 = i0 | (1u << tb);
-        T a = sp[i0], b = sp[i1];
-        if (!fwd) {
-            T l0 = sl[i0], l1 = sl[i1];
-            if constexpr (sizeof(R) == 8)
-                acc += im_term<AXIS>(l0, l1, a, b);
-            else
-                im_term_acc<AXIS>(facc, l0, l1, a, b);
-            rot_pair<AXIS>(cc, ss, l0.x, l0.y, l1.x, l1.y);
-            sl[i0] = l0;
-            sl[i1] = l1;
-        }
-        rot_pair<AXIS>(cc, ss, a.x, a.y, b.x, b.y);
-        sp[i0] = a;
-        sp[i1] = b;
-    }
-    if constexpr (sizeof(R) == 4)
-        return facc;
-    else
-        return acc;
-}
-
+// One gate of a double-float stage on the tile(s) in shared memory. fwd: psi only; reverse: psi and lambda,
+// with a rotation's inner-product term accumulated (before it is un-applied).
 template <int AXIS>
 __device__ __forceinline__ DfAcc tile_rot_df(float4* sp, float4* sl, uint32_t half, int tb, double c, double sn,
                                               bool fwd) {
@@ -192,33 +151,139 @@ __device__ __forceinline__ void tile_cnot(E* s, uint32_t half, int tb, int cb) {
     }
 }
 
-template <typename T>
-__device__ __forceinline__ void tile_fix1(T* s, uint32_t half, int tb, const double* m, bool adj) {
-    for (uint32_t p = threadIdx.x; p < half; p += kBT) {
-        const uint32_t i0 = pair_index(p, tb), i1 = i0 | (1u << tb);
-        double2 a = St<T>::d(s[i0]), b = St<T>::d(s[i1]);
-        mat2(m, adj, a, b);
-        s[i0] = St<T>::from(a);
-        s[i1] = St<T>::from(b);
+// Tiles [first, first + count) of a double-float stage.
+__device__ __noinline__ void batch_df(const BCirc& C, const BStage& S, const BOp* __restrict__ ops,
+                                      const double2* __restrict__ cs, uint64_t first, uint64_t count, bool fwd,
+                                      unsigned char* smem, double* __restrict__ partials, uint32_t j) {
+    float4* fp = reinterpret_cast<float4*>(smem);
+    float4* fl = fp + (1u << kBTileMax);
+    uint64_t* rowoff = reinterpret_cast<uint64_t*>(fl + (1u << kBTileMax));
+    double* sacc = reinterpret_cast<double*>(rowoff + (1 << kTileMaxHigh));  // [kBMaxRot][8 warps]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double2* psi = reinterpret_cast<double2*>(C.psi);
+    double2* lam = reinterpret_cast<double2*>(C.lam);
+    const uint32_t tsize = 1u << C.T, half = tsize >> 1, lmask = (1u << S.L) - 1u;
+    for (int r = threadIdx.x; r < (1 << S.H); r += kBT) {
+        uint64_t o = 0;
+        for (int b = 0; b < S.H; b++)
+            if (r >> b & 1) o |= 1ull << S.high[b];
+        rowoff[r] = o;
     }
+    if (!fwd)
+        for (int r = threadIdx.x; r < S.nrot * (kBT / 32); r += kBT) sacc[r] = 0.0;
+    __syncthreads();
+    for (uint64_t t = first; t < first + count; t++) {
+        uint64_t base = t;  // insert the tile's qubits as zero bits
+        for (int k = 0; k < C.T; k++) {
+            const int q = S.pos[k];
+            base = ((base >> q) << (q + 1)) | (base & ((1ull << q) - 1ull));
+        }
+        auto split = [](double2 v) {
+            float4 f;
+            df_split(v.x, f.x, f.y);
+            df_split(v.y, f.z, f.w);
+            return f;
+        };
+        auto join = [](float4 f) {
+            return make_double2(__dadd_rn(df_f2d(f.x), df_f2d(f.y)), __dadd_rn(df_f2d(f.z), df_f2d(f.w)));
+        };
+        for (uint32_t i = threadIdx.x; i < tsize; i += kBT) {
+            const uint64_t g = base + rowoff[i >> S.L] + (i & lmask);
+            fp[i] = split(__ldcg(psi + g));
+            if (!fwd) fl[i] = split(__ldcg(lam + g));
+        }
+        __syncthreads();
+        for (int o = 0; o < S.nops; o++) {
+            const BOp op = ops[S.op_off + o];
+            if (op.kind == kCnot) {
+                if (op.cglob < 0 || ((base >> op.cglob) & 1ull)) {  // outside control: the whole tile
+                    tile_cnot(fp, half, op.tb, op.cb);
+                    if (!fwd) tile_cnot(fl, half, op.tb, op.cb);
+                }
+            } else {
+                const double2 t2 = cs[op.cs];
+                DfAcc f;
+                if (op.kind == QS_GATE_RX) f = tile_rot_df<QS_GATE_RX>(fp, fl, half, op.tb, t2.x, t2.y, fwd);
+                else if (op.kind == QS_GATE_RY) f = tile_rot_df<QS_GATE_RY>(fp, fl, half, op.tb, t2.x, t2.y, fwd);
+                else f = tile_rot_df<QS_GATE_RZ>(fp, fl, half, op.tb, t2.x, t2.y, fwd);
+                if (!fwd) {  // float pairs over the warp, one FP64 rejoin
+                    f.warp_reduce();
+                    if (lane == 0) sacc[op.lrot * (kBT / 32) + warp] += __dadd_rn(df_f2d(f.s), df_f2d(f.c));
+                }
+            }
+            __syncthreads();
+        }
+        for (uint32_t i = threadIdx.x; i < tsize; i += kBT) {
+            const uint64_t g = base + rowoff[i >> S.L] + (i & lmask);
+            __stcg(psi + g, join(fp[i]));
+            if (!fwd) __stcg(lam + g, join(fl[i]));
+        }
+        __syncthreads();
+    }
+    if (!fwd)  // this item's partial of every rotation of the stage
+        for (int o = threadIdx.x; o < S.nops; o += kBT) {
+            const BOp op = ops[S.op_off + o];
+            if (op.kind == kCnot) continue;
+            double v = 0.0;
+            for (int w = 0; w < kBT / 32; w++) v += sacc[op.lrot * (kBT / 32) + w];
+            partials[C.rpart_off + (size_t(op.rslot) << C.ncht_log) + j] = v;
+        }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kBT) k_batch(const BCirc* __restrict__ circs, const BStage* __restrict__ stages,
-                                               const BOp* __restrict__ ops, const BPauli* __restrict__ terms,
-                                               const double2* __restrict__ cs, const uint32_t* __restrict__ seg_first,
-                                               const int4* __restrict__ segs, int nsegs, uint32_t nitems,
-                                               unsigned int* __restrict__ counters, double* __restrict__ partials,
-                                               unsigned int* __restrict__ ticket, int* __restrict__ err) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* sp = reinterpret_cast<T*>(smem_raw);
+// The sweep programs' tables, and what a run fills in from its parameters.
+struct BSweep {
+    const SweepRange* ranges;
+    const SweepPass* passes;
+    const TileOp* fixed;
+    const SweepCoef* coefs;
+    const double* sigmas;
+    const int* rslot;  // circuit-level slot of each program rotation
+};
+
+// Tiles [j * tpi, (j + 1) * tpi) of a stage through its program.
+template <typename T, int RB, bool REV>
+__device__ void batch_sweep(const BCirc& C, const BStage& S, const BSweep& W, uint64_t first, uint64_t count, bool store,
+                            unsigned char* smem, double* __restrict__ partials, uint32_t j) {
+    using G = typename Sw<T>::Glob;
+    const SweepRange R = W.ranges[S.prog];
+    T* sp = reinterpret_cast<T*>(smem);
     T* sl = sp + (1u << kBTileMax);
-    uint64_t* rowoff = reinterpret_cast<uint64_t*>(sl + (1u << kBTileMax));
-    double* sacc = reinterpret_cast<double*>(rowoff + 64);  // [kBMaxRot][8 warps]
+    const SweepSide<T> side(reinterpret_cast<unsigned char*>(sl + (1u << kBTileMax)), R.npass, R.nrot, R.ndiag, REV);
+    const SweepTile t{C.T, S.L, R.npass, R.nrot, R.ndiag, store, W.sigmas[S.prog]};
+    for (int r = threadIdx.x; r < (1 << S.H); r += kBT) {
+        uint64_t o = 0;
+        for (int b = 0; b < S.H; b++)
+            if (r >> b & 1) o |= 1ull << S.high[b];
+        side.rowoff[r] = o;
+    }
+    sw_begin<T>(side, W.passes + R.pass0, R.npass, W.coefs + R.coef0, R.nrot, C.T, REV, t.sigma, kBT);
+    for (uint64_t k = first; k < first + count; k++) {
+        uint64_t base = k;  // insert the tile's qubits as zero bits
+        for (int i = 0; i < C.T; i++) {
+            const int q = S.pos[i];
+            base = ((base >> q) << (q + 1)) | (base & ((1ull << q) - 1ull));
+        }
+        G* psi = reinterpret_cast<G*>(C.psi);
+        sw_tile<T, RB, REV, true>(psi, psi, reinterpret_cast<G*>(C.lam), base, t, sp, sl, side, W.fixed, kBT);
+    }
+    if (REV)  // this item's partial of every rotation of the stage
+        for (int r = threadIdx.x; r < R.nrot; r += kBT)
+            partials[C.rpart_off + (size_t(W.rslot[R.coef0 + r]) << C.ncht_log) + j] = sw_total<T>(side, r, kBT);
+}
+
+// T: the tile type; DF: stages marked df run as double-float tiles.
+template <typename TT, bool DF>
+__global__ void __launch_bounds__(kBT, sizeof(TT) == 16 ? 2 : 3)
+    k_batch(const BCirc* __restrict__ circs, const BStage* __restrict__ stages, const BOp* __restrict__ ops,
+            const BPauli* __restrict__ terms, const double2* __restrict__ cs, const __grid_constant__ BSweep sweep,
+            const uint32_t* __restrict__ seg_first, const int4* __restrict__ segs, int nsegs, uint32_t nitems,
+            unsigned int* __restrict__ counters, double* __restrict__ partials, unsigned int* __restrict__ ticket,
+            int* __restrict__ err) {
+    using T = typename Sw<TT>::Glob;
+    static_assert(!DF || sizeof(T) == 16, "double-float tiles hold complex128 states");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_item;
     __shared__ int s_seg, s_stop;
-    __shared__ float2 s_csf[kBMaxRot];  // complex64: the stage's rotation (cos, sin) rounded to float
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (;;) {
         if (threadIdx.x == 0) {
             s_item = atomicAdd(ticket, 1u);
@@ -307,135 +372,30 @@ __global__ void __launch_bounds__(kBT) k_batch(const BCirc* __restrict__ circs, 
         } else {  // a tiled stage: tiles [j * tpi, (j + 1) * tpi)
             const bool fwd = s < C.nfwd;
             const BStage S = stages[C.stage_off + (fwd ? s : s - 1)];
-            const uint32_t tsize = 1u << C.T, half = tsize >> 1;
             const uint64_t tpi = 1ull << (C.n - C.T - C.ncht_log);
-            const uint32_t lmask = (1u << S.L) - 1u;
-            for (int r = threadIdx.x; r < (1 << S.H); r += kBT) {
-                uint64_t o = 0;
-                for (int b = 0; b < S.H; b++)
-                    if (r >> b & 1) o |= 1ull << S.high[b];
-                rowoff[r] = o;
+            bool done = false;
+            if constexpr (DF) {
+                if (S.df) {
+                    batch_df(C, S, ops, cs, uint64_t(j) * tpi, tpi, fwd, smem_raw, partials, j);
+                    done = true;
+                }
             }
-            if (!fwd)
-                for (int r = threadIdx.x; r < S.nrot * (kBT / 32); r += kBT) sacc[r] = 0.0;
-            if constexpr (sizeof(T) == 8)  // one conversion per rotation per item, not per thread and tile
-                for (int o = threadIdx.x; o < S.nops; o += kBT) {
-                    const BOp op = ops[S.op_off + o];
-                    if (op.kind != kCnot && op.kind != kFix1) {
-                        const double2 t2 = cs[op.cs];
-                        s_csf[o] = make_float2(float(t2.x), float(t2.y));
-                    }
+            if (!done) {
+                const bool store = s + 1 < C.nsteps;  // nothing reads the vectors after the last step
+                const int rb = sw_register_bits(C.T);
+#define QS_B(RB)                                                                                                  \
+    if (fwd)                                                                                                      \
+        batch_sweep<TT, RB, false>(C, S, sweep, uint64_t(j) * tpi, tpi, store, smem_raw, partials, j);            \
+    else                                                                                                          \
+        batch_sweep<TT, RB, true>(C, S, sweep, uint64_t(j) * tpi, tpi, store, smem_raw, partials, j)
+                if (rb == 3) {
+                    QS_B(3);
+                } else if (rb == 2) {
+                    QS_B(2);
+                } else {
+                    QS_B(1);
                 }
-            __syncthreads();
-            float4* fp = reinterpret_cast<float4*>(sp);
-            float4* fl = reinterpret_cast<float4*>(sl);
-            const bool df = sizeof(T) == 16 && S.df;
-            for (uint64_t t = uint64_t(j) * tpi; t < uint64_t(j + 1) * tpi; t++) {
-                uint64_t base = t;  // insert the tile's qubits as zero bits
-                for (int k = 0; k < C.T; k++) {
-                    const int q = S.pos[k];
-                    base = ((base >> q) << (q + 1)) | (base & ((1ull << q) - 1ull));
-                }
-                for (uint32_t i = threadIdx.x; i < tsize; i += kBT) {
-                    const uint64_t g = base + rowoff[i >> S.L] + (i & lmask);
-                    const T v = St<T>::ld(psi, g);
-                    T w = v;
-                    if (!fwd) w = St<T>::ld(lam, g);
-                    if (df) {
-                        const double2 dv = St<T>::d(v), dw = St<T>::d(w);
-                        float4 f;
-                        df_split(dv.x, f.x, f.y);
-                        df_split(dv.y, f.z, f.w);
-                        fp[i] = f;
-                        if (!fwd) {
-                            df_split(dw.x, f.x, f.y);
-                            df_split(dw.y, f.z, f.w);
-                            fl[i] = f;
-                        }
-                    } else {
-                        sp[i] = v;
-                        if (!fwd) sl[i] = w;
-                    }
-                }
-                __syncthreads();
-                for (int o = 0; o < S.nops; o++) {
-                    const BOp op = ops[S.op_off + o];
-                    if (op.kind == kCnot) {
-                        if (op.cglob < 0 || ((base >> op.cglob) & 1ull)) {  // outside control: the whole tile
-                            if (df) {
-                                tile_cnot(fp, half, op.tb, op.cb);
-                                if (!fwd) tile_cnot(fl, half, op.tb, op.cb);
-                            } else {
-                                tile_cnot(sp, half, op.tb, op.cb);
-                                if (!fwd) tile_cnot(sl, half, op.tb, op.cb);
-                            }
-                        }
-                    } else if (op.kind == kFix1) {  // never in double-float stages
-                        if constexpr (true) {
-                            tile_fix1(sp, half, op.tb, op.m, !fwd);
-                            if (!fwd) tile_fix1(sl, half, op.tb, op.m, true);
-                        }
-                    } else if constexpr (sizeof(T) == 8) {  // complex64
-                        const float2 t2 = s_csf[o];
-                        DfAcc f;
-                        if (op.kind == QS_GATE_RX) f = tile_rot<T, QS_GATE_RX>(sp, sl, half, op.tb, t2.x, t2.y, fwd);
-                        else if (op.kind == QS_GATE_RY) f = tile_rot<T, QS_GATE_RY>(sp, sl, half, op.tb, t2.x, t2.y, fwd);
-                        else f = tile_rot<T, QS_GATE_RZ>(sp, sl, half, op.tb, t2.x, t2.y, fwd);
-                        if (!fwd) {  // the warp's float pairs reduced on the FP32 pipe, one FP64 rejoin
-                            f.warp_reduce();
-                            if (lane == 0) sacc[op.lrot * (kBT / 32) + warp] += __dadd_rn(df_f2d(f.s), df_f2d(f.c));
-                        }
-                    } else {
-                        const double2 t2 = cs[op.cs];
-                        double v;
-                        if (df) {
-                            DfAcc f;
-                            if (op.kind == QS_GATE_RX) f = tile_rot_df<QS_GATE_RX>(fp, fl, half, op.tb, t2.x, t2.y, fwd);
-                            else if (op.kind == QS_GATE_RY) f = tile_rot_df<QS_GATE_RY>(fp, fl, half, op.tb, t2.x, t2.y, fwd);
-                            else f = tile_rot_df<QS_GATE_RZ>(fp, fl, half, op.tb, t2.x, t2.y, fwd);
-                            v = 0.0;
-                            if (!fwd) {  // float pairs over the warp, one FP64 rejoin
-                                f.warp_reduce();
-                                v = __dadd_rn(df_f2d(f.s), df_f2d(f.c));
-                            }
-                        } else {
-                            if (op.kind == QS_GATE_RX) v = tile_rot<T, QS_GATE_RX>(sp, sl, half, op.tb, t2.x, t2.y, fwd);
-                            else if (op.kind == QS_GATE_RY) v = tile_rot<T, QS_GATE_RY>(sp, sl, half, op.tb, t2.x, t2.y, fwd);
-                            else v = tile_rot<T, QS_GATE_RZ>(sp, sl, half, op.tb, t2.x, t2.y, fwd);
-                        }
-                        if (!fwd) {
-                            if (!df) v = rd_warp_sum(v);
-                            if (lane == 0) sacc[op.lrot * (kBT / 32) + warp] += v;
-                        }
-                    }
-                    __syncthreads();
-                }
-                for (uint32_t i = threadIdx.x; i < tsize; i += kBT) {
-                    const uint64_t g = base + rowoff[i >> S.L] + (i & lmask);
-                    if (df) {
-                        const float4 f = fp[i];
-                        St<T>::st(psi, g, St<T>::from(make_double2(__dadd_rn(df_f2d(f.x), df_f2d(f.y)),
-                                                                   __dadd_rn(df_f2d(f.z), df_f2d(f.w)))));
-                        if (!fwd) {
-                            const float4 h = fl[i];
-                            St<T>::st(lam, g, St<T>::from(make_double2(__dadd_rn(df_f2d(h.x), df_f2d(h.y)),
-                                                                       __dadd_rn(df_f2d(h.z), df_f2d(h.w)))));
-                        }
-                    } else {
-                        St<T>::st(psi, g, sp[i]);
-                        if (!fwd) St<T>::st(lam, g, sl[i]);
-                    }
-                }
-                __syncthreads();
-            }
-            if (!fwd) {  // this item's partial of every rotation of the stage
-                for (int o = threadIdx.x; o < S.nops; o += kBT) {
-                    const BOp op = ops[S.op_off + o];
-                    if (op.kind == kCnot || op.kind == kFix1) continue;
-                    double v = 0.0;
-                    for (int w = 0; w < kBT / 32; w++) v += sacc[op.lrot * (kBT / 32) + w];
-                    partials[C.rpart_off + size_t(op.rslot << C.ncht_log) + j] = v;
-                }
+#undef QS_B
             }
         }
         __threadfence();
@@ -444,15 +404,16 @@ __global__ void __launch_bounds__(kBT) k_batch(const BCirc* __restrict__ circs, 
     }
 }
 
-// res[r] = sum of partials[rtab[r].x .. + rtab[r].y), in a fixed order.
+// res[r] = sum of partials[rtab[r].x .. + rtab[r].y), in a fixed order, times weights[wtab[r]] (wtab[r] < 0: 1).
 __global__ void __launch_bounds__(kBT) k_batch_reduce(const double* __restrict__ partials, const int2* __restrict__ rtab,
+                                                      const int* __restrict__ wtab, const double* __restrict__ weights,
                                                       int nres, double* __restrict__ res) {
     for (int r = blockIdx.x; r < nres; r += gridDim.x) {
         const int2 t = rtab[r];
         double a = 0.0, b = 0.0;
         for (int i = threadIdx.x; i < t.y; i += kBT) a += partials[t.x + i];
         rd_block_sum2<kBT>(a, b);
-        if (threadIdx.x == 0) res[r] = a;
+        if (threadIdx.x == 0) res[r] = wtab[r] < 0 ? a : a * weights[wtab[r]];
     }
 }
 
@@ -474,6 +435,17 @@ struct qs_batch {
     double* dpart = nullptr;
     double* dres = nullptr;
     int2* drtab = nullptr;
+    int* dwtab = nullptr;        // per result: coefficient whose weight it takes, -1: none
+    qs::SweepRange* dranges = nullptr;
+    qs::SweepPass* dpasses = nullptr;
+    qs::SweepRot* drots = nullptr;
+    qs::TileOp* dfixed = nullptr;
+    int* drslot = nullptr;
+    qs::SweepCoef* dcoefs = nullptr;
+    double* dweights = nullptr;
+    double* dsigmas = nullptr;
+    int nprogs = 0;
+    const void* kernel = nullptr;  // the k_batch instance
     int* derr = nullptr;
     unsigned int* dticket = nullptr;
     double2* hcs = nullptr;   // pinned: (cos, sin) of theta/2 per rotation
@@ -542,8 +514,13 @@ void build_schedule(qs_batch* b, std::vector<uint32_t>* first, std::vector<int4>
 }
 
 size_t batch_smem(int prec) {
-    const size_t amp = prec == QS_PREC_C64 ? 8 : 16;
-    return 2 * (amp << kBTileMax) + 64 * 8 + size_t(kBMaxRot) * (kBT / 32) * 8;
+    if (prec == QS_PREC_C64)
+        return 2 * (sizeof(float2) << kBTileMax) +
+               SweepSide<float2>::bytes(kSwMaxPass, kSwMaxRot, kSwMaxDiag, true, kTileMaxHigh);
+    const size_t side = std::max({SweepSide<FxC>::bytes(kSwMaxPass, kSwMaxRot, kSwMaxDiag, true, kTileMaxHigh),
+                                  SweepSide<double2>::bytes(kSwMaxPass, kSwMaxRot, kSwMaxDiag, true, kTileMaxHigh),
+                                  (size_t(8) << kTileMaxHigh) + size_t(kBMaxRot) * (kBT / 32) * 8});
+    return 2 * (sizeof(double2) << kBTileMax) + side;
 }
 
 cudaError_t capture(qs_batch* b) {
@@ -557,18 +534,27 @@ cudaError_t capture(qs_batch* b) {
     cudaMemsetAsync(b->dticket, 0, sizeof(unsigned int), s);
     cudaMemsetAsync(b->derr, 0, sizeof(int), s);
     const dim3 rg(uint32_t(b->sms * 2), uint32_t(b->count));
-    if (b->prec == QS_PREC_C64) {
+    if (b->nprogs)
+        k_sweep_coefs<<<b->nprogs, 64, 0, s>>>(b->dranges, b->dpasses, b->drots, b->dcs, b->dcoefs, b->dweights,
+                                              b->dsigmas);
+    const BSweep sw{b->dranges, b->dpasses, b->dfixed, b->dcoefs, b->dsigmas, b->drslot};
+    if (b->prec == QS_PREC_C64)
         k_batch_reset<float2><<<rg, kBT, 0, s>>>(b->dcirc);
-        k_batch<float2><<<b->sms * b->ctas, kBT, b->smem, s>>>(b->dcirc, b->dstages, b->dops, b->dterms, b->dcs,
-                                                               b->dseg_first, b->dsegs, b->nsegs, b->nitems,
-                                                               b->dcounters, b->dpart, b->dticket, b->derr);
-    } else {
+    else
         k_batch_reset<double2><<<rg, kBT, 0, s>>>(b->dcirc);
-        k_batch<double2><<<b->sms * b->ctas, kBT, b->smem, s>>>(b->dcirc, b->dstages, b->dops, b->dterms, b->dcs,
-                                                                b->dseg_first, b->dsegs, b->nsegs, b->nitems,
-                                                                b->dcounters, b->dpart, b->dticket, b->derr);
-    }
-    k_batch_reduce<<<std::min(b->nres, b->sms * 8), kBT, 0, s>>>(b->dpart, b->drtab, b->nres, b->dres);
+#define QS_BATCH(T, DF)                                                                                              \
+    if (b->kernel == reinterpret_cast<const void*>(k_batch<T, DF>))                                                  \
+    k_batch<T, DF><<<b->sms * b->ctas, kBT, b->smem, s>>>(b->dcirc, b->dstages, b->dops, b->dterms, b->dcs, sw,      \
+                                                          b->dseg_first, b->dsegs, b->nsegs, b->nitems, b->dcounters, \
+                                                          b->dpart, b->dticket, b->derr)
+    QS_BATCH(float2, false);
+    QS_BATCH(FxC, false);
+    QS_BATCH(double2, false);
+    QS_BATCH(FxC, true);
+    QS_BATCH(double2, true);
+#undef QS_BATCH
+    k_batch_reduce<<<std::min(b->nres, b->sms * 8), kBT, 0, s>>>(b->dpart, b->drtab, b->dwtab, b->dweights, b->nres,
+                                                                b->dres);
     cudaMemcpyAsync(b->hres, b->dres, sizeof(double) * b->nres, cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(b->herr, b->derr, sizeof(int), cudaMemcpyDeviceToHost, s);
     e = cudaStreamEndCapture(s, &b->graph);
@@ -592,24 +578,47 @@ OpDesc plan_desc(const qs_param_gate& G, bool cnot) {
     return d;
 }
 
-// Stages of one circuit (forward gates, then the reverse sweep) into the stage and op tables.
-void plan_circuit(const qs_batch_circuit& q, int T, bool df_ok, BCirc* C, const std::vector<int>& cs_of,
-                  const std::vector<int>& rslot_of, std::vector<BStage>* stages, std::vector<BOp>* ops) {
-    const int n = int(q.n), L = std::min(5, T);
+// The tables plan_circuit fills.
+struct BTables {
+    std::vector<BStage> stages;
+    std::vector<BOp> ops;
+    std::vector<SweepRange> ranges;
+    std::vector<SweepPass> passes;
+    std::vector<SweepRot> rots;
+    std::vector<TileOp> fixed;
+    std::vector<int> rslot;
+    std::vector<int> wtab;  // per rotation slot of the circuit being planned
+};
+
+// Stages of one circuit (forward gates, then the reverse sweep) into the tables. Double-float stages hold
+// rotations and CNOTs; the others become programs.
+void plan_circuit(const qs_batch_circuit& q, int T, int prec, bool df_ok, bool unitary, BCirc* C,
+                  const std::vector<int>& cs_of, const std::vector<int>& rslot_of, BTables* tb) {
+    const int n = int(q.n);
+    const bool fixed_point = prec == QS_PREC_C128 && unitary;
+    const int L = std::min(T, df_ok || !unitary ? 5 : prec == QS_PREC_C64 ? 4 : 3);  // rows of 128 bytes
     std::vector<char> cnot(q.m);
-    std::vector<OpDesc> fw;
-    for (size_t g = 0; g < q.m; g++) {
-        cnot[g] = q.gates[g].kind == QS_GATE_FIXED && q.gates[g].k == 2;
-        fw.push_back(plan_desc(q.gates[g], cnot[g]));
-    }
+    for (size_t g = 0; g < q.m; g++) cnot[g] = q.gates[g].kind == QS_GATE_FIXED && q.gates[g].k == 2;
     auto emit = [&](const std::vector<int>& order, bool fwd) {
-        std::vector<OpDesc> list;
-        for (int g : order) list.push_back(fw[g]);
-        const std::vector<TileStage> st = plan_tiles(list, n, T, L, false);
+        std::vector<OpDesc> list, fixed(q.m);
+        for (int g : order) {
+            const qs_param_gate& G = q.gates[g];
+            list.push_back(plan_desc(G, cnot[g]));
+            if (G.kind != QS_GATE_FIXED) continue;
+            if (cnot[g] || fwd) {
+                classify_gate(G.matrix, G.k, G.targets, &fixed[g]);
+            } else {  // the adjoint of a 1-qubit gate
+                const double* m = G.matrix;
+                const double h[8] = {m[0], -m[1], m[4], -m[5], m[2], -m[3], m[6], -m[7]};
+                classify_gate(h, 1, G.targets, &fixed[g]);
+            }
+        }
+        const std::vector<TileStage> st = plan_tiles(list, n, T, L, false, df_ok || !unitary ? kMaxStageOps : kSwMaxRot);
         int count = 0;
         for (const TileStage& S : st) {
             BStage B{};
-            B.op_off = int(ops->size());
+            B.prog = -1;
+            B.op_off = int(tb->ops.size());
             B.L = S.L;
             B.H = int(S.high.size());
             std::vector<int> qpos;
@@ -624,40 +633,65 @@ void plan_circuit(const qs_batch_circuit& q, int T, bool df_ok, BCirc* C, const 
                     if (S.high[i] == qb) return S.L + i;
                 return -1;
             };
-            B.df = df_ok ? 1 : 0;
-            for (int idx : S.ops) {
-                const int g = order[idx];
-                const qs_param_gate& G = q.gates[g];
-                BOp o{};
-                o.cb = o.cglob = -1;
-                if (cnot[g]) {  // CNOT's matrix: targets[1] = 1 swaps the rows of targets[0]
-                    o.kind = kCnot;
+            bool moves = df_ok;
+            for (int idx : S.ops) moves = moves && (q.gates[order[idx]].kind != QS_GATE_FIXED || cnot[order[idx]]);
+            if (moves) {
+                B.df = 1;
+                for (int idx : S.ops) {
+                    const int g = order[idx];
+                    const qs_param_gate& G = q.gates[g];
+                    BOp o{};
+                    o.cb = o.cglob = -1;
                     o.tb = local(int(G.targets[0]));
-                    o.cb = local(int(G.targets[1]));
-                    if (o.cb < 0) o.cglob = int(G.targets[1]);
-                } else if (G.kind == QS_GATE_FIXED) {
-                    o.kind = kFix1;
-                    o.tb = local(int(G.targets[0]));
-                    for (int i = 0; i < 8; i++) o.m[i] = G.matrix[i];
-                    B.df = 0;  // double-float stages take rotations and CNOTs
-                } else {
-                    o.kind = G.kind;
-                    o.tb = local(int(G.targets[0]));
-                    o.cs = cs_of[g];
-                    o.rslot = rslot_of[g];
-                    o.lrot = B.nrot++;
+                    if (cnot[g]) {  // CNOT's matrix: targets[1] = 1 swaps the rows of targets[0]
+                        o.kind = kCnot;
+                        o.cb = local(int(G.targets[1]));
+                        if (o.cb < 0) o.cglob = int(G.targets[1]);
+                    } else {
+                        o.kind = G.kind;
+                        o.cs = cs_of[g];
+                        o.rslot = rslot_of[g];
+                        o.lrot = B.nrot++;
+                    }
+                    tb->ops.push_back(o);
+                    B.nops++;
                 }
-                ops->push_back(o);
-                B.nops++;
+                tb->stages.push_back(B);
+                count++;
+                continue;
             }
-            stages->push_back(B);
-            count++;
+            std::vector<SweepGate> sg;
+            for (int idx : S.ops) {
+                SweepGate e;
+                e.gate = order[idx];
+                const qs_param_gate& G = q.gates[e.gate];
+                if (G.kind == QS_GATE_FIXED) {
+                    e.fixed = &fixed[e.gate];
+                } else {
+                    e.axis = G.kind;
+                    e.target = int(G.targets[0]);
+                }
+                sg.push_back(e);
+            }
+            for (const SweepProgram& p : build_sweep(sg, S, fixed_point, !fwd, !unitary, &tb->fixed)) {
+                B.prog = int(tb->ranges.size());
+                tb->ranges.push_back(SweepRange{int(tb->passes.size()), int(p.passes.size()), int(tb->rots.size()),
+                                                int(p.rots.size()), p.ndiag, !fixed_point, prec == QS_PREC_C64, 0});
+                for (int g : p.rots) {
+                    if (!fwd) tb->wtab[rslot_of[g]] = int(tb->rots.size());
+                    tb->rots.push_back(SweepRot{cs_of[g], q.gates[g].kind});
+                    tb->rslot.push_back(rslot_of[g]);
+                }
+                tb->passes.insert(tb->passes.end(), p.passes.begin(), p.passes.end());
+                tb->stages.push_back(B);
+                count++;
+            }
         }
         return count;
     };
     std::vector<int> order(q.m);
     for (size_t g = 0; g < q.m; g++) order[g] = int(g);
-    C->stage_off = int(stages->size());
+    C->stage_off = int(tb->stages.size());
     C->nfwd = emit(order, true);
     std::reverse(order.begin(), order.end());
     const int nrev = emit(order, false);
@@ -688,9 +722,17 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, dev);
     // ---- validate and plan
-    std::vector<BStage> stages;
-    std::vector<BOp> ops;
+    BTables tb;
     std::vector<BPauli> terms;
+    std::vector<int> wtab;
+    const bool df_ok = b->prec == QS_PREC_C128 && b->arith == QS_ARITH_DF64;
+    bool unitary = true;  // fixed-point tiles need gates that keep norms
+    for (size_t c = 0; c < count && unitary; c++)
+        for (size_t g = 0; g < circuits[c].m && circuits[c].gates && unitary; g++) {
+            const qs_param_gate& G = circuits[c].gates[g];
+            if (G.kind == QS_GATE_FIXED && G.k == 1 && G.matrix) unitary = is_unitary(G.matrix, 1);
+        }
+    const bool fixed_point = b->prec == QS_PREC_C128 && unitary;
     const size_t amp = b->prec == QS_PREC_C64 ? 8 : 16;
     size_t state_bytes = 0;
     int counters = 0;
@@ -745,8 +787,10 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
                              uint32_t(__builtin_popcountll(q.terms[t].x_mask & q.terms[t].z_mask) & 3), 0u});
         }
         C.nrot = int(rp.size());
-        plan_circuit(q, C.T, b->prec == QS_PREC_C128 && b->arith == QS_ARITH_DF64, &C, cs_of, rslot_of, &stages,
-                     &ops);
+        tb.wtab.assign(rp.size(), -1);
+        plan_circuit(q, C.T, b->prec, df_ok, unitary, &C, cs_of, rslot_of, &tb);
+        wtab.push_back(-1);  // the energy
+        wtab.insert(wtab.end(), tb.wtab.begin(), tb.wtab.end());
         C.counter_off = counters;
         counters += C.nsteps;
         b->rot_param.push_back(rp);
@@ -770,8 +814,15 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
     b->nres = int(rtab.size());
     // ---- arena
     const size_t o_circ = 0, o_stages = o_circ + al(sizeof(BCirc) * count + 1),
-                 o_ops = o_stages + al(sizeof(BStage) * stages.size() + 1),
-                 o_terms = o_ops + al(sizeof(BOp) * ops.size() + 1),
+                 o_ops = o_stages + al(sizeof(BStage) * tb.stages.size() + 1),
+                 o_range = o_ops + al(sizeof(BOp) * tb.ops.size() + 1),
+                 o_pass = o_range + al(sizeof(SweepRange) * tb.ranges.size() + 1),
+                 o_rot = o_pass + al(sizeof(SweepPass) * tb.passes.size() + 1),
+                 o_fix = o_rot + al(sizeof(SweepRot) * tb.rots.size() + 1),
+                 o_rslot = o_fix + al(sizeof(TileOp) * tb.fixed.size() + 1),
+                 o_coef = o_rslot + al(4 * tb.rslot.size() + 1), o_wt = o_coef + al(sizeof(SweepCoef) * tb.rots.size() + 1),
+                 o_sig = o_wt + al(8 * tb.rots.size() + 8), o_wtab = o_sig + al(8 * tb.ranges.size() + 8),
+                 o_terms = o_wtab + al(4 * wtab.size() + 4),
                  o_cs = o_terms + al(sizeof(BPauli) * terms.size() + 1), o_first = o_cs + al(16 * (size_t(b->ncs) + 1)),
                  o_segs = o_first + al(4 * max_segs + 4), o_ctr = o_segs + al(sizeof(int4) * max_segs + 16),
                  o_part = o_ctr + al(4 * size_t(counters) + 4), o_res = o_part + al(8 * part_max + 8),
@@ -784,10 +835,14 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
     if (e == cudaSuccess) e = cudaMallocHost(&b->herr, sizeof(int));
     if (e == cudaSuccess) *b->herr = 0;  // page-locked memory comes uninitialised; read even when no run precedes
     b->smem = batch_smem(b->prec);
+    b->nprogs = int(tb.ranges.size());
+    b->kernel = b->prec == QS_PREC_C64 ? reinterpret_cast<const void*>(k_batch<float2, false>)
+                : df_ok ? (fixed_point ? reinterpret_cast<const void*>(k_batch<FxC, true>)
+                                       : reinterpret_cast<const void*>(k_batch<double2, true>))
+                        : (fixed_point ? reinterpret_cast<const void*>(k_batch<FxC, false>)
+                                       : reinterpret_cast<const void*>(k_batch<double2, false>));
     if (e == cudaSuccess)
-        e = b->prec == QS_PREC_C64
-                ? cudaFuncSetAttribute(k_batch<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b->smem))
-                : cudaFuncSetAttribute(k_batch<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b->smem));
+        e = cudaFuncSetAttribute(b->kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b->smem));
     if (e != cudaSuccess) {
         release(b);
         return fail(e == cudaErrorMemoryAllocation ? QS_OUT_OF_MEMORY : QS_CUDA_ERROR,
@@ -805,6 +860,15 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
     b->dpart = reinterpret_cast<double*>(A + o_part);
     b->dres = reinterpret_cast<double*>(A + o_res);
     b->drtab = reinterpret_cast<int2*>(A + o_rtab);
+    b->dranges = reinterpret_cast<SweepRange*>(A + o_range);
+    b->dpasses = reinterpret_cast<SweepPass*>(A + o_pass);
+    b->drots = reinterpret_cast<SweepRot*>(A + o_rot);
+    b->dfixed = reinterpret_cast<TileOp*>(A + o_fix);
+    b->drslot = reinterpret_cast<int*>(A + o_rslot);
+    b->dcoefs = reinterpret_cast<SweepCoef*>(A + o_coef);
+    b->dweights = reinterpret_cast<double*>(A + o_wt);
+    b->dsigmas = reinterpret_cast<double*>(A + o_sig);
+    b->dwtab = reinterpret_cast<int*>(A + o_wtab);
     b->derr = reinterpret_cast<int*>(A + o_err);
     b->dticket = reinterpret_cast<unsigned int*>(A + o_tick);
     size_t off = o_states;
@@ -844,22 +908,27 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
             e2 = cudaMemcpy(b->dsegs, segs.data(), segs.size() * sizeof(int4), cudaMemcpyHostToDevice);
         return e2;
     };
-    if (!stages.empty())
-        e = cudaMemcpy(b->dstages, stages.data(), sizeof(BStage) * stages.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !ops.empty())
-        e = cudaMemcpy(b->dops, ops.data(), sizeof(BOp) * ops.size(), cudaMemcpyHostToDevice);
+    auto put = [&](void* to, const void* from, size_t bytes) {
+        if (e == cudaSuccess && bytes) e = cudaMemcpy(to, from, bytes, cudaMemcpyHostToDevice);
+    };
+    put(b->dstages, tb.stages.data(), sizeof(BStage) * tb.stages.size());
+    put(b->dops, tb.ops.data(), sizeof(BOp) * tb.ops.size());
+    put(b->dranges, tb.ranges.data(), sizeof(SweepRange) * tb.ranges.size());
+    put(b->dpasses, tb.passes.data(), sizeof(SweepPass) * tb.passes.size());
+    put(b->drots, tb.rots.data(), sizeof(SweepRot) * tb.rots.size());
+    put(b->dfixed, tb.fixed.data(), sizeof(TileOp) * tb.fixed.size());
+    put(b->drslot, tb.rslot.data(), 4 * tb.rslot.size());
+    put(b->dwtab, wtab.data(), 4 * wtab.size());
     if (e == cudaSuccess && !terms.empty())
         e = cudaMemcpy(b->dterms, terms.data(), sizeof(BPauli) * terms.size(), cudaMemcpyHostToDevice);
     for (int i = 0; i < b->ncs; i++) b->hcs[i] = make_double2(1.0, 0.0);
     // ---- chunk size and persistence: from options, the autotune cache, or by timing candidates
     int max_per_sm = 1;
     if (e == cudaSuccess)
-        e = b->prec == QS_PREC_C64
-                ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_per_sm, k_batch<float2>, kBT, b->smem)
-                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_per_sm, k_batch<double2>, kBT, b->smem);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_per_sm, b->kernel, kBT, b->smem);
     max_per_sm = std::max(1, max_per_sm);
     std::ostringstream key;
-    key << "batch2:p" << b->prec << ":a" << (b->arith == QS_ARITH_DF64) << ":c" << count << ":items";
+    key << "batch3:p" << b->prec << ":a" << (b->arith == QS_ARITH_DF64) << ":c" << count << ":items";
     {
         uint64_t sig = 0;
         for (size_t c = 0; c < count; c++) sig = sig * 1315423911ull + uint64_t(circuits[c].n) * 131 + circuits[c].m;
@@ -885,7 +954,7 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
             if (r == cudaSuccess) r = cudaGraphUpload(b->exec, b->stream);
             if (r == cudaSuccess && !warmed) {
                 r = cudaGraphLaunch(b->exec, b->stream);
-                if (r == cudaSuccess) note_launches(3);
+                if (r == cudaSuccess) note_launches(b->nprogs ? 4 : 3);
                 warmed = true;
             }
             if (r == cudaSuccess) r = cudaStreamSynchronize(b->stream);
@@ -893,7 +962,7 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
             const auto t0 = std::chrono::steady_clock::now();
             r = cudaGraphLaunch(b->exec, b->stream);
             if (r == cudaSuccess) r = cudaStreamSynchronize(b->stream);
-            if (r == cudaSuccess) note_launches(3);
+            if (r == cudaSuccess) note_launches(b->nprogs ? 4 : 3);
             *dt = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
             return r;
         };
@@ -944,7 +1013,7 @@ extern "C" int qs_batch_run(qs_batch* b, const double* params, double* energies,
         b->hcs[i] = make_double2(std::cos(0.5 * th), std::sin(0.5 * th));
     }
     cudaError_t e = cudaGraphLaunch(b->exec, b->stream);
-    if (e == cudaSuccess) note_launches(3);  // the graph's reset, persistent and reduction kernels
+    if (e == cudaSuccess) note_launches(b->nprogs ? 4 : 3);  // the graph's coefficient, reset, persistent and reduction kernels
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) {
         set_last_error_message(std::string("batch run: ") + cudaGetErrorString(e));
