@@ -548,7 +548,8 @@ static void plan_sweep(const qs_param_gate* gates, size_t m, const double2* angl
     P->weight_at.assign(std::max(1, nrot), -1);
     // rows of 128 bytes: more of the tile's qubits are free to choose
     const int low = df || ordered ? 5 : type == SW_C64 ? 4 : 3;
-    P->stages = plan_tiles(P->ops, n, tq, std::min(low, tq), false, df || ordered ? kAdjMaxOps : kSwMaxRot);
+    P->stages = plan_tiles(P->ops, n, tq, std::min(low, tq), false, df || ordered ? kAdjMaxOps : kSwMaxRot, false,
+                           !df && !ordered);
     for (size_t si = 0; si < P->stages.size(); si++) {
         const TileStage& st = P->stages[si];
         SweepPlan::Launch L;

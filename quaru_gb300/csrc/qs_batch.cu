@@ -613,7 +613,7 @@ void plan_circuit(const qs_batch_circuit& q, int T, int prec, bool df_ok, bool u
                 classify_gate(h, 1, G.targets, &fixed[g]);
             }
         }
-        const std::vector<TileStage> st = plan_tiles(list, n, T, L, false, df_ok || !unitary ? kMaxStageOps : kSwMaxRot);
+        const std::vector<TileStage> st = plan_tiles(list, n, T, L, false, kMaxStageOps, false, !df_ok && unitary);
         int count = 0;
         for (const TileStage& S : st) {
             BStage B{};

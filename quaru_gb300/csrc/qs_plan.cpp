@@ -35,50 +35,79 @@ static uint64_t qubit_mask(const OpDesc& op) {
 static bool pure_move(const OpDesc& op) { return op.kind == OP_MONO_PF || op.kind == OP_NOOP; }
 
 std::vector<TileStage> plan_tiles(const std::vector<OpDesc>& ops, int n, int T, int L, bool exact_order,
-                                  int max_ops, bool blocks_only) {
+                                  int max_ops, bool blocks_only, bool search) {
     std::vector<TileStage> stages;
     max_ops = std::max(1, std::min(max_ops, kMaxStageOps));
     if (T > n) T = n;
     if (L > T) L = T;
     const int H = std::min(T - L, kTileMaxHigh);
     const uint64_t low_mask = (L >= 64) ? ~0ull : ((1ull << L) - 1ull);
-    std::vector<int> remaining;
-    for (size_t i = 0; i < ops.size(); i++)
-        if (ops[i].kind != OP_NOOP) remaining.push_back(int(i));
-    while (!remaining.empty()) {
-        TileStage st;
-        st.tiled = true;
-        st.T = L + H;
-        st.L = L;
-        uint64_t high = 0, blocked = 0;
+    const uint64_t all = n >= 64 ? ~0ull : (1ull << n) - 1ull;
+    struct Item {
+        int idx;
+        bool move, fits;      // a pure move; the stage kernel can take it
+        uint64_t qm, need;    // its qubits; the high qubits its targets want in the tile
+    };
+    std::vector<Item> remaining, rest;
+    for (size_t i = 0; i < ops.size(); i++) {
+        const OpDesc& op = ops[i];
+        if (op.kind == OP_NOOP) continue;
+        Item it{int(i), pure_move(op), blocks_only ? op.kind == OP_BLOCK : tileable(op), qubit_mask(op), 0};
+        for (int j = 0; j < op.k; j++) it.need |= 1ull << op.tq[j];
+        it.need &= ~low_mask;
+        remaining.push_back(it);
+    }
+    // The gates a stage takes: in order, those that fit its high qubits and share no qubit with a gate
+    // left behind. With grow, the high qubits start from none and are claimed by the gates in turn;
+    // otherwise they are given. take / leave (nullable) get the two lists.
+    auto pack = [&](uint64_t* high, bool grow, std::vector<int>* take, std::vector<Item>* leave) {
+        uint64_t blocked = 0;
         bool arith_deferred = false;  // an arithmetic gate has been deferred in this pass
-        std::vector<int> rest;
-        for (int idx : remaining) {
-            const OpDesc& op = ops[idx];
-            const uint64_t qm = qubit_mask(op);
-            if ((qm & blocked) || (exact_order && arith_deferred && !pure_move(op))) {
-                blocked |= qm;
-                if (!pure_move(op)) arith_deferred = true;
-                rest.push_back(idx);
-                continue;
-            }
-            uint64_t need = 0;
-            for (int j = 0; j < op.k; j++) need |= 1ull << op.tq[j];
-            need &= ~low_mask;
-            const bool fits = blocks_only ? op.kind == OP_BLOCK : tileable(op);
-            if (fits && __builtin_popcountll(high | need) <= H && st.ops.size() < size_t(max_ops)) {
-                high |= need;
-                st.ops.push_back(idx);
+        int count = 0;
+        for (const Item& it : remaining) {
+            bool ok = !(it.qm & blocked) && !(exact_order && arith_deferred && !it.move) && it.fits && count < max_ops;
+            if (ok) ok = grow ? __builtin_popcountll(*high | it.need) <= H : (it.need & ~*high) == 0;
+            if (ok) {
+                *high |= it.need;
+                count++;
+                if (take) take->push_back(it.idx);
             } else {
-                blocked |= qm;
-                if (!pure_move(op)) arith_deferred = true;
-                rest.push_back(idx);
+                blocked |= it.qm;
+                if (!it.move) arith_deferred = true;
+                if (leave) leave->push_back(it);
+                else if (blocked == all) break;  // counting only: nothing more can run
             }
         }
+        return count;
+    };
+    while (!remaining.empty()) {
+        uint64_t high = 0;
+        bool grow = true;
+        if (search && n > T) {
+            // Besides the high qubits that the first gates claim, every window of H neighbouring ones: a
+            // ladder of CNOTs lets a window run several layers of a circuit, where claiming in turn stops
+            // at its edge (20-qubit ansatz, 10 layers: 11 stages instead of 22). The most gates win.
+            uint64_t h = 0;
+            int best = pack(&h, true, nullptr, nullptr);
+            for (int w = L; w + H <= n; w++) {
+                uint64_t c = ((1ull << H) - 1ull) << w;
+                const int count = pack(&c, false, nullptr, nullptr);
+                if (count > best) {
+                    best = count;
+                    high = c;
+                    grow = false;
+                }
+            }
+        }
+        TileStage st;
+        st.tiled = true;
+        st.L = L;
+        rest.clear();
+        pack(&high, grow, &st.ops, &rest);
         if (st.ops.empty()) {
             // The first remaining gate cannot be tiled: it runs on its own.
             TileStage single;
-            single.single = remaining[0];
+            single.single = remaining[0].idx;
             stages.push_back(single);
             remaining.erase(remaining.begin());
             continue;

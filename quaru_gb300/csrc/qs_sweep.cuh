@@ -201,6 +201,33 @@ __device__ __forceinline__ float2 sw_fma2(float2 a, float2 b, float2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(sw_pack(a)), "l"(sw_pack(b)), "l"(sw_pack(c)));
     return sw_unpack(r);
 }
+__device__ __forceinline__ float2 sw_mul2(float2 a, float2 b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(sw_pack(a)), "l"(sw_pack(b)));
+    return sw_unpack(r);
+}
+__device__ __forceinline__ float2 sw_add2(float2 a, float2 b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(sw_pack(a)), "l"(sw_pack(b)));
+    return sw_unpack(r);
+}
+__device__ __forceinline__ float2 sw_sub2(float2 a, float2 b) { return sw_fma2(b, make_float2(-1.0f, -1.0f), a); }
+// (x + y) of d as a compensated pair (TwoSum)
+__device__ __forceinline__ DfAcc sw_across(float2 d) {
+    DfAcc a;
+    a.s = __fadd_rn(d.x, d.y);
+    const float bb = __fsub_rn(a.s, d.x);
+    a.c = __fadd_rn(__fsub_rn(d.x, __fsub_rn(a.s, bb)), __fsub_rn(d.y, bb));
+    return a;
+}
+// d + f, both components, then across (TwoSum on both at once)
+__device__ __forceinline__ DfAcc sw_across(float2 d, float2 f) {
+    const float2 s = sw_add2(d, f), bb = sw_sub2(s, d);
+    const float2 e = sw_add2(sw_sub2(d, sw_sub2(s, bb)), sw_sub2(f, bb));
+    DfAcc a = sw_across(s);
+    a.c = __fadd_rn(a.c, __fadd_rn(e.x, e.y));
+    return a;
+}
 __device__ __forceinline__ float2 sw_axpy(float t, float2 b, float2 a) { return sw_fma2(make_float2(t, t), b, a); }
 
 template <typename T>
@@ -291,28 +318,26 @@ __device__ __forceinline__ double sw_inner(const double2 (&p)[N], const double2 
     }
     return s;
 }
-// complex64: real and imaginary parts side by side (packed operations); up to four products per chain, as
+// complex64: real and imaginary parts side by side (packed operations); chains of at most four products, as
 // one pair's four products take, then compensated sums.
 template <int J, int N>
 __device__ __forceinline__ DfAcc sw_inner(const float2 (&p)[N], const float2 (&l)[N]) {
-    float2 d[N / 2];
-    int n = 0;
+    float2 d[2];
 #pragma unroll
-    for (int r = 0; r < N; r++) {
-        if (r & (1 << J)) continue;
-        const int k = r | (1 << J);
-        const float2 m = sw_fma2(sw_minus(l[r]), p[k], make_float2(0.0f, 0.0f));
-        d[n++] = sw_fma2(l[k], p[r], m);
-    }
-    DfAcc acc;
-    acc.s = d[0].x;
-    acc.add(d[0].y);
+    for (int h = 0; h < (N > 4 ? 2 : 1); h++) {
+        float2 plus = make_float2(0.0f, 0.0f), minus = plus;
+        bool first = true;
 #pragma unroll
-    for (int i = 1; i < N / 2; i++) {
-        acc.add(d[i].x);
-        acc.add(d[i].y);
+        for (int i = 0; i < (N > 2 ? 2 : 1); i++) {
+            const int q = 2 * h + i, r = ((q >> J) << (J + 1)) | (q & ((1 << J) - 1)), k = r | (1 << J);
+            plus = first ? sw_mul2(l[k], p[r]) : sw_fma2(l[k], p[r], plus);
+            minus = first ? sw_mul2(l[r], p[k]) : sw_fma2(l[r], p[k], minus);
+            first = false;
+        }
+        d[h] = sw_sub2(plus, minus);
     }
-    return acc;
+    if constexpr (N > 4) return sw_across(d[0], d[1]);
+    else return sw_across(d[0]);
 }
 // fixed point: positive and negative products apart (each sum of 8 stays below 2^63 by the norms)
 struct FxSum {
@@ -370,26 +395,29 @@ __device__ __forceinline__ void sw_rotations(T* sp, T* sl, uint32_t tsize, const
     constexpr int N = 1 << RB;
     const uint32_t ntup = tsize >> RB, p = threadIdx.x;
     if ((p & ~31u) >= ntup) return;
-    const bool on = p < ntup;
     uint32_t base = p & P.seg[0];
     base |= (p << 1) & P.seg[1];
     if (RB > 1) base |= (p << 2) & P.seg[2];
     if (RB > 2) base |= (p << 3) & P.seg[3];
-    const uint32_t pb = S::at(base);
-    uint32_t w[RB];
+    uint32_t at[N];  // byte offsets
+    at[0] = S::at(base) * uint32_t(sizeof(T));
 #pragma unroll
-    for (int j = 0; j < RB; j++) w[j] = S::at(1u << P.rbit[j]);
-    auto where = [&](int r) {
-        uint32_t a = pb;
+    for (int j = 0; j < RB; j++) {
+        const uint32_t w = S::at(1u << P.rbit[j]) * uint32_t(sizeof(T));
 #pragma unroll
-        for (int j = 0; j < RB; j++)
-            if (r >> j & 1) a ^= w[j];
-        return a;
-    };
+        for (int r = 0; r < (1 << j); r++) at[r | (1 << j)] = at[r] ^ w;
+    }
     const uint32_t rx = P.rx;
+    const bool on = p < ntup;  // false only in the one warp of a tile of fewer than 32 tuples
     auto load = [&](const T* s, T (&x)[N]) {
+        if (ntup >= 32u) {
 #pragma unroll
-        for (int r = 0; r < N; r++) x[r] = on ? s[where(r)] : T{0, 0};
+            for (int r = 0; r < N; r++) x[r] = *reinterpret_cast<const T*>(reinterpret_cast<const char*>(s) + at[r]);
+        } else {
+#pragma unroll
+            for (int r = 0; r < N; r++)
+                x[r] = on ? *reinterpret_cast<const T*>(reinterpret_cast<const char*>(s) + at[r]) : T{0, 0};
+        }
         if (rx) sw_frames(rx, false, x);
     };
     if (REV) {
@@ -425,7 +453,7 @@ __device__ __forceinline__ void sw_rotations(T* sp, T* sl, uint32_t tsize, const
         if (rx) sw_frames(rx, true, x);
         if (on) {
 #pragma unroll
-            for (int r = 0; r < N; r++) s[where(r)] = x[r];
+            for (int r = 0; r < N; r++) *reinterpret_cast<T*>(reinterpret_cast<char*>(s) + at[r]) = x[r];
         }
     }
 }
@@ -493,7 +521,10 @@ __device__ __forceinline__ void sw_moves(T* sp, T* sl, uint32_t tsize, int tq, u
     if (on) {
 #pragma unroll
         for (int r = 0; r < N; r++) {
-            const uint32_t y = S::at(from(r));
+            uint32_t y = S::at(f);
+#pragma unroll
+            for (int j = 0; j < RB; j++)
+                if (r >> j & 1) y ^= S::at(c[j]);
             x[r] = sp[y];
             if (REV) l[r] = sl[y];
         }
@@ -594,7 +625,7 @@ __device__ __forceinline__ void sw_moves(T* sp, T* sl, uint32_t tsize, int tq, u
     if (on) {
 #pragma unroll
         for (int r = 0; r < N; r++) {
-            const uint32_t i = S::at(p | (uint32_t(r) << TB));
+            const uint32_t i = S::at(p) ^ S::at(uint32_t(r) << TB);
             sp[i] = x[r];
             if (REV) sl[i] = l[r];
         }
@@ -775,15 +806,16 @@ __device__ __forceinline__ float fx_relative(double v, uint32_t e) {  // |v| 2^(
 }
 __device__ __forceinline__ void fx_warp_norm(const double2* raw, uint32_t tsize, int nt, FxWarpNorm* box) {
     uint32_t e = 0;
-    for (uint32_t i = threadIdx.x; i < tsize; i += nt) {
-        const double2 v = raw[Sw<FxC>::at(i)];
+    const uint32_t ap = Sw<FxC>::at(threadIdx.x);
+    for (uint32_t i = 0; i + threadIdx.x < tsize; i += nt) {
+        const double2 v = raw[ap ^ Sw<FxC>::at(i)];
         e = max(e, max(fx_field(v.x), fx_field(v.y)));
     }
     e = __reduce_max_sync(0xffffffffu, e);
     float s = 0.0f;
     if (e != 0u && e != 0x7ffu)
-        for (uint32_t i = threadIdx.x; i < tsize; i += nt) {
-            const double2 v = raw[Sw<FxC>::at(i)];
+        for (uint32_t i = 0; i + threadIdx.x < tsize; i += nt) {
+            const double2 v = raw[ap ^ Sw<FxC>::at(i)];
             const float a = fx_relative(v.x, e), b = fx_relative(v.y, e);
             s = fmaf(a, a, fmaf(b, b, s));
         }
@@ -995,14 +1027,24 @@ __device__ __forceinline__ void sw_tile(const typename Sw<T>::Glob* src, typenam
     using S = Sw<T>;
     using G = typename S::Glob;
     constexpr bool FX = sizeof(T) == 16 && sizeof(typename S::Coef) != 16;
-    const uint32_t tsize = 1u << t.T, rmask = (1u << t.RL) - 1u;
+    const uint32_t tsize = 1u << t.T, rmask = (1u << t.RL) - 1u, p = threadIdx.x;
     G* rp = reinterpret_cast<G*>(sp);
     G* rl = reinterpret_cast<G*>(sl);
-#pragma unroll 4
-    for (uint32_t i = threadIdx.x; i < tsize; i += nt) {
-        const uint64_t g = base + side.rowoff[i >> t.RL] + (i & rmask);
-        rp[S::at(i)] = CG ? __ldcg(src + g) : src[g];
-        if (REV) rl[S::at(i)] = CG ? __ldcg(lam + g) : lam[g];
+    // element k of a thread is p | k nt: its place in memory and in the tile are those of p and of k nt put
+    // together (disjoint bits), the latter the same for the whole block
+    const uint64_t gp = base + side.rowoff[(p & (tsize - 1u)) >> t.RL] + (p & rmask);
+    const uint32_t ap = S::at(p);
+    auto place = [&](uint32_t i, uint64_t* g, uint32_t* at) {  // i = k nt
+        *g = gp + (side.rowoff[i >> t.RL] + (i & rmask));
+        *at = ap ^ S::at(i);
+    };
+#pragma unroll 8
+    for (uint32_t i = 0; i + p < tsize; i += nt) {
+        uint64_t g;
+        uint32_t at;
+        place(i, &g, &at);
+        rp[at] = CG ? __ldcg(src + g) : src[g];
+        if (REV) rl[at] = CG ? __ldcg(lam + g) : lam[g];
     }
     int kp = 0, kl = 0;
     double unit = 1.0;
@@ -1017,12 +1059,13 @@ __device__ __forceinline__ void sw_tile(const typename Sw<T>::Glob* src, typenam
         if (finite) {
             const int eu = 1023 + 60 - kp - kl;
             unit = eu > 0 && eu < 2047 ? __hiloint2double(eu << 20, 0) : fx_to_double_any(1, eu - 1023);
-            for (uint32_t i = threadIdx.x; i < tsize; i += nt) {
-                const double2 v = rp[S::at(i)];
-                sp[S::at(i)] = T{fx_from(v.x, kp), fx_from(v.y, kp)};
+            for (uint32_t i = 0; i + p < tsize; i += nt) {
+                const uint32_t at = ap ^ S::at(i);
+                const double2 v = rp[at];
+                sp[at] = T{fx_from(v.x, kp), fx_from(v.y, kp)};
                 if (REV) {
-                    const double2 w = rl[S::at(i)];
-                    sl[S::at(i)] = T{fx_from(w.x, kl), fx_from(w.y, kl)};
+                    const double2 w = rl[at];
+                    sl[at] = T{fx_from(w.x, kl), fx_from(w.y, kl)};
                 }
             }
         }
@@ -1043,16 +1086,18 @@ __device__ __forceinline__ void sw_tile(const typename Sw<T>::Glob* src, typenam
     }
     if (t.store) {
         const bool scaled = !FX && t.ndiag == 0;
-        for (uint32_t i = threadIdx.x; i < tsize; i += nt) {
-            const uint64_t g = base + side.rowoff[i >> t.RL] + (i & rmask);
+        for (uint32_t i = 0; i + p < tsize; i += nt) {
+            uint64_t g;
+            uint32_t at;
+            place(i, &g, &at);
             auto out = [&](const T* s, int k) {
                 G v;
                 if constexpr (FX) {
-                    const T a = s[S::at(i)];
+                    const T a = s[at];
                     if (finite) v = G{fx_to(a.x, k), fx_to(a.y, k)};
                     else v.x = v.y = __longlong_as_double(0x7ff8ll << 48);
                 } else {
-                    v = s[S::at(i)];
+                    v = s[at];
                     if (scaled) v.x *= decltype(v.x)(t.sigma), v.y *= decltype(v.y)(t.sigma);
                 }
                 return v;

@@ -19,9 +19,9 @@
 namespace qs {
 
 constexpr int kSwMaxT = 11;        // tile qubits
-constexpr int kSwMaxPass = 48;     // passes of a program
-constexpr int kSwMaxDiag = 4;      // of them with phases (their factor tables stay in shared memory)
-constexpr int kSwMaxRot = 48;      // rotations of a program (their sums stay in shared memory)
+constexpr int kSwMaxPass = 64;     // passes of a program
+constexpr int kSwMaxDiag = 6;      // of them with phases (their factor tables stay in shared memory)
+constexpr int kSwMaxRot = 64;      // rotations of a program (their sums stay in shared memory)
 constexpr int kSwOutside = 6;      // controls outside the tile of one pass's moves
 
 enum SwKind : uint8_t { SW_ROT = 0, SW_MOVE = 1, SW_FIXED = 2 };

@@ -120,9 +120,11 @@ bool tileable(const OpDesc& op);
 // Greedy stage planner with reordering of commuting gates (gates that share no
 // qubit). exact_order keeps arithmetic gates in their original relative order; a stage holds at most
 // max_ops (<= kMaxStageOps) gates. blocks_only (the tensor-core stages) admits OP_BLOCK ops only;
-// every other op runs on its own.
+// every other op runs on its own. search: choose each stage's high qubits among several sets instead of
+// letting the first gates claim them.
 std::vector<TileStage> plan_tiles(const std::vector<OpDesc>& ops, int n, int T, int L, bool exact_order,
-                                  int max_ops = kMaxStageOps, bool blocks_only = false);
+                                  int max_ops = kMaxStageOps, bool blocks_only = false,
+                                  bool search = false);
 
 // Device image of one op inside `stage`.
 TileOp make_tile_op(const OpDesc& op, const TileStage& stage);
