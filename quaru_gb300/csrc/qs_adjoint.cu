@@ -420,7 +420,7 @@ int expval_pauli(const void* psi, int prec, int n, const qs_pauli_term* terms, s
                  o_lam = o_res + 256, total = o_lam + N * amp;
     std::vector<PauliDev> ht = pauli_table(terms, nt);
     double res[2] = {0, 0};
-    AJ_CHECK(cudaMallocAsync((void**)&blob, total, s), "expval buffers");
+    AJ_CHECK(device_alloc((void**)&blob, total, s), "expval buffers");
     if (nt) AJ_CHECK(cudaMemcpyAsync(blob + o_terms, ht.data(), nt * sizeof(PauliDev), cudaMemcpyHostToDevice, s),
                      "terms upload");
     if (prec == QS_PREC_C64)
@@ -671,7 +671,7 @@ static int upload_sweep(const SweepPlan& P, const std::vector<double2>& angles, 
                  o_ang = o_at + al(P.weight_at.size() * sizeof(int)), up = o_ang + al(angles.size() * sizeof(double2)),
                  o_coef = up, o_wt = o_coef + al(P.rots.size() * sizeof(SweepCoef)), o_sig = o_wt + al(P.rots.size() * 8 + 8),
                  total = o_sig + al(P.ranges.size() * 8 + 8);
-    cudaError_t e = cudaMallocAsync((void**)&tb->dev, total, s);
+    cudaError_t e = device_alloc((void**)&tb->dev, total, s);
     if (e != cudaSuccess) {
         tb->dev = nullptr;
         return fail(e, "sweep tables", msg);
@@ -852,7 +852,7 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
     SweepPlan fplan, rplan;
     SweepTables ftab, rtab;
     int rc = QS_OK;
-    AJ_CHECK(cudaMallocAsync((void**)&blob, total, s), "adjoint buffers");
+    AJ_CHECK(device_alloc((void**)&blob, total, s), "adjoint buffers");
     {
         void* lam = blob + o_lam;
         void* psi = blob + o_psi;  // the register's own state is only read

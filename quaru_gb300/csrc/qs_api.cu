@@ -30,10 +30,11 @@ struct qs_register {
     int device = 0;
     int sms = 1;
     void* state = nullptr;
+    bool pooled = false;         // state and mscratch come from the library's pool (small registers)
     cudaStream_t stream = nullptr;
     double* partials = nullptr;  // device: per-block reduction partials
     double* dres = nullptr;      // device: small results
-    double* hres = nullptr;      // pinned host mirror of dres
+    double* hres = nullptr;      // pinned host: small results, written by kernels or copied from dres
     // Qubits collapsed by measurements with no gate on them since: every amplitude whose zmask bits
     // differ from zval is an exact zero, so later measurements visit only the live subspace.
     uint64_t zmask = 0;
@@ -132,16 +133,87 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 size_t amp_bytes(int prec) { return prec == QS_PREC_C64 ? 8 : 16; }
 
+// What a register has besides its state: a stream, partial sums and result slots. Making them costs more
+// than a small program's gates (with the state 450 us of a 12-qubit program's 3.2 ms), so up to
+// kSupports sets of freed registers wait for the next ones. Their streams are idle.
+struct Support {
+    int device = 0;
+    cudaStream_t stream = nullptr;
+    double* partials = nullptr;
+    double* dres = nullptr;
+    double* hres = nullptr;
+};
+constexpr size_t kSupports = 4;
+std::mutex g_support_mu;
+std::vector<Support> g_supports;
+
+void release_support(const Support& u) {
+    if (u.partials) cudaFree(u.partials);
+    if (u.dres) cudaFree(u.dres);
+    if (u.hres) cudaFreeHost(u.hres);
+    if (u.stream) cudaStreamDestroy(u.stream);
+}
+
+cudaError_t acquire_support(int device, Support* u) {
+    {
+        std::lock_guard<std::mutex> lock(g_support_mu);
+        for (size_t i = 0; i < g_supports.size(); i++)
+            if (g_supports[i].device == device) {
+                *u = g_supports[i];
+                g_supports.erase(g_supports.begin() + long(i));
+                return cudaSuccess;
+            }
+    }
+    u->device = device;
+    cudaError_t e = cudaStreamCreateWithFlags(&u->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMalloc(&u->partials, 2 * kMaxPartials * sizeof(double));
+    if (e == cudaSuccess) e = cudaMalloc(&u->dres, 64 * sizeof(double));
+    if (e == cudaSuccess) e = cudaMallocHost(&u->hres, 64 * sizeof(double));
+    if (e != cudaSuccess) {
+        release_support(*u);
+        *u = Support();
+    }
+    return e;
+}
+
+// States up to this size (and their scratch) come from the library's pool, larger ones from cudaMalloc.
+constexpr size_t kPooledState = size_t(32) << 20;
+
+// State-sized memory: pooled, or from cudaMalloc after the pool has given its own back.
+cudaError_t state_alloc(bool pooled, void** p, size_t bytes, cudaStream_t s) {
+    if (pooled) return qs::device_alloc(p, bytes, s);
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        qs::give_back_memory();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 void destroy(qs_register* r) {
     if (!r) return;
-    if (r->stream) cudaStreamSynchronize(r->stream);
-    if (r->state) cudaFree(r->state);
-    if (r->partials) cudaFree(r->partials);
-    if (r->dres) cudaFree(r->dres);
-    if (r->mscratch) cudaFree(r->mscratch);
-    if (r->hres) cudaFreeHost(r->hres);
-    if (r->stream) cudaStreamDestroy(r->stream);
+    bool idle = true;
+    if (r->stream) idle = cudaStreamSynchronize(r->stream) == cudaSuccess;
+    for (void* p : {r->state, r->mscratch}) {
+        if (!p) continue;
+        if (r->pooled) cudaFreeAsync(p, r->stream);
+        else cudaFree(p);
+    }
+    if (r->stream) {
+        const Support u{r->device, r->stream, r->partials, r->dres, r->hres};
+        bool kept = false;
+        if (idle) {
+            std::lock_guard<std::mutex> lock(g_support_mu);
+            if (g_supports.size() < kSupports) {
+                g_supports.push_back(u);
+                kept = true;
+            }
+        }
+        if (!kept) release_support(u);
+    }
     delete r;
+    qs::object_destroyed();
 }
 
 // Allocate a register with uninitialised state.
@@ -150,22 +222,27 @@ int allocate(size_t n, int prec, qs_register** out) {
     *out = nullptr;
     if (prec != QS_PREC_C128 && prec != QS_PREC_C64) return set_err(QS_INVALID_ARGUMENT, "unknown precision");
     if (n > kMaxQubits) return set_err(QS_INVALID_ARGUMENT, "too many qubits for one GPU");
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
     auto* r = new qs_register();
+    qs::object_created();
     r->n = int(n);
     r->prec = prec;
-    cudaError_t e = cudaGetDevice(&r->device);
-    if (e != cudaSuccess) {
-        delete r;
-        return cuda_fail(e, "cudaGetDevice");
-    }
+    r->device = device;
     cudaDeviceGetAttribute(&r->sms, cudaDevAttrMultiProcessorCount, r->device);
     if (r->sms < 1) r->sms = 1;
     const size_t bytes = (size_t(1) << n) * amp_bytes(prec);
-    if ((e = cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking)) != cudaSuccess ||
-        (e = cudaMalloc(&r->state, bytes)) != cudaSuccess ||
-        (e = cudaMalloc(&r->partials, 2 * kMaxPartials * sizeof(double))) != cudaSuccess ||
-        (e = cudaMalloc(&r->dres, 64 * sizeof(double))) != cudaSuccess ||
-        (e = cudaMallocHost(&r->hres, 64 * sizeof(double))) != cudaSuccess) {
+    r->pooled = bytes <= kPooledState;
+    Support u;
+    e = acquire_support(device, &u);
+    r->stream = u.stream;
+    r->partials = u.partials;
+    r->dres = u.dres;
+    r->hres = u.hres;
+    if (e == cudaSuccess) e = state_alloc(r->pooled, &r->state, bytes, r->stream);
+    if (e != cudaSuccess) {
+        r->state = nullptr;
         destroy(r);
         return cuda_fail(e, "allocating register");
     }
@@ -212,7 +289,8 @@ bool sequential_sums(const qs_register* reg) {
 
 // The register's half-state scratch, null when it cannot be had.
 void* measure_scratch(qs_register* reg) {
-    if (!reg->mscratch && cudaMalloc(&reg->mscratch, (size_t(1) << (reg->n - 1)) * amp_bytes(reg->prec)) != cudaSuccess) {
+    if (!reg->mscratch && state_alloc(reg->pooled, &reg->mscratch, (size_t(1) << (reg->n - 1)) * amp_bytes(reg->prec),
+                                      reg->stream) != cudaSuccess) {
         cudaGetLastError();
         reg->mscratch = nullptr;
     }
@@ -304,6 +382,8 @@ int qs_register_clone(const qs_register* src, qs_register** out) {
     if (e == cudaSuccess)
         e = cudaMemcpyAsync((*out)->state, src->state, (size_t(1) << src->n) * amp_bytes(src->prec),
                             cudaMemcpyDeviceToDevice, (*out)->stream);
+    // the source may be changed or freed on its own stream as soon as this call returns
+    if (e == cudaSuccess) e = cudaStreamSynchronize((*out)->stream);
     if (e != cudaSuccess) {
         destroy(*out);
         *out = nullptr;
@@ -402,11 +482,9 @@ int qs_try_measure(qs_register* reg, size_t target, double draw, int* outcome, d
         return set_err(QS_INVALID_TARGET, "InvalidTarget(" + std::to_string(target) + ")");
     }
     QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(target), reg->partials, kMaxPartials,
-                                     reg->dres, reg->stream, reg->sms, reg->zmask, reg->zval, sequential_sums(reg),
+                                     reg->hres, reg->stream, reg->sms, reg->zmask, reg->zval, sequential_sums(reg),
                                      seq_squares(reg)),
             "measure_probs");
-    QS_CUDA(cudaMemcpyAsync(reg->hres, reg->dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, reg->stream),
-            "measure readback");
     QS_CUDA(cudaStreamSynchronize(reg->stream), "measure sync");
     const double p0 = reg->hres[0], p1 = reg->hres[1];
     const int res = draw > p0 ? 1 : 0;  // src/register.rs:321
@@ -447,7 +525,7 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
     if (!scratch) return 1;
     const bool exactq = exact_quotient(reg);
     QS_CUDA(qs::launch_measure_probs(reg->state, n, reg->prec, int(targets[0]), reg->partials, kMaxPartials,
-                                     reg->dres, reg->stream, reg->sms),
+                                     reg->hres, reg->stream, reg->sms),
             "measure_probs");
     std::vector<int> free_bits(n);  // the source buffer's index bits, as qubits, ascending
     for (int q = 0; q < n; q++) free_bits[q] = q;
@@ -457,8 +535,6 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
     const void* src = reg->state;
     void* dst = nullptr;
     for (size_t k = 0; k < m; k++) {
-        QS_CUDA(cudaMemcpyAsync(reg->hres, reg->dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, reg->stream),
-                "measure readback");
         QS_CUDA(cudaStreamSynchronize(reg->stream), "measure sync");
         const double p0 = reg->hres[0], p1 = reg->hres[1];
         const int res = draws[k] > p0 ? 1 : 0;  // src/register.rs:321
@@ -471,7 +547,7 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
         const int next_pos = k + 1 < m ? index_of(targets[k + 1]) : -1;
         dst = (k % 2 == 0) ? scratch : reg->state;  // the first pass reads the whole state
         QS_CUDA(qs::launch_collapse_compact(src, dst, nfree, reg->prec, pos, res, d, rinv, next_pos, reg->partials,
-                                            kMaxPartials, reg->dres, reg->stream, reg->sms, exactq),
+                                            kMaxPartials, reg->hres, reg->stream, reg->sms, exactq),
                 "collapse_compact");
         record_outcome(reg, targets[k], res);
         src = dst;
@@ -529,11 +605,9 @@ int qs_measure_sequence(qs_register* reg, const size_t* targets, size_t m, const
         if (rc != 1) return rc;
     }
     QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(targets[0]), reg->partials, kMaxPartials,
-                                     reg->dres, reg->stream, reg->sms, reg->zmask, reg->zval, seq, seq_squares(reg)),
+                                     reg->hres, reg->stream, reg->sms, reg->zmask, reg->zval, seq, seq_squares(reg)),
             "measure_probs");
     for (size_t k = 0; k < m; k++) {
-        QS_CUDA(cudaMemcpyAsync(reg->hres, reg->dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, reg->stream),
-                "measure readback");
         QS_CUDA(cudaStreamSynchronize(reg->stream), "measure sync");
         const double p0 = reg->hres[0], p1 = reg->hres[1];
         const int res = draws[k] > p0 ? 1 : 0;
@@ -543,7 +617,7 @@ int qs_measure_sequence(qs_register* reg, const size_t* targets, size_t m, const
         const int t = int(targets[k]);
         if (k + 1 < m && !seq) {
             QS_CUDA(qs::launch_collapse_probs(reg->state, reg->n, reg->prec, t, res, d, rinv, int(targets[k + 1]),
-                                              reg->partials, kMaxPartials, reg->dres, reg->stream, reg->sms,
+                                              reg->partials, kMaxPartials, reg->hres, reg->stream, reg->sms,
                                               reg->zmask, reg->zval, exact_quotient(reg)),
                     "collapse_probs");
             record_outcome(reg, targets[k], res);
@@ -554,7 +628,7 @@ int qs_measure_sequence(qs_register* reg, const size_t* targets, size_t m, const
             record_outcome(reg, targets[k], res);
             if (k + 1 < m)
                 QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(targets[k + 1]), reg->partials,
-                                                 kMaxPartials, reg->dres, reg->stream, reg->sms, reg->zmask,
+                                                 kMaxPartials, reg->hres, reg->stream, reg->sms, reg->zmask,
                                                  reg->zval, seq, seq_squares(reg)),
                         "measure_probs");
         }
@@ -573,10 +647,8 @@ int qs_measure_probabilities(qs_register* reg, size_t target, double* prob0, dou
         return set_err(QS_INVALID_TARGET, "InvalidTarget(" + std::to_string(target) + ")");
     }
     QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(target), reg->partials, kMaxPartials,
-                                     reg->dres, reg->stream, reg->sms),
+                                     reg->hres, reg->stream, reg->sms),
             "measure_probs");
-    QS_CUDA(cudaMemcpyAsync(reg->hres, reg->dres, 2 * sizeof(double), cudaMemcpyDeviceToHost, reg->stream),
-            "measure readback");
     QS_CUDA(cudaStreamSynchronize(reg->stream), "measure sync");
     if (prob0) *prob0 = reg->hres[0];
     if (prob1) *prob1 = reg->hres[1];
@@ -670,7 +742,7 @@ int qs_get_state(const qs_register* reg, double* dst) {
     }
     const uint64_t chunk = std::min<uint64_t>(N, 1ull << 22);
     double* tmp = nullptr;
-    QS_CUDA(cudaMallocAsync((void**)&tmp, chunk * 16, reg->stream), "get_state temp");
+    QS_CUDA(qs::device_alloc((void**)&tmp, chunk * 16, reg->stream), "get_state temp");
     for (uint64_t f = 0; f < N; f += chunk) {
         const uint64_t c = std::min<uint64_t>(chunk, N - f);
         QS_CUDA(qs::launch_to_c128(reg->state, reg->prec, f, c, tmp, reg->stream, reg->sms), "to_c128");
@@ -693,7 +765,7 @@ int qs_set_state(qs_register* reg, const double* src) {
     }
     const uint64_t chunk = std::min<uint64_t>(N, 1ull << 22);
     double* tmp = nullptr;
-    QS_CUDA(cudaMallocAsync((void**)&tmp, chunk * 16, reg->stream), "set_state temp");
+    QS_CUDA(qs::device_alloc((void**)&tmp, chunk * 16, reg->stream), "set_state temp");
     for (uint64_t f = 0; f < N; f += chunk) {
         const uint64_t c = std::min<uint64_t>(chunk, N - f);
         QS_CUDA(cudaMemcpyAsync(tmp, src + 2 * f, c * 16, cudaMemcpyHostToDevice, reg->stream), "set_state copy");
@@ -710,7 +782,7 @@ int qs_probabilities(const qs_register* reg, double* dst) {
     const uint64_t N = 1ull << reg->n;
     const uint64_t chunk = std::min<uint64_t>(N, 1ull << 22);
     double* tmp = nullptr;
-    QS_CUDA(cudaMallocAsync((void**)&tmp, chunk * 8, reg->stream), "probabilities temp");
+    QS_CUDA(qs::device_alloc((void**)&tmp, chunk * 8, reg->stream), "probabilities temp");
     for (uint64_t f = 0; f < N; f += chunk) {
         const uint64_t c = std::min<uint64_t>(chunk, N - f);
         QS_CUDA(qs::launch_norm_sqr(reg->state, reg->prec, f, c, tmp, reg->stream, reg->sms), "norm_sqr");

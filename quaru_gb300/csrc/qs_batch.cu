@@ -480,6 +480,9 @@ size_t al(size_t x) { return (x + 255) / 256 * 256; }
 
 void release(qs_batch* b) {
     if (!b) return;
+    struct Gone {
+        ~Gone() { object_destroyed(); }
+    } gone;
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
@@ -715,6 +718,7 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
     if (opts) o = *opts;
     if (o.precision != QS_PREC_C128 && o.precision != QS_PREC_C64) return fail(QS_INVALID_ARGUMENT, "unknown precision");
     auto* b = new qs_batch();
+    object_created();
     b->prec = o.precision;
     b->arith = o.arith;
     b->count = int(count);
@@ -830,6 +834,11 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
                  o_tick = o_err + 256, o_states = o_tick + 256, total = o_states + state_bytes;
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&b->arena, total);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        give_back_memory();
+        e = cudaMalloc(&b->arena, total);
+    }
     if (e == cudaSuccess) e = cudaMallocHost(&b->hcs, 16 * (size_t(b->ncs) + 1));
     if (e == cudaSuccess) e = cudaMallocHost(&b->hres, 8 * (size_t(b->nres) + 1));
     if (e == cudaSuccess) e = cudaMallocHost(&b->herr, sizeof(int));

@@ -44,7 +44,7 @@ int apply_op(void* state, int n, int prec, int arith, const OpDesc& op, cudaStre
     const size_t o_off = 0, o_src = o_off + off.size() * 8, o_pf = o_src + off_src.size() * 8,
                  o_lane = o_pf + ((pf.size() + 15) / 16) * 16, o_mat = o_lane + ((lane.size() + 15) / 16) * 16,
                  o_state = o_mat + ((mat.size() + 255) / 256) * 256, total = o_state + sbytes;
-    cudaError_t e = cudaMallocAsync((void**)&blob, total, s);
+    cudaError_t e = device_alloc((void**)&blob, total, s);
     if (e != cudaSuccess) return fail(e, "wide gate buffers", msg);
     BigOpBuffers b;
     b.off = reinterpret_cast<const uint64_t*>(blob + o_off);

@@ -38,6 +38,14 @@ cudaError_t resident_blocks(const void* func, int threads, size_t smem, int* per
 // the stream that reads it before returning, so the next request finds the copy done.
 void* pinned_staging(int slot, size_t bytes);
 
+// Stream-ordered device memory from the library's own pool (qs_memory.cpp), freed by cudaFreeAsync.
+cudaError_t device_alloc(void** p, size_t bytes, cudaStream_t s);
+// Every free byte of the pool back to the driver.
+void give_back_memory();
+// Registers and batches announce themselves: without any, the pool keeps one allocation unit.
+void object_created();
+void object_destroyed();
+
 // Set the message qs_last_error() returns on the calling thread.
 void set_last_error_message(const std::string& msg);
 

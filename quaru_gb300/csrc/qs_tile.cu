@@ -759,7 +759,7 @@ int run_tiled(void* state, int n, int prec, int arith, const std::vector<OpDesc>
     unsigned char* dblob = nullptr;
     const size_t ops_bytes = ((host.size() * sizeof(TileOp) + 255) / 256) * 256;
     {
-        cudaError_t e = cudaMallocAsync((void**)&dblob, ops_bytes + 256, s);
+        cudaError_t e = device_alloc((void**)&dblob, ops_bytes + 256, s);
         if (e != cudaSuccess) return tile_fail(e, "tile op table", msg);
         dops = reinterpret_cast<TileOp*>(dblob);
         derr = derr_dev ? derr_dev : reinterpret_cast<int*>(dblob + ops_bytes);
@@ -777,7 +777,7 @@ int run_tiled(void* state, int n, int prec, int arith, const std::vector<OpDesc>
     }
     float4* dfrag = nullptr;
     if (block_frags && !block_frags->empty()) {
-        cudaError_t e = cudaMallocAsync((void**)&dfrag, block_frags->size() * sizeof(float), s);
+        cudaError_t e = device_alloc((void**)&dfrag, block_frags->size() * sizeof(float), s);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(dfrag, block_frags->data(), block_frags->size() * sizeof(float),
                                 cudaMemcpyHostToDevice, s);

@@ -66,12 +66,30 @@ def _matrix(m) -> np.ndarray:
     return np.ascontiguousarray(np.asarray(m, dtype=np.complex128))
 
 
+_C128 = np.dtype(np.complex128)
+_TARGETS = [ctypes.c_size_t * k for k in range(9)]  # array types of the common arities
+
+
+class _Scratch(ctypes.Structure):
+    """What one gate or measurement call writes."""
+
+    _fields_ = [("err", ctypes.c_size_t * 3), ("p0", ctypes.c_double), ("p1", ctypes.c_double), ("out", ctypes.c_int)]
+
+
 class Register:
     """A quantum register of n qubits whose state lives in GPU memory (src/register.rs:22-37)."""
 
     def __init__(self, handle: int, rng: Callable[[], float] | None = None):
         self._h = ctypes.c_void_p(handle)
-        self._rng = rng or np.random.default_rng().random
+        self._generator = rng or None
+        self._scratch = _Scratch()
+        self._at = ctypes.addressof(self._scratch)
+
+    @property
+    def _rng(self) -> Callable[[], float]:
+        if self._generator is None:  # made when first drawn from
+            self._generator = np.random.default_rng().random
+        return self._generator
 
     # ---- construction (src/register.rs:41-102)
     @classmethod
@@ -141,13 +159,22 @@ class Register:
 
     # ---- gate application (src/register.rs:134-191, 259-281)
     def try_apply_fast(self, op: Operation) -> "Register":
-        m = _matrix(op.matrix)
-        t = np.ascontiguousarray(np.array(list(op.targets), dtype=np.uintp))
-        err = np.zeros(3, dtype=np.uintp)
+        m = op.matrix
+        if type(m) is not np.ndarray or m.dtype is not _C128 or m.ndim != 2 or not m.flags.c_contiguous:
+            m = _matrix(m)
+        targets = op.targets if type(op.targets) is list else list(op.targets)
+        k = len(targets)
+        try:
+            if k and min(targets) < 0:  # ctypes would wrap it
+                raise ValueError
+            t = (_TARGETS[k] if k < 9 else ctypes.c_size_t * k)(*targets)
+        except (TypeError, ValueError):  # what else numpy takes as integers, or its error
+            t = (ctypes.c_size_t * k)(*np.array(targets, dtype=np.uintp).tolist())
         rows = m.shape[0]
         cols = m.shape[1] if m.ndim == 2 else 1
-        _check(_lib.load().qs_try_apply_fast(self._h, _dp(m.view(np.float64)), rows, cols, _sp(t), len(t),
-                                             _sp(err)), err)
+        rc = _lib.apply_at(self._h, m.__array_interface__["data"][0], rows, cols, t, k, self._at)
+        if rc:
+            _check(rc, np.array(self._scratch.err, dtype=np.uintp))
         return self
 
     try_apply = try_apply_fast
@@ -225,13 +252,13 @@ class Register:
     # ---- measurement (src/register.rs:291-342)
     def try_measure(self, target: int, draw: float | None = None) -> bool:
         x = self._rng() if draw is None else float(draw)
-        out = ctypes.c_int(0)
-        p0, p1 = ctypes.c_double(0), ctypes.c_double(0)
-        err = np.zeros(3, dtype=np.uintp)
-        _check(_lib.load().qs_try_measure(self._h, target, x, ctypes.byref(out), ctypes.byref(p0), ctypes.byref(p1),
-                                          _sp(err)), err)
-        self.last_probs = (p0.value, p1.value)
-        return bool(out.value)
+        at, w = self._at, self._scratch
+        rc = _lib.measure_at(self._h, target, x, at + _Scratch.out.offset, at + _Scratch.p0.offset,
+                             at + _Scratch.p1.offset, at)
+        if rc:
+            _check(rc, np.array(w.err, dtype=np.uintp))
+        self.last_probs = (w.p0, w.p1)
+        return bool(w.out)
 
     def measure(self, target: int, draw: float | None = None) -> bool:
         try:
@@ -242,7 +269,7 @@ class Register:
     # ---- host views (src/register.rs:35, 379-413)
     @property
     def state(self) -> np.ndarray:
-        st = np.zeros(1 << self.size(), dtype=np.complex128)
+        st = np.empty(1 << self.size(), dtype=np.complex128)
         _check(_lib.load().qs_get_state(self._h, _dp(st.view(np.float64))))
         return st
 
