@@ -704,6 +704,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tile_tc(float2* __restrict__ 
 
 static cudaError_t launch_tile_tc(void* state, int n, const TileStage& st, int op_begin, int op_end,
                                   const TileOp* dops, const float4* dfrag, int* derr, cudaStream_t s, int sms) {
+    if (st.T != 12) return cudaErrorInvalidValue;  // its index tables address 12-qubit tiles: rows of 4 qubits or more
     const StageArgs sa = stage_args(st, op_begin, op_end);
     const int nops = op_end - op_begin;
     const size_t tile_bytes = sizeof(float2) << st.T;
