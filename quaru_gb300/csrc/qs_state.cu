@@ -170,16 +170,68 @@ static uint64_t subspace_pairs(int n, int target, uint64_t zmask) {
     return 1ull << (n - 1 - __builtin_popcountll(zmask & ~(1ull << target)));
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kT) k_prob_partials(const T* __restrict__ st, uint64_t npairs, uint64_t tb,
+// Sums of squares of complex64 amplitudes, split by a bit, without the FP64 pipe (64 cycles per warp
+// instruction and sub-partition on sm_103a, where conversion, square and sum of an amplitude took five). The
+// square of a float is a 48-bit integer at an even power of two, so a thread adds squares as 64-bit integers
+// on a scale set by the largest amplitude seen: kSqGuard bits below the unit of that amplitude's square, and
+// one binade above it for larger ones to come (2^-54 of its square is the unit). At most kSqChunks chunks
+// (128 squares, 2^63) go into one integer before it is added to the FP64 sum, so what is cut off is no more
+// than what the FP64 additions that it replaces would round.
+// 30 qubits, the first sums (2^30 amplitudes): 3.63 ms to 2.46 ms, bound by the integer pipe now.
+constexpr int kSqChunk = 8;    // amplitudes of a thread per chunk, their loads in flight together
+constexpr int kSqChunks = 8;   // chunks per FP64 addition
+constexpr int kSqGuard = 10;
+constexpr int kSqBlocks = 4;   // resident blocks per SM
+constexpr uint32_t kSqTop = 0x7f800000u;           // infinities and NaN: summed in FP64
+constexpr uint32_t kSqLow = uint32_t(48) << 23;    // a chunk with nothing of 2^-79 or more: in FP64 too
+
+struct SquareSum {  // of one value of the bit: the rarer outcome keeps its own scale
+    unsigned long long s = 0;
+    uint32_t e = 48;  // biased exponent of the scale; zeros and subnormals shift out of any scale used
+    int chunks = 0;
+    double p = 0.0;
+
+    __device__ __forceinline__ void flush() {
+        // unit: 2^(2 (e - 150) - kSqGuard)
+        p = fma(__ull2double_rn(s), __hiloint2double(int(uint32_t(1023 + 2 * (int(e) - 150) - kSqGuard) << 20), 0), p);
+        s = 0;
+        chunks = 0;
+    }
+    // before a chunk whose largest component has the bits `top` (sign cleared)
+    __device__ __forceinline__ void open(uint32_t top) {
+        const uint32_t et = (top >> 23) + 1u;
+        if (et > e || chunks == kSqChunks) {
+            flush();
+            e = max(et, 48u);
+        }
+        chunks++;
+    }
+};
+
+// the square of the component with the bits a (sign cleared) on the scale of exponent e
+__device__ __forceinline__ unsigned long long scaled_square(uint32_t a, uint32_t e) {
+    const uint32_t m = ((a & 0x007fffffu) | 0x00800000u) << (kSqGuard / 2);
+    unsigned long long q;
+    asm("{\n\t.reg .u64 w;\n\tmul.wide.u32 w, %1, %1;\n\tshr.u64 %0, w, %2;\n\t}"
+        : "=l"(q)
+        : "r"(m), "r"(2u * (e - (a >> 23))));
+    return q;
+}
+
+// A chunk's largest component (bits, sign cleared) allows integers: 0, or of a normal size.
+__device__ __forceinline__ bool top_fits(uint32_t top) { return top == 0u || top - kSqLow < kSqTop - kSqLow; }
+
+__device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+
+__global__ void __launch_bounds__(kT) k_prob_partials(const double2* __restrict__ st, uint64_t npairs, uint64_t tb,
                                                       const __grid_constant__ IndexMap map,
                                                       double* __restrict__ partials) {
     const uint64_t stride = uint64_t(gridDim.x) * kT;
     double p0 = 0.0, p1 = 0.0;
     for (uint64_t t = uint64_t(blockIdx.x) * kT + threadIdx.x; t < npairs; t += stride) {
         const uint64_t i0 = expand_index(t, map);
-        const double2 a = to_d2_int(st[i0]);
-        const double2 b = to_d2_int(st[i0 | tb]);
+        const double2 a = st[i0];
+        const double2 b = st[i0 | tb];
         p0 = fma(a.x, a.x, p0);
         p0 = fma(a.y, a.y, p0);
         p1 = fma(b.x, b.x, p1);
@@ -189,6 +241,61 @@ __global__ void __launch_bounds__(kT) k_prob_partials(const T* __restrict__ st, 
     if (threadIdx.x == 0) {
         partials[2 * blockIdx.x] = p0;
         partials[2 * blockIdx.x + 1] = p1;
+    }
+}
+
+// The same on complex64: chunks of kSqChunk / 2 pairs per thread.
+__global__ void __launch_bounds__(kT, kSqBlocks)
+    k_prob_partials_c64(const float2* __restrict__ st, uint64_t npairs, uint64_t tb, const __grid_constant__ IndexMap map,
+                        double* __restrict__ partials) {
+    constexpr int P = kSqChunk / 2;
+    const uint64_t stride = uint64_t(gridDim.x) * (kT * P);
+    SquareSum sum0, sum1;
+    for (uint64_t t0 = uint64_t(blockIdx.x) * (kT * P) + threadIdx.x; t0 < npairs; t0 += stride) {
+        float2 v[kSqChunk];
+        uint32_t top0 = 0, top1 = 0;
+#pragma unroll
+        for (int j = 0; j < P; j++) {
+            const uint64_t t = t0 + uint64_t(j) * kT;
+            v[2 * j] = v[2 * j + 1] = make_float2(0.0f, 0.0f);
+            if (t < npairs) {
+                const uint64_t i0 = expand_index(t, map);
+                v[2 * j] = st[i0];
+                v[2 * j + 1] = st[i0 | tb];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < P; j++) {
+            top0 = max(top0, max(abs_bits(v[2 * j].x), abs_bits(v[2 * j].y)));
+            top1 = max(top1, max(abs_bits(v[2 * j + 1].x), abs_bits(v[2 * j + 1].y)));
+        }
+        if (top_fits(top0) && top_fits(top1)) {
+            sum0.open(top0);
+            sum1.open(top1);
+#pragma unroll
+            for (int j = 0; j < P; j++) {
+                sum0.s += scaled_square(abs_bits(v[2 * j].x), sum0.e) + scaled_square(abs_bits(v[2 * j].y), sum0.e);
+                sum1.s +=
+                    scaled_square(abs_bits(v[2 * j + 1].x), sum1.e) + scaled_square(abs_bits(v[2 * j + 1].y), sum1.e);
+            }
+        } else {
+#pragma unroll 1
+            for (int j = 0; j < P; j++) {
+                const uint64_t t = t0 + uint64_t(j) * kT;
+                if (t >= npairs) break;
+                const uint64_t i0 = expand_index(t, map);
+                const double2 a = to_d2_int(st[i0]), b = to_d2_int(st[i0 | tb]);
+                sum0.p += fma(a.x, a.x, a.y * a.y);
+                sum1.p += fma(b.x, b.x, b.y * b.y);
+            }
+        }
+    }
+    sum0.flush();
+    sum1.flush();
+    block_sum2(sum0.p, sum1.p);
+    if (threadIdx.x == 0) {
+        partials[2 * blockIdx.x] = sum0.p;
+        partials[2 * blockIdx.x + 1] = sum1.p;
     }
 }
 
@@ -511,11 +618,12 @@ cudaError_t launch_measure_probs(const void* state, int n, int prec, int target,
         return counted(cudaGetLastError());
     }
     int grid = grid_cap(npairs, sms, 4);
+    if (prec == QS_PREC_C64) grid = std::min(grid, kSqBlocks * sms);  // one wave
     if (grid > max_partials) grid = max_partials;
     if (prec == QS_PREC_C64)
-        k_prob_partials<float2><<<grid, kT, 0, s>>>((const float2*)state, npairs, tb, map, partials);
+        k_prob_partials_c64<<<grid, kT, 0, s>>>((const float2*)state, npairs, tb, map, partials);
     else
-        k_prob_partials<double2><<<grid, kT, 0, s>>>((const double2*)state, npairs, tb, map, partials);
+        k_prob_partials<<<grid, kT, 0, s>>>((const double2*)state, npairs, tb, map, partials);
     k_prob_final<<<1, kT, 0, s>>>(partials, grid, out);
     return counted(cudaGetLastError(), 2);
 }
@@ -535,7 +643,7 @@ __device__ __forceinline__ double div_markstein(double x, double d, double rinv)
 // RN(1/d) is not usable), or one multiply by RN(1/d), within one ulp of the quotient (registers in
 // the other arithmetic forms, held to 1e-14: GB300's FP64 pipe bounds a collapse, and this form
 // takes 2 FP64 operations per amplitude instead of 6).
-constexpr int kDivMarkstein = 0, kDivTrue = 1, kDivMul = 2;
+constexpr int kDivMarkstein = 0, kDivTrue = 1, kDivMul = 2, kDivPair = 3;
 
 // The kept amplitude divided by sqrt(total) (src/register.rs:337), in the state's type.
 template <typename T, int DIV>
@@ -566,6 +674,123 @@ __device__ __forceinline__ T collapse_value(T v, double d, double rinv, double2*
         *as_double = to_d2_int(r);
         return r;
     }
+}
+
+// Complex64 collapse on the FP32 and integer pipes. 1/d = rh + rl to 48 bits, so p = x rh rounded, its
+// remainder x rh - p (exact) plus x rl, and p plus that sum is x / d within 2^-46 before its one rounding
+// to a float: the value of the FP64 product. That holds for 2^-100 <= |p| < inf (below, the remainder
+// would not be exact) and reciprocals that the host found within 2^+-60; a chunk with any other
+// component but 0 takes the FP64 form of collapse_value. src(t) and dst(t) are the kept amplitude's places,
+// drop(t) clears the other one, one(t) is the next target's bit. 30 qubits, all 30 collapses: 16.5 ms with five
+// FP64 instructions an amplitude, 5.0 ms now.
+constexpr uint32_t kPairLow = uint32_t(127 - 100) << 23;
+
+__device__ __forceinline__ float pair_product(float x, float rh, float rl) {
+    const float p = x * rh;
+    const float y = p + fmaf(x, rl, fmaf(x, rh, -p));
+    return __uint_as_float((__float_as_uint(y) & 0x7fffffffu) | (__float_as_uint(p) & 0x80000000u));  // keeps -0
+}
+
+template <int DIV, bool SUMS, typename Src, typename Dst, typename Drop, typename One>
+__device__ __forceinline__ void collapse_chunks(uint64_t npairs, double d, double rinv, double* __restrict__ partials,
+                                                Src src, Dst dst, Drop drop, One one) {
+    const uint64_t stride = uint64_t(gridDim.x) * (kT * kSqChunk);
+    const float rh = float(rinv), rl = float(rinv - double(rh));
+    SquareSum sum0, sum1;
+    for (uint64_t t0 = uint64_t(blockIdx.x) * (kT * kSqChunk) + threadIdx.x; t0 < npairs; t0 += stride) {
+        bool fast = false;
+        if constexpr (DIV == kDivPair) {
+            float2 y[kSqChunk];
+            uint32_t top0 = 0, top1 = 0, low = ~0u;
+#pragma unroll
+            for (int j = 0; j < kSqChunk; j++) {
+                const uint64_t t = t0 + uint64_t(j) * kT;
+                y[j] = make_float2(0.0f, 0.0f);
+                if (t < npairs) y[j] = *src(t);
+            }
+#pragma unroll
+            for (int j = 0; j < kSqChunk; j++) {
+                y[j].x = pair_product(y[j].x, rh, rl);
+                y[j].y = pair_product(y[j].y, rh, rl);
+                const uint32_t a = abs_bits(y[j].x), b = abs_bits(y[j].y);
+                const bool o = SUMS && one(t0 + uint64_t(j) * kT);
+                top0 = max(top0, o ? 0u : max(a, b));
+                top1 = max(top1, o ? max(a, b) : 0u);
+                low = min(low, min(a - 1u, b - 1u));  // zeros don't count
+            }
+            fast = top_fits(top0) && top_fits(top1) && low >= kPairLow;
+            if (fast) {
+                if (SUMS) {
+                    sum0.open(top0);
+                    sum1.open(top1);
+                }
+#pragma unroll
+                for (int j = 0; j < kSqChunk; j++) {
+                    const uint64_t t = t0 + uint64_t(j) * kT;
+                    if (SUMS) {
+                        const bool o = one(t);
+                        const uint32_t e = o ? sum1.e : sum0.e;
+                        const unsigned long long q = scaled_square(abs_bits(y[j].x), e) + scaled_square(abs_bits(y[j].y), e);
+                        sum0.s += o ? 0ull : q;
+                        sum1.s += o ? q : 0ull;
+                    }
+                    if (t < npairs) {
+                        *dst(t) = y[j];
+                        drop(t);
+                    }
+                }
+            }
+        }
+        if (!fast) {
+#pragma unroll 1
+            for (int j = 0; j < kSqChunk; j++) {
+                const uint64_t t = t0 + uint64_t(j) * kT;
+                if (t >= npairs) break;
+                double2 y;
+                *dst(t) = collapse_value<float2, DIV == kDivPair ? kDivMul : DIV>(*src(t), d, rinv, &y);
+                drop(t);
+                const double q = fma(y.x, y.x, y.y * y.y);
+                const bool o = SUMS && one(t);
+                sum0.p += o ? 0.0 : q;
+                sum1.p += o ? q : 0.0;
+            }
+        }
+    }
+    if (SUMS) {
+        sum0.flush();
+        sum1.flush();
+        block_sum2(sum0.p, sum1.p);
+        if (threadIdx.x == 0) {
+            partials[2 * blockIdx.x] = sum0.p;
+            partials[2 * blockIdx.x + 1] = sum1.p;
+        }
+    }
+}
+
+// In place: the pass of k_collapse, and with SUMS of k_collapse_probs.
+template <int DIV, bool SUMS>
+__global__ void __launch_bounds__(kT, kSqBlocks)
+    k_collapse_c64(float2* st, uint64_t npairs, uint64_t tb, const __grid_constant__ IndexMap map, int outcome, double d,
+                   double rinv, uint64_t next_tb, double* __restrict__ partials) {
+    const uint64_t kb = outcome ? tb : 0;
+    auto at = [&](uint64_t t) { return st + (expand_index(t, map) | kb); };
+    collapse_chunks<DIV, SUMS>(npairs, d, rinv, partials, at, at,
+                               [&](uint64_t t) { st[expand_index(t, map) | (tb ^ kb)] = make_float2(0.0f, 0.0f); },
+                               [&](uint64_t t) { return ((expand_index(t, map) | kb) & next_tb) != 0; });
+}
+
+template <bool SUMS>
+static void collapse_c64(void* state, uint64_t npairs, uint64_t tb, const IndexMap& map, int outcome, double d,
+                         double rinv, int mode, uint64_t ntb, double* partials, int grid, cudaStream_t s) {
+    auto k = mode == kDivTrue ? k_collapse_c64<kDivTrue, SUMS>
+             : mode == kDivMul ? k_collapse_c64<kDivMul, SUMS>
+                               : k_collapse_c64<kDivPair, SUMS>;
+    k<<<grid, kT, 0, s>>>(static_cast<float2*>(state), npairs, tb, map, outcome, d, rinv, ntb, partials);
+}
+
+// Grid of a collapse: shared by the in-place and the compact form, whose sums have to agree.
+static int collapse_grid(uint64_t npairs, int prec, int sms) {
+    return prec == QS_PREC_C64 ? std::min(grid_cap(npairs, sms, kSqChunk), kSqBlocks * sms) : grid_cap(npairs, sms, 2);
 }
 
 template <typename T, int DIV>
@@ -616,6 +841,13 @@ static int div_mode(double d, double rinv, bool exact_quotient) {
     return exact_quotient ? kDivMarkstein : kDivMul;
 }
 
+// Complex64 multiplies by RN(1/d) unless it must divide: as a pair of floats where both fit well inside
+// their range.
+static int div_mode_c64(double d, double rinv) {
+    const int mode = div_mode(d, rinv, false);
+    return mode == kDivMul && rinv > 0x1p-60 && rinv < 0x1p60 ? kDivPair : mode;
+}
+
 template <typename T, int DIV>
 static void collapse_t(void* state, uint64_t npairs, uint64_t tb, const IndexMap& map, int outcome, double d,
                        double rinv, int grid, cudaStream_t s) {
@@ -633,13 +865,10 @@ cudaError_t launch_collapse(void* state, int n, int prec, int target, int outcom
     const IndexMap map = subspace_map(target, zmask, zval);
     const uint64_t npairs = subspace_pairs(n, target, zmask);
     const uint64_t tb = 1ull << target;
-    const int grid = grid_cap(npairs, sms, 2);
-    const int mode = div_mode(d, rinv, exact_quotient);
-    if (prec == QS_PREC_C64) {  // complex64 multiplies by RN(1/d) unless it must divide
-        if (mode == kDivTrue)
-            collapse_t<float2, kDivTrue>(state, npairs, tb, map, outcome, d, rinv, grid, s);
-        else
-            collapse_t<float2, kDivMul>(state, npairs, tb, map, outcome, d, rinv, grid, s);
+    const int grid = collapse_grid(npairs, prec, sms);
+    const int mode = prec == QS_PREC_C64 ? div_mode_c64(d, rinv) : div_mode(d, rinv, exact_quotient);
+    if (prec == QS_PREC_C64) {
+        collapse_c64<false>(state, npairs, tb, map, outcome, d, rinv, mode, 0, nullptr, grid, s);
     } else if (mode == kDivTrue) {
         collapse_t<double2, kDivTrue>(state, npairs, tb, map, outcome, d, rinv, grid, s);
     } else if (mode == kDivMul) {
@@ -656,14 +885,11 @@ cudaError_t launch_collapse_probs(void* state, int n, int prec, int target, int 
     const IndexMap map = subspace_map(target, zmask, zval);
     const uint64_t npairs = subspace_pairs(n, target, zmask);
     const uint64_t tb = 1ull << target, ntb = 1ull << next_target;
-    int grid = grid_cap(npairs, sms, 2);
+    int grid = collapse_grid(npairs, prec, sms);
     if (grid > max_partials) grid = max_partials;
-    const int mode = div_mode(d, rinv, exact_quotient);
+    const int mode = prec == QS_PREC_C64 ? div_mode_c64(d, rinv) : div_mode(d, rinv, exact_quotient);
     if (prec == QS_PREC_C64) {
-        if (mode == kDivTrue)
-            collapse_probs_t<float2, kDivTrue>(state, npairs, tb, map, outcome, d, rinv, ntb, partials, grid, s);
-        else
-            collapse_probs_t<float2, kDivMul>(state, npairs, tb, map, outcome, d, rinv, ntb, partials, grid, s);
+        collapse_c64<true>(state, npairs, tb, map, outcome, d, rinv, mode, ntb, partials, grid, s);
     } else if (mode == kDivTrue) {
         collapse_probs_t<double2, kDivTrue>(state, npairs, tb, map, outcome, d, rinv, ntb, partials, grid, s);
     } else if (mode == kDivMul) {
@@ -711,6 +937,28 @@ __global__ void __launch_bounds__(kT) k_collapse_compact(const T* __restrict__ s
     }
 }
 
+template <int DIV, bool SUMS>
+__global__ void __launch_bounds__(kT, kSqBlocks)
+    k_collapse_compact_c64(const float2* __restrict__ src, float2* __restrict__ dst, uint64_t npairs,
+                           const __grid_constant__ IndexMap map, uint64_t keepbit, double d, double rinv,
+                           uint64_t next_bit, double* __restrict__ partials) {
+    collapse_chunks<DIV, SUMS>(npairs, d, rinv, partials,
+                               [&](uint64_t t) { return src + (expand_index(t, map) | keepbit); },
+                               [&](uint64_t t) { return dst + t; }, [](uint64_t) {},
+                               [&](uint64_t t) { return (t & next_bit) != 0; });
+}
+
+template <bool SUMS>
+static void collapse_compact_c64(const void* src, void* dst, uint64_t npairs, const IndexMap& map, uint64_t keepbit,
+                                 double d, double rinv, int mode, int next_pos, double* partials, int grid,
+                                 cudaStream_t s) {
+    auto k = mode == kDivTrue ? k_collapse_compact_c64<kDivTrue, SUMS>
+             : mode == kDivMul ? k_collapse_compact_c64<kDivMul, SUMS>
+                               : k_collapse_compact_c64<kDivPair, SUMS>;
+    k<<<grid, kT, 0, s>>>(static_cast<const float2*>(src), static_cast<float2*>(dst), npairs, map, keepbit, d, rinv,
+                          SUMS ? 1ull << next_pos : 0ull, partials);
+}
+
 template <typename T, int DIV>
 static void collapse_compact_t(const void* src, void* dst, uint64_t npairs, const IndexMap& map, uint64_t keepbit,
                                double d, double rinv, int next_pos, double* partials, int grid, cudaStream_t s) {
@@ -728,14 +976,14 @@ cudaError_t launch_collapse_compact(const void* src, void* dst, int nfree, int p
     const IndexMap map = subspace_map(pos, 0, 0);
     const uint64_t npairs = 1ull << (nfree - 1);
     const uint64_t keepbit = outcome ? (1ull << pos) : 0ull;
-    int grid = grid_cap(npairs, sms, 2);
+    int grid = collapse_grid(npairs, prec, sms);
     if (next_pos >= 0 && grid > max_partials) grid = max_partials;  // the in-place pass's grid
-    const int mode = div_mode(d, rinv, exact_quotient);
+    const int mode = prec == QS_PREC_C64 ? div_mode_c64(d, rinv) : div_mode(d, rinv, exact_quotient);
     if (prec == QS_PREC_C64) {
-        if (mode == kDivTrue)
-            collapse_compact_t<float2, kDivTrue>(src, dst, npairs, map, keepbit, d, rinv, next_pos, partials, grid, s);
+        if (next_pos >= 0)
+            collapse_compact_c64<true>(src, dst, npairs, map, keepbit, d, rinv, mode, next_pos, partials, grid, s);
         else
-            collapse_compact_t<float2, kDivMul>(src, dst, npairs, map, keepbit, d, rinv, next_pos, partials, grid, s);
+            collapse_compact_c64<false>(src, dst, npairs, map, keepbit, d, rinv, mode, 0, nullptr, grid, s);
     } else if (mode == kDivTrue) {
         collapse_compact_t<double2, kDivTrue>(src, dst, npairs, map, keepbit, d, rinv, next_pos, partials, grid, s);
     } else if (mode == kDivMul) {
