@@ -39,6 +39,8 @@ struct qs_register {
     // differ from zval is an exact zero, so later measurements visit only the live subspace.
     uint64_t zmask = 0;
     uint64_t zval = 0;
+    // The same knowledge for the gates, which also hold it from a basis state on: a superset of zmask.
+    qs::LiveSpace known;
     // Scratch of the compact measurement sequences and of the squares of reference-order sums (half
     // the state), allocated by the first one and kept until the register is destroyed.
     void* mscratch = nullptr;
@@ -269,8 +271,9 @@ void touch_qubits(qs_register* reg, const double* matrix, const size_t* targets,
     }
     const size_t entries = k < 32 ? (size_t(2) << (2 * k)) : 0;
     for (size_t i = 0; i < entries; i++)
-        if (!std::isfinite(matrix[i])) {
+        if (!std::isfinite(reg->prec == QS_PREC_C64 ? double(float(matrix[i])) : matrix[i])) {
             reg->zmask = reg->zval = 0;
+            reg->known = qs::LiveSpace{};
             break;
         }
 }
@@ -307,6 +310,8 @@ void record_outcome(qs_register* reg, size_t target, int res) {
     const uint64_t b = 1ull << target;
     reg->zmask |= b;
     reg->zval = (reg->zval & ~b) | (res ? b : 0ull);
+    reg->known.mask |= b;
+    reg->known.val = (reg->known.val & ~b) | (res ? b : 0ull);
 }
 
 }  // namespace
@@ -327,6 +332,8 @@ int qs_register_from_int(size_t n, size_t k, int precision, qs_register** out) {
         *out = nullptr;
         return cuda_fail(e, "init_basis");
     }
+    (*out)->known.mask = n < 64 ? (1ull << n) - 1ull : ~0ull;
+    (*out)->known.val = k;
     return QS_OK;
 }
 
@@ -378,6 +385,7 @@ int qs_register_clone(const qs_register* src, qs_register** out) {
     (*out)->arith = src->arith;
     (*out)->zmask = src->zmask;
     (*out)->zval = src->zval;
+    (*out)->known = src->known;
     cudaError_t e = cudaStreamSynchronize(src->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync((*out)->state, src->state, (size_t(1) << src->n) * amp_bytes(src->prec),
@@ -417,7 +425,8 @@ int qs_try_apply_fast(qs_register* reg, const double* matrix, size_t rows, size_
     qs::OpDesc op;
     qs::classify_gate(matrix, k, targets, &op);
     touch_qubits(reg, matrix, targets, k);
-    rc = qs::apply_op(reg->state, reg->n, reg->prec, reg->arith, op, reg->stream, reg->sms, &msg);
+    rc = qs::apply_op(reg->state, reg->n, reg->prec, reg->arith, op, reg->stream, reg->sms, &msg, &reg->known);
+    if (rc) reg->known = qs::LiveSpace{};
     return rc ? set_err(rc, msg) : QS_OK;
 }
 
@@ -469,7 +478,9 @@ int qs_apply_circuit(qs_register* reg, const qs_gate* gates, size_t m, const qs_
     } else if (o.fuse == 3) {
         o.fuse = 1;  // tuning switched off: stages at the automatic tile size
     }
-    int rc = qs::run_circuit(reg->state, reg->n, reg->prec, reg->arith, ops, gates, o, reg->stream, reg->sms, &msg);
+    int rc = qs::run_circuit(reg->state, reg->n, reg->prec, reg->arith, ops, gates, o, reg->stream, reg->sms, &msg,
+                             nullptr, &reg->known);
+    if (rc) reg->known = qs::LiveSpace{};  // part of it ran
     return rc ? set_err(rc, msg) : QS_OK;
 }
 
@@ -695,6 +706,7 @@ int qs_adjoint_gradient(qs_register* reg, const qs_param_gate* gates, size_t m, 
     if (!terms_fit(terms, nterms, reg->n)) return set_err(QS_INVALID_ARGUMENT, "Pauli term acts on a qubit >= n");
     std::string msg;
     reg->zmask = reg->zval = 0;  // the state is restored on return, but not assumed collapsed any more
+    reg->known = qs::LiveSpace{};
     int rc = qs::adjoint_gradient(reg->state, reg->n, reg->prec, reg->arith, gates, m, params, nparams, terms, nterms,
                                   reg->stream, reg->sms, energy, grad, err, &msg);
     return rc ? set_err(rc, msg) : QS_OK;
@@ -757,6 +769,7 @@ int qs_set_state(qs_register* reg, const double* src) {
     qs::TraceRange trace("qs_set_state");
     if (!reg || !src) return set_err(QS_INVALID_ARGUMENT, "null argument");
     reg->zmask = reg->zval = 0;
+    reg->known = qs::LiveSpace{};
     const uint64_t N = 1ull << reg->n;
     if (reg->prec == QS_PREC_C128) {
         QS_CUDA(cudaMemcpyAsync(reg->state, src, N * 16, cudaMemcpyHostToDevice, reg->stream), "set_state");

@@ -10,13 +10,17 @@
 
 namespace qs {
 
-// Apply one classified gate (any width) in place on the register's stream.
-int apply_op(void* state, int n, int prec, int arith, const OpDesc& op, cudaStream_t s, int sms, std::string* msg);
+// Apply one classified gate (any width) in place on the register's stream. live (nullable): what is known of
+// the state; only the amplitudes that can be non-zero are visited, and it is kept up to date.
+int apply_op(void* state, int n, int prec, int arith, const OpDesc& op, cudaStream_t s, int sms, std::string* msg,
+             LiveSpace* live = nullptr);
 
 // Apply a classified gate list with the fusion strategy in `opts` (gates are
-// the same list, unclassified, for dense-block fusion). derr_dev: see run_tiled.
+// the same list, unclassified, for dense-block fusion). derr_dev: see run_tiled. live: see
+// apply_op.
 int run_circuit(void* state, int n, int prec, int arith, const std::vector<OpDesc>& ops, const qs_gate* gates,
-                const qs_circuit_options& opts, cudaStream_t s, int sms, std::string* msg, int* derr_dev = nullptr);
+                const qs_circuit_options& opts, cudaStream_t s, int sms, std::string* msg, int* derr_dev = nullptr,
+                LiveSpace* live = nullptr);
 
 // ---- fusion autotuner (qs_autotune.cpp) ----
 struct TuneChoice {

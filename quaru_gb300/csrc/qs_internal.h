@@ -52,6 +52,22 @@ struct OpDesc {
     int block = -1;               // OP_BLOCK: index of the fused block
 };
 
+// What is known of a state: every amplitude whose index differs from val in a bit of mask is an exact zero.
+// A gate with finite entries keeps that for the qubits it does not act on.
+struct LiveSpace {
+    uint64_t mask = 0, val = 0;
+    void release(uint64_t qubits) {
+        mask &= ~qubits;
+        val &= ~qubits;
+    }
+};
+
+inline uint64_t target_mask(const OpDesc& op) {
+    uint64_t t = 0;
+    for (int j = 0; j < op.k; j++) t |= 1ull << op.tq[j];
+    return t;
+}
+
 // Shape/target validation in the order of Register::try_apply_fast
 // (src/register.rs:141-153). Returns QS_OK or a status with err filled.
 int validate_gate(size_t n, size_t rows, size_t cols, const size_t* targets, size_t k, size_t* err,

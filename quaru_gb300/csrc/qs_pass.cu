@@ -195,17 +195,19 @@ cudaError_t launch_pass(void* state, int n, const TileStage& st, int op_begin, i
     std::vector<int> qpos;
     for (int q = 0; q < st.L; q++) qpos.push_back(q);
     for (int q : st.high) qpos.push_back(q);
+    for (int q = 0; q < 64; q++)
+        if (st.known.mask >> q & 1ull) qpos.push_back(q);
     std::sort(qpos.begin(), qpos.end());
     pa.outer.npos = int(qpos.size());
     for (size_t i = 0; i < qpos.size(); i++) pa.outer.pos[i] = uint8_t(qpos[i]);
-    pa.outer.fixval = 0;
+    pa.outer.fixval = st.known.val;
     const size_t tile_bytes = sizeof(float2) << st.T;
     const size_t fixed =
         12 * sizeof(uint64_t) + sizeof(TileOp) * size_t(op_end - op_begin) + (sizeof(uint64_t) << pa.RH);
     // three buffers where two blocks still fit an SM (4096-amplitude tiles), or one block (8192)
     pa.nbuf = (3 * tile_bytes + fixed <= (st.T >= 13 ? 220 : 110) * 1024) ? 3 : 2;
     const size_t smem = size_t(pa.nbuf) * tile_bytes + fixed;
-    const uint64_t ntiles = 1ull << (n - st.T);
+    const uint64_t ntiles = stage_tiles(n, st);
     auto go = [&](auto kern, int nthreads) -> cudaError_t {
         int per_sm = 0;
         cudaError_t e = resident_blocks(reinterpret_cast<const void*>(kern), nthreads, smem, &per_sm);

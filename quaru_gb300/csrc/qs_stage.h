@@ -34,10 +34,12 @@ inline StageArgs stage_args(const TileStage& st, int op_begin, int op_end) {
     std::vector<int> qpos;
     for (int q = 0; q < st.L; q++) qpos.push_back(q);
     for (int q : st.high) qpos.push_back(q);
+    for (int q = 0; q < 64; q++)
+        if (st.known.mask >> q & 1ull) qpos.push_back(q);
     std::sort(qpos.begin(), qpos.end());
     sa.outer.npos = int(qpos.size());
     for (size_t i = 0; i < qpos.size(); i++) sa.outer.pos[i] = uint8_t(qpos[i]);
-    sa.outer.fixval = 0;
+    sa.outer.fixval = st.known.val;
     // Copy rows: high qubits L, L + 1, ... continue the contiguous low run.
     int run = 0;
     while (run < sa.H && st.high[run] == st.L + run) run++;

@@ -575,7 +575,7 @@ static cudaError_t launch_tile(void* state, int n, const TileStage& st, int op_b
                          (sizeof(uint64_t) << sa.RH);
     sa.nbuf = (3 * tile_bytes + fixed <= 110 * 1024) ? 3 : 2;  // three buffers where two blocks still fit an SM
     const size_t smem = size_t(sa.nbuf) * tile_bytes + fixed;
-    const uint64_t ntiles = 1ull << (n - st.T);
+    const uint64_t ntiles = stage_tiles(n, st);
     // One wave exactly: every CTA walks the same number of tiles, so a grid larger than what is
     // resident would leave a second, partly empty wave.
     int per_sm = 0;
@@ -711,7 +711,7 @@ static cudaError_t launch_tile_tc(void* state, int n, const TileStage& st, int o
     const size_t smem = size_t(nops) * 2 * kTcBBytes + size_t(2 * kTcGroups) * tile_bytes +
                         size_t(nops) * 4 * kTcIdxWords + sizeof(TileOp) * size_t(nops) + (sizeof(uint64_t) << sa.RH) +
                         sizeof(uint64_t) * (1 + 3 * kTcGroups) + 16;
-    const uint64_t ntiles = 1ull << (n - st.T);
+    const uint64_t ntiles = stage_tiles(n, st);
     int per_sm = 0;
     cudaError_t oe = resident_blocks(reinterpret_cast<const void*>(k_tile_tc), kTcThreads, smem, &per_sm);
     if (oe != cudaSuccess) return oe;
@@ -735,7 +735,7 @@ static bool df64_range_ok(const OpDesc& op) {
 
 int run_tiled(void* state, int n, int prec, int arith, const std::vector<OpDesc>& ops,
               const std::vector<TileStage>& stages, cudaStream_t s, int sms, std::string* msg,
-              const std::vector<float>* block_frags, int* derr_dev) {
+              const std::vector<float>* block_frags, int* derr_dev, LiveSpace* live) {
     // tile arithmetic: exact order, FP64 FMA (also for QS_ARITH_FX64, whose one-gate sweeps are
     // fixed-point), double-float, complex64
     int rep = (prec == QS_PREC_C64) ? 3 : (arith == QS_ARITH_EXACT ? 0 : (arith == QS_ARITH_DF64 ? 2 : 1));
@@ -789,10 +789,16 @@ int run_tiled(void* state, int n, int prec, int arith, const std::vector<OpDesc>
     }
     int rc = QS_OK;
     for (size_t i = 0; i < stages.size() && rc == QS_OK; i++) {
-        const TileStage& st = stages[i];
-        if (!st.tiled) {
-            rc = apply_op(state, n, prec, arith, ops[st.single], s, sms, msg);
+        if (!stages[i].tiled) {
+            rc = apply_op(state, n, prec, arith, ops[stages[i].single], s, sms, msg, live);
             continue;
+        }
+        TileStage st = stages[i];
+        if (live && live->mask) {  // the qubits known outside the tile: only tiles at their values are visited
+            st.known = *live;
+            st.known.release((1ull << st.L) - 1ull);
+            for (int q : st.high) st.known.release(1ull << q);
+            for (int o : st.ops) live->release(target_mask(ops[o]));
         }
         const int b = first[i], e2 = (i + 1 < stages.size()) ? first[i + 1] : int(host.size());
         cudaError_t e;

@@ -112,7 +112,13 @@ struct TileStage {
     int T = 0, L = 0;
     std::vector<int> high;      // sorted global qubits on local bits L..T-1
     std::vector<int> ops;       // op indices, in execution order
+    LiveSpace known;            // of the qubits outside the tile, as the stage runs
 };
+
+// Tiles of a stage: those that can hold a non-zero amplitude.
+inline uint64_t stage_tiles(int n, const TileStage& st) {
+    return 1ull << (n - st.T - __builtin_popcountll(st.known.mask));
+}
 
 // Whether the tile kernel can run `op` (targets must still fit the tile).
 bool tileable(const OpDesc& op);
@@ -152,9 +158,11 @@ cudaError_t launch_pass(void* state, int n, const TileStage& st, int op_begin, i
 // Run stages on the device; ops are the host descriptors. With derr_dev null, waits for the stages and
 // reports a tile kernel's bounded wait that gave up (QS_TIMEOUT); otherwise the kernels raise the
 // caller's device flag *derr_dev (zeroed by the caller) and the call returns once the stages are
-// queued, leaving the wait and the check to the caller.
+// queued, leaving the wait and the check to the caller. live (nullable): what is known of the state, kept up
+// to date; a stage's tiles are those that can hold a non-zero amplitude (30 qubits from a basis state: 3 of
+// 9 stages visit next to nothing).
 int run_tiled(void* state, int n, int prec, int arith, const std::vector<OpDesc>& ops,
               const std::vector<TileStage>& stages, cudaStream_t s, int sms, std::string* msg,
-              const std::vector<float>* block_frags = nullptr, int* derr_dev = nullptr);
+              const std::vector<float>* block_frags = nullptr, int* derr_dev = nullptr, LiveSpace* live = nullptr);
 
 }  // namespace qs

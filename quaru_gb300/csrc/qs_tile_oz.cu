@@ -563,7 +563,7 @@ cudaError_t launch_tile_oz(void* state, int n, const TileStage& st, int op_begin
     const size_t tile_bytes = sizeof(double2) << st.T;
     const size_t smem = kOzBBytes + kOzScaleBytes + 2 * tile_bytes + 4 * size_t(kOzIdxWords) + sizeof(TileOp) +
                         (sizeof(uint64_t) << sa.RH) + 2 * kOzMath * 4 + kOzBars * sizeof(uint64_t) + 16;
-    const uint64_t ntiles = 1ull << (n - st.T);
+    const uint64_t ntiles = stage_tiles(n, st);
     int per_sm = 0;
     cudaError_t oe = resident_blocks(reinterpret_cast<const void*>(k_tile_oz), kOzThreads, smem, &per_sm);
     if (oe != cudaSuccess) return oe;
