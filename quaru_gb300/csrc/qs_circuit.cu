@@ -31,7 +31,8 @@ int apply_op(void* state, int n, int prec, int arith, const OpDesc& op, cudaStre
     if (op.kind == OP_NOOP) return QS_OK;
     if (live && live->mask) {
         // A circuit starts from a basis state and a gate frees its own qubits only: of the first layer on 28
-        // qubits a gate on qubit q has 2^(q + 1) amplitudes to visit (28 qubits, 84 gates: 113.6 ms without this, 96.5 with it).
+        // qubits a gate on qubit q has 2^(q + 1) amplitudes to visit (28 qubits, 84 gates: 113.6 ms without
+        // this, 96.5 ms with it).
         // The known qubits act as controls at their values, the highest ones at 0 as a smaller register.
         const uint64_t targets = target_mask(op), known = live->mask & ~targets;
         const uint64_t val = live->val;
@@ -116,6 +117,7 @@ static int run_blocks(void* state, int n, int prec, int arith, const qs_gate* ga
     std::vector<FusedBlock> blocks = fuse_blocks(gates, m, W, search);
     std::vector<OpDesc> ops;
     std::vector<float> frags;
+    std::vector<double> mats;
     for (FusedBlock& b : blocks) {
         if (live && !all_finite(b.u, prec)) *live = LiveSpace{};
         std::vector<size_t> tq(b.qubits.begin(), b.qubits.end());
@@ -127,13 +129,14 @@ static int run_blocks(void* state, int n, int prec, int arith, const qs_gate* ga
             op.orig_k = 5;
             for (int j = 0; j < 5; j++) op.tq[j] = b.qubits[j];
             op.touched_rows = 32;
-            const size_t per = oz ? kOzFragBytes / 4 : 4 * kBlockFragFloat4;  // floats per block
-            op.block = int(frags.size() / per);
-            frags.resize(frags.size() + per);
-            if (oz)
-                oz_fragments(b.u, reinterpret_cast<unsigned char*>(frags.data() + frags.size() - per));
-            else
+            const size_t per = 4 * kBlockFragFloat4;  // floats per complex64 block
+            op.block = int(oz ? mats.size() / 2048 : frags.size() / per);
+            if (oz) {
+                mats.insert(mats.end(), b.u.begin(), b.u.end());
+            } else {
+                frags.resize(frags.size() + per);
                 block_fragments(b.u, frags.data() + frags.size() - per);
+            }
         } else {
             tq.assign(b.qubits.begin(), b.qubits.end());
             classify_gate(b.u.data(), tq.size(), tq.data(), &op);
@@ -151,7 +154,7 @@ static int run_blocks(void* state, int n, int prec, int arith, const qs_gate* ga
     // (30 qubits, 4 layers: 9 stages against 11 with rows of 256 bytes)
     const int T = std::min(12, n), L = std::min(oz ? 5 : 4, T);
     std::vector<TileStage> stages = plan_tiles(ops, n, T, L, false, oz ? kMaxOzBlocks : kMaxTcBlocks, true);
-    return run_tiled(state, n, prec, arith, ops, stages, s, sms, msg, &frags, nullptr, live);
+    return run_tiled(state, n, prec, arith, ops, stages, s, sms, msg, &frags, nullptr, live, &mats);
 }
 
 int run_circuit(void* state, int n, int prec, int arith, const std::vector<OpDesc>& ops, const qs_gate* gates,

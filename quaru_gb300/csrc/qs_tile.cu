@@ -735,7 +735,8 @@ static bool df64_range_ok(const OpDesc& op) {
 
 int run_tiled(void* state, int n, int prec, int arith, const std::vector<OpDesc>& ops,
               const std::vector<TileStage>& stages, cudaStream_t s, int sms, std::string* msg,
-              const std::vector<float>* block_frags, int* derr_dev, LiveSpace* live) {
+              const std::vector<float>* block_frags, int* derr_dev, LiveSpace* live,
+              const std::vector<double>* block_mats) {
     // tile arithmetic: exact order, FP64 FMA (also for QS_ARITH_FX64, whose one-gate sweeps are
     // fixed-point), double-float, complex64
     int rep = (prec == QS_PREC_C64) ? 3 : (arith == QS_ARITH_EXACT ? 0 : (arith == QS_ARITH_DF64 ? 2 : 1));
@@ -777,7 +778,18 @@ int run_tiled(void* state, int n, int prec, int arith, const std::vector<OpDesc>
         }
     }
     float4* dfrag = nullptr;
-    if (block_frags && !block_frags->empty()) {
+    if (block_mats && !block_mats->empty()) {
+        const size_t blocks = block_mats->size() / 2048, mats = block_mats->size() * sizeof(double);
+        cudaError_t e = device_alloc((void**)&dfrag, blocks * kOzFragBytes + mats, s);
+        unsigned char* m = reinterpret_cast<unsigned char*>(dfrag) + blocks * kOzFragBytes;
+        if (e == cudaSuccess) e = cudaMemcpyAsync(m, block_mats->data(), mats, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = launch_oz_fragments(m, int(blocks), reinterpret_cast<unsigned char*>(dfrag), s);
+        if (e != cudaSuccess) {
+            cudaFreeAsync(dblob, s);
+            if (dfrag) cudaFreeAsync(dfrag, s);
+            return tile_fail(e, "block operands", msg);
+        }
+    } else if (block_frags && !block_frags->empty()) {
         cudaError_t e = device_alloc((void**)&dfrag, block_frags->size() * sizeof(float), s);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(dfrag, block_frags->data(), block_frags->size() * sizeof(float),

@@ -100,7 +100,8 @@ constexpr int kOzSlices = 7;
 constexpr uint32_t kOzBBytes = kOzSlices * kOzSliceBytes;
 constexpr uint32_t kOzScaleBytes = 256u;
 constexpr uint32_t kOzFragBytes = kOzBBytes + kOzScaleBytes + 64u * 64u * 8u;
-void oz_fragments(const std::vector<double>& u32x32, unsigned char* out /* kOzFragBytes */);
+// From `blocks` 32 x 32 complex matrices (2048 doubles each) on the device.
+cudaError_t launch_oz_fragments(const void* mats, int blocks, unsigned char* frags, cudaStream_t s);
 
 // Fused blocks per FP64-accurate tensor-core stage (the complex128 tiles take the room a second
 // block's slices would need).
@@ -159,10 +160,11 @@ cudaError_t launch_pass(void* state, int n, const TileStage& st, int op_begin, i
 // reports a tile kernel's bounded wait that gave up (QS_TIMEOUT); otherwise the kernels raise the
 // caller's device flag *derr_dev (zeroed by the caller) and the call returns once the stages are
 // queued, leaving the wait and the check to the caller. live (nullable): what is known of the state, kept up
-// to date; a stage's tiles are those that can hold a non-zero amplitude (30 qubits from a basis state: 3 of
+// to date (block_frags: complex64 operand images; block_mats: complex128 block matrices); a stage's tiles are those that can hold a non-zero amplitude (30 qubits from a basis state: 3 of
 // 9 stages visit next to nothing).
 int run_tiled(void* state, int n, int prec, int arith, const std::vector<OpDesc>& ops,
               const std::vector<TileStage>& stages, cudaStream_t s, int sms, std::string* msg,
-              const std::vector<float>* block_frags = nullptr, int* derr_dev = nullptr, LiveSpace* live = nullptr);
+              const std::vector<float>* block_frags = nullptr, int* derr_dev = nullptr, LiveSpace* live = nullptr,
+              const std::vector<double>* block_mats = nullptr);
 
 }  // namespace qs
