@@ -172,8 +172,15 @@ int run_circuit(void* state, int n, int prec, int arith, const std::vector<OpDes
         }
         T = std::min(T, n);
         const int L = std::min(5, T);
-        std::vector<TileStage> stages =
-            plan_tiles(ops, n, T, L, prec == QS_PREC_C128 && arith == QS_ARITH_EXACT);
+        const bool exact_order = prec == QS_PREC_C128 && arith == QS_ARITH_EXACT;
+        std::vector<TileStage> stages = plan_tiles(ops, n, T, L, exact_order);
+        // Choosing each stage's qubits (60..100 us of host time for 400 gates) gives fewer stages for some circuits
+        // and more for others (layers of random pairs: 27 qubits 13 for 14, complex64 19.2 ms to 17.7 ms; 24
+        // qubits 15 for 14). Taken where it gives fewer, on states of 64 MiB and more: a stage takes 60 us there.
+        if ((uint64_t(prec == QS_PREC_C64 ? 8 : 16) << n) >= (uint64_t(64) << 20)) {
+            std::vector<TileStage> searched = plan_tiles(ops, n, T, L, exact_order, kMaxStageOps, false, true);
+            if (searched.size() < stages.size()) stages.swap(searched);
+        }
         return run_tiled(state, n, prec, arith, ops, stages, s, sms, msg, nullptr, derr_dev, live);
     }
     for (size_t g = 0; g < ops.size(); g++) {
