@@ -282,10 +282,6 @@ void touch_qubits(qs_register* reg, const double* matrix, const size_t* targets,
 // up to this size; larger registers and the other forms use the parallel tree reduction.
 constexpr int kSequentialMaxQubits = 20;
 
-// Registers in the reference's arithmetic divide by sqrt(total) with the correctly rounded quotient
-// (bit-identical collapses); the other forms multiply by its reciprocal (within one ulp).
-bool exact_quotient(const qs_register* reg) { return reg->prec == QS_PREC_C128 && reg->arith == QS_ARITH_EXACT; }
-
 bool sequential_sums(const qs_register* reg) {
     return reg->prec == QS_PREC_C128 && reg->arith == QS_ARITH_EXACT && reg->n <= kSequentialMaxQubits;
 }
@@ -503,7 +499,7 @@ int qs_try_measure(qs_register* reg, size_t target, double draw, int* outcome, d
     const double d = std::sqrt(total);
     const double rinv = 1.0 / d;
     QS_CUDA(qs::launch_collapse(reg->state, reg->n, reg->prec, int(target), res, d, rinv, reg->stream, reg->sms,
-                                reg->zmask, reg->zval, exact_quotient(reg)),
+                                reg->zmask, reg->zval),
             "collapse");
     record_outcome(reg, target, res);
     if (outcome) *outcome = res;
@@ -534,7 +530,6 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
     const size_t amp = amp_bytes(reg->prec);
     void* scratch = measure_scratch(reg);
     if (!scratch) return 1;
-    const bool exactq = exact_quotient(reg);
     QS_CUDA(qs::launch_measure_probs(reg->state, n, reg->prec, int(targets[0]), reg->partials, kMaxPartials,
                                      reg->hres, reg->stream, reg->sms),
             "measure_probs");
@@ -558,7 +553,7 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
         const int next_pos = k + 1 < m ? index_of(targets[k + 1]) : -1;
         dst = (k % 2 == 0) ? scratch : reg->state;  // the first pass reads the whole state
         QS_CUDA(qs::launch_collapse_compact(src, dst, nfree, reg->prec, pos, res, d, rinv, next_pos, reg->partials,
-                                            kMaxPartials, reg->hres, reg->stream, reg->sms, exactq),
+                                            kMaxPartials, reg->hres, reg->stream, reg->sms),
                 "collapse_compact");
         record_outcome(reg, targets[k], res);
         src = dst;
@@ -629,12 +624,12 @@ int qs_measure_sequence(qs_register* reg, const size_t* targets, size_t m, const
         if (k + 1 < m && !seq) {
             QS_CUDA(qs::launch_collapse_probs(reg->state, reg->n, reg->prec, t, res, d, rinv, int(targets[k + 1]),
                                               reg->partials, kMaxPartials, reg->hres, reg->stream, reg->sms,
-                                              reg->zmask, reg->zval, exact_quotient(reg)),
+                                              reg->zmask, reg->zval),
                     "collapse_probs");
             record_outcome(reg, targets[k], res);
         } else {
             QS_CUDA(qs::launch_collapse(reg->state, reg->n, reg->prec, t, res, d, rinv, reg->stream, reg->sms,
-                                        reg->zmask, reg->zval, exact_quotient(reg)),
+                                        reg->zmask, reg->zval),
                     "collapse");
             record_outcome(reg, targets[k], res);
             if (k + 1 < m)

@@ -85,25 +85,23 @@ cudaError_t launch_measure_probs(const void* state, int n, int prec, int target,
                                  int max_partials, double* out, cudaStream_t s, int sms, uint64_t zmask = 0,
                                  uint64_t zval = 0, bool sequential = false, double* squares = nullptr);
 // Zero amplitudes whose target bit != outcome and divide the rest by d (rinv = 1/d), within the
-// live subspace: complex128 with exact_quotient as the correctly rounded quotient (Rust's `/`),
-// otherwise within one ulp of it (a multiply by rinv).
+// live subspace: complex128 as the correctly rounded quotient (Rust's `/`), complex64 as the float next to it.
 cudaError_t launch_collapse(void* state, int n, int prec, int target, int outcome, double d, double rinv,
-                            cudaStream_t s, int sms, uint64_t zmask = 0, uint64_t zval = 0,
-                            bool exact_quotient = true);
+                            cudaStream_t s, int sms, uint64_t zmask = 0, uint64_t zval = 0);
 // The same collapse, with the probability sums of next_target over the kept amplitudes written to
 // out[0], out[1] (device) in the same pass.
 cudaError_t launch_collapse_probs(void* state, int n, int prec, int target, int outcome, double d, double rinv,
                                   int next_target, double* partials, int max_partials, double* out, cudaStream_t s,
-                                  int sms, uint64_t zmask, uint64_t zval, bool exact_quotient = true);
+                                  int sms, uint64_t zmask, uint64_t zval);
 // One pass of a measurement sequence on a compact buffer: `src` holds 2^nfree amplitudes indexed by
 // the free bits in ascending order; the amplitudes whose bit `pos` equals `outcome` are divided by d
-// (rinv = 1/d; correctly rounded with exact_quotient on complex128) and written densely to `dst`
+// (rinv = 1/d; correctly rounded on complex128) and written densely to `dst`
 // (2^(nfree-1) amplitudes, bit pos removed). With next_pos >= 0, the probability sums of bit
 // next_pos of dst's index go to out[0], out[1] (device) in the same pass. Same pairs, order, grid and
 // arithmetic as launch_collapse_probs.
 cudaError_t launch_collapse_compact(const void* src, void* dst, int nfree, int prec, int pos, int outcome, double d,
                                     double rinv, int next_pos, double* partials, int max_partials, double* out,
-                                    cudaStream_t s, int sms, bool exact_quotient);
+                                    cudaStream_t s, int sms);
 // Write the 2^(n - popcount(zmask)) amplitudes of `src` (indexed by the free bits) to their places in
 // the state: the bits of zmask set to those of zval.
 cudaError_t launch_scatter_live(void* state, const void* src, int n, int prec, uint64_t zmask, uint64_t zval,

@@ -628,52 +628,89 @@ cudaError_t launch_measure_probs(const void* state, int n, int prec, int target,
     return counted(cudaGetLastError(), 2);
 }
 
-// x / d for the kept half. With rinv = RN(1/d), q = RN(x * rinv) is within
-// one ulp of x/d, and Markstein's correction (r = x - q*d exactly by FMA,
-// q' = RN(q + r*rinv); P. Markstein, IBM J. Res. Dev. 34(1), 1990) rounds
-// it to the correctly rounded quotient, the value Rust's `/` gives.
-__device__ __forceinline__ double div_markstein(double x, double d, double rinv) {
-    const double q = x * rinv;
-    const double r = fma(-q, d, x);
-    return fma(r, rinv, q);
+// How the kept amplitudes are divided by d = sqrt(total). Complex128: the correctly rounded quotient (Rust's `/`)
+// on the integer pipe (quotient). Complex64: as a pair of floats, one FP64 multiply by RN(1/d), or a true division
+// where RN(1/d) is not usable.
+constexpr int kDivTrue = 1, kDivMul = 2, kDivPair = 3;
+
+// d for integer quotients: with the 53-bit significands mx and md, mx / md 2^62 is the upper half of 2^11 mx times
+// r = floor(2^115 / md), or up to 2 less.
+struct Divisor {
+    double d, rinv;
+    uint32_t rh, rl;
+    uint32_t low, span;  // exponent fields (<< 20) of x that give a normal quotient
+    int32_t base;        // of the quotient's high word, beside x's exponent
+};
+
+static Divisor make_divisor(double d, double rinv) {
+    Divisor v;
+    std::memset(&v, 0, sizeof(v));
+    v.d = d;
+    v.rinv = rinv;
+    uint64_t bits;
+    std::memcpy(&bits, &d, 8);
+    const int e = int(bits >> 52);  // the sign is clear, or d is a NaN
+    if (!(std::isfinite(rinv) && d > 1e-300 && std::isfinite(d))) return v;  // span 0: true divisions
+    const uint64_t md = (bits & 0xfffffffffffffull) | (1ull << 52);
+    // 2^115 / md by long division: at most 2^63
+    uint64_t q = 0, rem = 0;
+    for (int i = 115; i >= 0; i--) {
+        rem = (rem << 1) | (i == 115 ? 1u : 0u);
+        q <<= 1;
+        if (rem >= md) rem -= md, q |= 1;
+    }
+    v.rh = uint32_t(q >> 32);
+    v.rl = uint32_t(q);
+    const int lo = std::max(1, e - 1020), hi = std::min(2046, e + 1020);
+    v.low = uint32_t(lo) << 20;
+    v.span = uint32_t(std::max(0, hi - lo + 1)) << 20;
+    v.base = (1021 - e) * (1 << 20);
+    return v;
 }
 
-// How the kept amplitudes are divided by d = sqrt(total): the correctly rounded quotient (Markstein's
-// step; what Rust's `/` gives, for registers in the reference's arithmetic), a true division (when
-// RN(1/d) is not usable), or one multiply by RN(1/d), within one ulp of the quotient (registers in
-// the other arithmetic forms, held to 1e-14: GB300's FP64 pipe bounds a collapse, and this form
-// takes 2 FP64 operations per amplitude instead of 6).
-constexpr int kDivMarkstein = 0, kDivTrue = 1, kDivMul = 2, kDivPair = 3;
+// x / d where the integers do not say: a quotient so near to the middle of two doubles that its missing part
+// decides (Markstein's step: with q = RN(x rinv) within an ulp, r = x - q d exactly by FMA, RN(q + r rinv) is the
+// correctly rounded quotient; P. Markstein, IBM J. Res. Dev. 34(1), 1990), and what is not normal.
+__device__ __noinline__ double quotient_rare(double x, double d, double rinv, bool middle) {
+    if (!middle) return x / d;
+    const double q = x * rinv;
+    return fma(fma(-q, d, x), rinv, q);
+}
+
+// The correctly rounded x / d: Q = mx / md 2^62 to within 2 below, rounded at bit 9 or 10. A quotient of two 53-bit
+// significands is never the middle of two doubles, so only Q's lower bits just below the middle are undecided (1 in
+// 512). FP64 took 3 instructions a component, at 64 cycles per warp and sub-partition: 27 qubits, every qubit
+// measured, 2.85 ms in the collapses then, 1.45 ms now (their traffic: 0.95 ms).
+__device__ __forceinline__ double quotient(double x, const Divisor& v) {
+    const uint32_t hi = uint32_t(__double2hiint(x)), lo = uint32_t(__double2loint(x)), h = hi & 0x7fffffffu;
+    if (h - v.low >= v.span) return (h | lo) == 0u && v.span ? x : quotient_rare(x, v.d, v.rinv, false);
+    const uint32_t xh = __funnelshift_l(lo, hi, 11) | 0x80000000u, xl = lo << 11;
+    const uint64_t t = im_madw(xl, v.rl, 0ull);
+    const uint64_t u = im_madw(xh, v.rl, t >> 32);
+    const uint64_t w = im_madw(xl, v.rh, u & 0xffffffffull);
+    const uint64_t Q = im_madw(xh, v.rh, u >> 32) + (w >> 32);
+    const uint32_t top = uint32_t(Q >> 62);  // 1: the quotient of the significands is 1 or more
+    const uint64_t q = Q << (1u - top);
+    if ((uint32_t(q) & 1023u) == 510u + top) return quotient_rare(x, v.d, v.rinv, true);
+    const uint64_t r = (q + 512u) >> 10;  // the implicit bit (and a carry) adds to the exponent
+    const uint32_t rh = uint32_t(r >> 32) + (h & 0x7ff00000u) + uint32_t(v.base) + (top << 20);
+    return __hiloint2double(int(rh | (hi & 0x80000000u)), int(uint32_t(r)));
+}
 
 // The kept amplitude divided by sqrt(total) (src/register.rs:337), in the state's type.
-template <typename T, int DIV>
-__device__ __forceinline__ T collapse_value(T v, double d, double rinv, double2* as_double) {
-    if constexpr (sizeof(T) == 8 && DIV != kDivTrue) {
-        // complex64: one FP64 multiply by RN(1/d) per component, rounded to float on the integer
-        // pipe (the quotient is stored as a float, so the exactly rounded double quotient of the
-        // complex128 path buys nothing here)
-        const double2 x = to_d2_int(v);
-        const T y{d2f_int(x.x * rinv), d2f_int(x.y * rinv)};
-        *as_double = make_double2(df_f2d(y.x), df_f2d(y.y));
-        return y;
-    } else {
-        const double2 x = to_d2_int(v);
-        double2 y;
-        if constexpr (DIV == kDivTrue) {
-            y.x = x.x / d;
-            y.y = x.y / d;
-        } else if constexpr (DIV == kDivMul) {
-            y.x = x.x * rinv;
-            y.y = x.y * rinv;
-        } else {
-            y.x = div_markstein(x.x, d, rinv);
-            y.y = div_markstein(x.y, d, rinv);
-        }
-        T r;
-        from_d2(&r, y);
-        *as_double = to_d2_int(r);
-        return r;
-    }
+__device__ __forceinline__ double2 collapse_value(double2 v, const Divisor& d) {
+    return make_double2(quotient(v.x, d), quotient(v.y, d));
+}
+template <int DIV>
+__device__ __forceinline__ float2 collapse_value(float2 v, double d, double rinv, double2* as_double) {
+    const double2 x = to_d2_int(v);
+    float2 y;
+    if constexpr (DIV == kDivTrue)
+        y = make_float2(float(x.x / d), float(x.y / d));
+    else  // rounded to float on the integer pipe
+        y = make_float2(d2f_int(x.x * rinv), d2f_int(x.y * rinv));
+    *as_double = make_double2(df_f2d(y.x), df_f2d(y.y));
+    return y;
 }
 
 // Complex64 collapse on the FP32 and integer pipes. 1/d = rh + rl to 48 bits, so p = x rh rounded, its
@@ -747,7 +784,7 @@ __device__ __forceinline__ void collapse_chunks(uint64_t npairs, double d, doubl
                 const uint64_t t = t0 + uint64_t(j) * kT;
                 if (t >= npairs) break;
                 double2 y;
-                *dst(t) = collapse_value<float2, DIV == kDivPair ? kDivMul : DIV>(*src(t), d, rinv, &y);
+                *dst(t) = collapse_value<DIV == kDivPair ? kDivMul : DIV>(*src(t), d, rinv, &y);
                 drop(t);
                 const double q = fma(y.x, y.x, y.y * y.y);
                 const bool o = SUMS && one(t);
@@ -767,7 +804,7 @@ __device__ __forceinline__ void collapse_chunks(uint64_t npairs, double d, doubl
     }
 }
 
-// In place: the pass of k_collapse, and with SUMS of k_collapse_probs.
+// In place, as k_collapse.
 template <int DIV, bool SUMS>
 __global__ void __launch_bounds__(kT, kSqBlocks)
     k_collapse_c64(float2* st, uint64_t npairs, uint64_t tb, const __grid_constant__ IndexMap map, int outcome, double d,
@@ -793,110 +830,73 @@ static int collapse_grid(uint64_t npairs, int prec, int sms) {
     return prec == QS_PREC_C64 ? std::min(grid_cap(npairs, sms, kSqChunk), kSqBlocks * sms) : grid_cap(npairs, sms, 2);
 }
 
-template <typename T, int DIV>
-__global__ void __launch_bounds__(kT) k_collapse(T* __restrict__ st, uint64_t npairs, uint64_t tb,
-                                                 const __grid_constant__ IndexMap map, int outcome, double d,
-                                                 double rinv) {
-    const uint64_t stride = uint64_t(gridDim.x) * kT;
-    for (uint64_t t = uint64_t(blockIdx.x) * kT + threadIdx.x; t < npairs; t += stride) {
-        const uint64_t i0 = expand_index(t, map);
-        const uint64_t keep = outcome ? (i0 | tb) : i0, drop = outcome ? i0 : (i0 | tb);
-        double2 unused;
-        st[keep] = collapse_value<T, DIV>(st[keep], d, rinv, &unused);
-        st[drop] = T{0, 0};
-    }
-}
-
-// The collapse of one measurement fused with the probability sums of the next one (measure_circuit,
-// src/register.rs:371-377): the kept amplitudes, once divided, are the only non-zero amplitudes the
-// next target sees, so their squares are summed by that target's bit in the same pass.
-template <typename T, int DIV>
-__global__ void __launch_bounds__(kT) k_collapse_probs(T* __restrict__ st, uint64_t npairs, uint64_t tb,
-                                                       const __grid_constant__ IndexMap map, int outcome, double d,
-                                                       double rinv, uint64_t next_tb, double* __restrict__ partials) {
+// In place on complex128. With SUMS, the collapse of one measurement fused with the probability sums of the next
+// one (measure_circuit, src/register.rs:371-377): the kept amplitudes, once divided, are the only non-zero
+// amplitudes the next target sees, so their squares are summed by that target's bit in the same pass.
+template <bool SUMS>
+__global__ void __launch_bounds__(kT) k_collapse(double2* __restrict__ st, uint64_t npairs, uint64_t tb,
+                                                 const __grid_constant__ IndexMap map, int outcome,
+                                                 const __grid_constant__ Divisor d, uint64_t next_tb,
+                                                 double* __restrict__ partials) {
     const uint64_t stride = uint64_t(gridDim.x) * kT;
     double p0 = 0.0, p1 = 0.0;
     for (uint64_t t = uint64_t(blockIdx.x) * kT + threadIdx.x; t < npairs; t += stride) {
         const uint64_t i0 = expand_index(t, map);
         const uint64_t keep = outcome ? (i0 | tb) : i0, drop = outcome ? i0 : (i0 | tb);
-        double2 y;
-        st[keep] = collapse_value<T, DIV>(st[keep], d, rinv, &y);
-        st[drop] = T{0, 0};
-        const double q = fma(y.x, y.x, y.y * y.y);
-        if (keep & next_tb)
-            p1 += q;
-        else
-            p0 += q;
+        const double2 y = collapse_value(st[keep], d);
+        st[keep] = y;
+        st[drop] = make_double2(0.0, 0.0);
+        if constexpr (SUMS) {
+            const double q = fma(y.x, y.x, y.y * y.y);
+            if (keep & next_tb)
+                p1 += q;
+            else
+                p0 += q;
+        }
     }
-    block_sum2(p0, p1);
-    if (threadIdx.x == 0) {
-        partials[2 * blockIdx.x] = p0;
-        partials[2 * blockIdx.x + 1] = p1;
+    if constexpr (SUMS) {
+        block_sum2(p0, p1);
+        if (threadIdx.x == 0) {
+            partials[2 * blockIdx.x] = p0;
+            partials[2 * blockIdx.x + 1] = p1;
+        }
     }
-}
-
-static int div_mode(double d, double rinv, bool exact_quotient) {
-    // Markstein's step and the multiply need a finite reciprocal of a normal divisor.
-    if (!(std::isfinite(rinv) && d > 1e-300 && std::isfinite(d))) return kDivTrue;
-    return exact_quotient ? kDivMarkstein : kDivMul;
 }
 
 // Complex64 multiplies by RN(1/d) unless it must divide: as a pair of floats where both fit well inside
 // their range.
 static int div_mode_c64(double d, double rinv) {
-    const int mode = div_mode(d, rinv, false);
-    return mode == kDivMul && rinv > 0x1p-60 && rinv < 0x1p60 ? kDivPair : mode;
-}
-
-template <typename T, int DIV>
-static void collapse_t(void* state, uint64_t npairs, uint64_t tb, const IndexMap& map, int outcome, double d,
-                       double rinv, int grid, cudaStream_t s) {
-    k_collapse<T, DIV><<<grid, kT, 0, s>>>((T*)state, npairs, tb, map, outcome, d, rinv);
-}
-
-template <typename T, int DIV>
-static void collapse_probs_t(void* state, uint64_t npairs, uint64_t tb, const IndexMap& map, int outcome, double d,
-                             double rinv, uint64_t ntb, double* partials, int grid, cudaStream_t s) {
-    k_collapse_probs<T, DIV><<<grid, kT, 0, s>>>((T*)state, npairs, tb, map, outcome, d, rinv, ntb, partials);
+    if (!(std::isfinite(rinv) && d > 1e-300 && std::isfinite(d))) return kDivTrue;
+    return rinv > 0x1p-60 && rinv < 0x1p60 ? kDivPair : kDivMul;
 }
 
 cudaError_t launch_collapse(void* state, int n, int prec, int target, int outcome, double d, double rinv,
-                            cudaStream_t s, int sms, uint64_t zmask, uint64_t zval, bool exact_quotient) {
+                            cudaStream_t s, int sms, uint64_t zmask, uint64_t zval) {
     const IndexMap map = subspace_map(target, zmask, zval);
     const uint64_t npairs = subspace_pairs(n, target, zmask);
     const uint64_t tb = 1ull << target;
     const int grid = collapse_grid(npairs, prec, sms);
-    const int mode = prec == QS_PREC_C64 ? div_mode_c64(d, rinv) : div_mode(d, rinv, exact_quotient);
-    if (prec == QS_PREC_C64) {
-        collapse_c64<false>(state, npairs, tb, map, outcome, d, rinv, mode, 0, nullptr, grid, s);
-    } else if (mode == kDivTrue) {
-        collapse_t<double2, kDivTrue>(state, npairs, tb, map, outcome, d, rinv, grid, s);
-    } else if (mode == kDivMul) {
-        collapse_t<double2, kDivMul>(state, npairs, tb, map, outcome, d, rinv, grid, s);
-    } else {
-        collapse_t<double2, kDivMarkstein>(state, npairs, tb, map, outcome, d, rinv, grid, s);
-    }
+    if (prec == QS_PREC_C64)
+        collapse_c64<false>(state, npairs, tb, map, outcome, d, rinv, div_mode_c64(d, rinv), 0, nullptr, grid, s);
+    else
+        k_collapse<false><<<grid, kT, 0, s>>>(static_cast<double2*>(state), npairs, tb, map, outcome,
+                                              make_divisor(d, rinv), 0, nullptr);
     return counted(cudaGetLastError());
 }
 
 cudaError_t launch_collapse_probs(void* state, int n, int prec, int target, int outcome, double d, double rinv,
                                   int next_target, double* partials, int max_partials, double* out, cudaStream_t s,
-                                  int sms, uint64_t zmask, uint64_t zval, bool exact_quotient) {
+                                  int sms, uint64_t zmask, uint64_t zval) {
     const IndexMap map = subspace_map(target, zmask, zval);
     const uint64_t npairs = subspace_pairs(n, target, zmask);
     const uint64_t tb = 1ull << target, ntb = 1ull << next_target;
     int grid = collapse_grid(npairs, prec, sms);
     if (grid > max_partials) grid = max_partials;
-    const int mode = prec == QS_PREC_C64 ? div_mode_c64(d, rinv) : div_mode(d, rinv, exact_quotient);
-    if (prec == QS_PREC_C64) {
-        collapse_c64<true>(state, npairs, tb, map, outcome, d, rinv, mode, ntb, partials, grid, s);
-    } else if (mode == kDivTrue) {
-        collapse_probs_t<double2, kDivTrue>(state, npairs, tb, map, outcome, d, rinv, ntb, partials, grid, s);
-    } else if (mode == kDivMul) {
-        collapse_probs_t<double2, kDivMul>(state, npairs, tb, map, outcome, d, rinv, ntb, partials, grid, s);
-    } else {
-        collapse_probs_t<double2, kDivMarkstein>(state, npairs, tb, map, outcome, d, rinv, ntb, partials, grid, s);
-    }
+    if (prec == QS_PREC_C64)
+        collapse_c64<true>(state, npairs, tb, map, outcome, d, rinv, div_mode_c64(d, rinv), ntb, partials, grid, s);
+    else
+        k_collapse<true><<<grid, kT, 0, s>>>(static_cast<double2*>(state), npairs, tb, map, outcome,
+                                             make_divisor(d, rinv), ntb, partials);
     k_prob_final<<<1, kT, 0, s>>>(partials, grid, out);
     return counted(cudaGetLastError(), 2);
 }
@@ -907,19 +907,19 @@ cudaError_t launch_collapse_probs(void* state, int n, int prec, int target, int 
 // move whole 32-byte sectors for every live 16-byte amplitude. Here each pass instead reads the
 // kept half of a buffer whose index runs over the free bits only and writes it, divided, densely
 // into the next buffer; the sums of the next target come from the same pass. Every pass visits the
-// pairs t in the order and with the grid of k_collapse_probs (the free bits in ascending order, the
+// pairs t in the order and with the grid of k_collapse (the free bits in ascending order, the
 // target's bit inserted) and divides as it does, so the sums, outcomes and divided amplitudes are
 // bit for bit those of the in-place passes.
-template <typename T, int DIV, bool SUMS>
-__global__ void __launch_bounds__(kT) k_collapse_compact(const T* __restrict__ src, T* __restrict__ dst,
+template <bool SUMS>
+__global__ void __launch_bounds__(kT) k_collapse_compact(const double2* __restrict__ src, double2* __restrict__ dst,
                                                          uint64_t npairs, const __grid_constant__ IndexMap map,
-                                                         uint64_t keepbit, double d, double rinv, uint64_t next_bit,
-                                                         double* __restrict__ partials) {
+                                                         uint64_t keepbit, const __grid_constant__ Divisor d,
+                                                         uint64_t next_bit, double* __restrict__ partials) {
     const uint64_t stride = uint64_t(gridDim.x) * kT;
     double p0 = 0.0, p1 = 0.0;
     for (uint64_t t = uint64_t(blockIdx.x) * kT + threadIdx.x; t < npairs; t += stride) {
-        double2 y;
-        dst[t] = collapse_value<T, DIV>(src[expand_index(t, map) | keepbit], d, rinv, &y);
+        const double2 y = collapse_value(src[expand_index(t, map) | keepbit], d);
+        dst[t] = y;
         if constexpr (SUMS) {
             const double q = fma(y.x, y.x, y.y * y.y);
             if (t & next_bit)
@@ -959,38 +959,25 @@ static void collapse_compact_c64(const void* src, void* dst, uint64_t npairs, co
                           SUMS ? 1ull << next_pos : 0ull, partials);
 }
 
-template <typename T, int DIV>
-static void collapse_compact_t(const void* src, void* dst, uint64_t npairs, const IndexMap& map, uint64_t keepbit,
-                               double d, double rinv, int next_pos, double* partials, int grid, cudaStream_t s) {
-    if (next_pos >= 0)
-        k_collapse_compact<T, DIV, true><<<grid, kT, 0, s>>>((const T*)src, (T*)dst, npairs, map, keepbit, d, rinv,
-                                                             1ull << next_pos, partials);
-    else
-        k_collapse_compact<T, DIV, false><<<grid, kT, 0, s>>>((const T*)src, (T*)dst, npairs, map, keepbit, d, rinv,
-                                                              0ull, partials);
-}
-
 cudaError_t launch_collapse_compact(const void* src, void* dst, int nfree, int prec, int pos, int outcome, double d,
                                     double rinv, int next_pos, double* partials, int max_partials, double* out,
-                                    cudaStream_t s, int sms, bool exact_quotient) {
+                                    cudaStream_t s, int sms) {
     const IndexMap map = subspace_map(pos, 0, 0);
     const uint64_t npairs = 1ull << (nfree - 1);
     const uint64_t keepbit = outcome ? (1ull << pos) : 0ull;
     int grid = collapse_grid(npairs, prec, sms);
     if (next_pos >= 0 && grid > max_partials) grid = max_partials;  // the in-place pass's grid
-    const int mode = prec == QS_PREC_C64 ? div_mode_c64(d, rinv) : div_mode(d, rinv, exact_quotient);
+    const uint64_t nb = next_pos >= 0 ? 1ull << next_pos : 0ull;
     if (prec == QS_PREC_C64) {
+        const int mode = div_mode_c64(d, rinv);
         if (next_pos >= 0)
             collapse_compact_c64<true>(src, dst, npairs, map, keepbit, d, rinv, mode, next_pos, partials, grid, s);
         else
             collapse_compact_c64<false>(src, dst, npairs, map, keepbit, d, rinv, mode, 0, nullptr, grid, s);
-    } else if (mode == kDivTrue) {
-        collapse_compact_t<double2, kDivTrue>(src, dst, npairs, map, keepbit, d, rinv, next_pos, partials, grid, s);
-    } else if (mode == kDivMul) {
-        collapse_compact_t<double2, kDivMul>(src, dst, npairs, map, keepbit, d, rinv, next_pos, partials, grid, s);
     } else {
-        collapse_compact_t<double2, kDivMarkstein>(src, dst, npairs, map, keepbit, d, rinv, next_pos, partials, grid,
-                                                   s);
+        auto k = next_pos >= 0 ? k_collapse_compact<true> : k_collapse_compact<false>;
+        k<<<grid, kT, 0, s>>>(static_cast<const double2*>(src), static_cast<double2*>(dst), npairs, map, keepbit,
+                              make_divisor(d, rinv), nb, partials);
     }
     if (next_pos < 0) return counted(cudaGetLastError());
     k_prob_final<<<1, kT, 0, s>>>(partials, grid, out);
