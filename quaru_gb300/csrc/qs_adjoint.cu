@@ -83,10 +83,22 @@ struct PauliDev {
     uint32_t pad_;
 };
 
-// out_i = sum_t c_t * i^{|x&z|} * (-1)^{|z & (i^x)|} * psi_{i^x}
+// out_i = sum_t c_t * i^{|x&z|} * (-1)^{|z & (i^x)|} * psi_{i^x}, and the block's part of Re <psi|out> (out as
+// it is stored). A pass of its own for the inner product read both vectors again: 25 us at 20 qubits, and two more
+// links in the chain of launches that a gradient of a small state waits for.
 template <typename T, bool DFC>
 __global__ void __launch_bounds__(kAT) k_pauli_sum(const T* __restrict__ psi, T* __restrict__ out, uint64_t N,
-                                                   const PauliDev* __restrict__ terms, int nt) {
+                                                   const PauliDev* __restrict__ terms, int nt,
+                                                   double* __restrict__ partials) {
+    double energy = 0.0, none = 0.0;
+    auto put = [&](uint64_t i, T v) {
+        out[i] = v;
+        const double2 a = ld2(psi, i), b = ld2(&v, 0);
+        energy = fma(a.x, b.x, fma(a.y, b.y, energy));
+    };
+    // the parity of z & j: the qubits of most states fit one word
+    const bool narrow = N <= (1ull << 32);
+    auto odd = [&](uint64_t zj) { return ((narrow ? __popc(uint32_t(zj)) : __popcll(zj)) & 1) != 0; };
     static_assert(!DFC || sizeof(T) == 8, "float-pair coefficients serve complex64 states");
     if constexpr (DFC) {
         // complex64: each term's product by TwoProduct on the FP32 pipe, summed with TwoSum (DfAcc), the
@@ -97,7 +109,7 @@ __global__ void __launch_bounds__(kAT) k_pauli_sum(const T* __restrict__ psi, T*
                 const PauliDev& p = terms[t];
                 const uint64_t j = i ^ p.x;
                 const float2 v = reinterpret_cast<const float2*>(psi)[j];
-                const bool neg = __popcll(p.z & j) & 1;
+                const bool neg = odd(p.z & j);
                 const float ch = neg ? -p.ch : p.ch, cl = neg ? -p.cl : p.cl;
                 float xr, xi;  // i^cls * v
                 switch (p.cls) {
@@ -111,7 +123,7 @@ __global__ void __launch_bounds__(kAT) k_pauli_sum(const T* __restrict__ psi, T*
                 im.add_prod(ch, xi);
                 im.c = __fmaf_rn(cl, xi, im.c);
             }
-            reinterpret_cast<float2*>(out)[i] = make_float2(__fadd_rn(re.s, re.c), __fadd_rn(im.s, im.c));
+            put(i, make_float2(__fadd_rn(re.s, re.c), __fadd_rn(im.s, im.c)));
         }
     } else {
         for (uint64_t i = uint64_t(blockIdx.x) * kAT + threadIdx.x; i < N; i += uint64_t(gridDim.x) * kAT) {
@@ -121,28 +133,35 @@ __global__ void __launch_bounds__(kAT) k_pauli_sum(const T* __restrict__ psi, T*
                 const uint64_t j = i ^ p.x;
                 const double2 v = ld2(psi, j);
                 double c = p.c;
-                if (__popcll(p.z & j) & 1) c = -c;
-                switch (__popcll(p.x & p.z) & 3) {
+                if (odd(p.z & j)) c = -c;
+                switch (p.cls) {
                     case 0: re = fma(c, v.x, re); im = fma(c, v.y, im); break;
                     case 1: re = fma(-c, v.y, re); im = fma(c, v.x, im); break;  // i * v
                     case 2: re = fma(-c, v.x, re); im = fma(-c, v.y, im); break;
                     default: re = fma(c, v.y, re); im = fma(-c, v.x, im); break;  // -i * v
                 }
             }
-            st2(out, i, make_double2(re, im));
+            T v;
+            st2(&v, 0, make_double2(re, im));
+            put(i, v);
         }
     }
+    rd_block_sum2<kAT>(energy, none);
+    if (threadIdx.x == 0) partials[blockIdx.x] = energy;
 }
 
-// Block g sums partials[g * nblocks .. (g+1) * nblocks) into out[g], times weights[at[g]] (at[g] < 0: 1).
-__global__ void __launch_bounds__(kAT) k_grad_final(const double* __restrict__ partials, int nblocks,
+// Block 0 sums the nenergy partials of the energy into out[0]; block g + 1 sums partials[g * nblocks ..
+// (g + 1) * nblocks) into out[g + 1], times weights[at[g]] (at[g] < 0: 1).
+__global__ void __launch_bounds__(kAT) k_grad_final(const double* __restrict__ energy, int nenergy,
+                                                    const double* __restrict__ partials, int nblocks,
                                                     const double* __restrict__ weights, const int* __restrict__ at,
                                                     double* __restrict__ out) {
-    const double* p = partials + size_t(blockIdx.x) * nblocks;
+    const int g = int(blockIdx.x) - 1, count = g < 0 ? nenergy : nblocks;
+    const double* p = g < 0 ? energy : partials + size_t(g) * nblocks;
     double a = 0.0, b = 0.0;
-    for (int i = threadIdx.x; i < nblocks; i += kAT) a += p[i];
+    for (int i = threadIdx.x; i < count; i += kAT) a += p[i];
     rd_block_sum2<kAT>(a, b);
-    if (threadIdx.x == 0) out[blockIdx.x] = at[blockIdx.x] < 0 ? a : a * weights[at[blockIdx.x]];
+    if (threadIdx.x == 0) out[blockIdx.x] = g < 0 || at[g] < 0 ? a : a * weights[at[g]];
 }
 
 // ---------------------------------------------------------------- tiled sweeps
@@ -399,15 +418,19 @@ static bool pauli_df_ok(const std::vector<PauliDev>& ht) {
     return true;
 }
 
+// Returns the number of blocks: partials of the energy written (at most 16 per SM).
 template <typename T>
-static void launch_pauli_sum(const void* psi, void* out, int n, const PauliDev* dterms, int nt, bool df_ok,
-                             cudaStream_t s, int sms) {
+static int launch_pauli_sum(const void* psi, void* out, int n, const PauliDev* dterms, int nt, bool df_ok,
+                            double* partials, cudaStream_t s, int sms) {
     const uint64_t N = 1ull << n;
+    const int grid = grid_for_pairs(N, sms);
     if (sizeof(T) == 8 && df_ok)
-        k_pauli_sum<float2, true><<<grid_for_pairs(N, sms), kAT, 0, s>>>((const float2*)psi, (float2*)out, N, dterms, nt);
+        k_pauli_sum<float2, true>
+            <<<grid, kAT, 0, s>>>((const float2*)psi, (float2*)out, N, dterms, nt, partials);
     else
-        k_pauli_sum<T, false><<<grid_for_pairs(N, sms), kAT, 0, s>>>((const T*)psi, (T*)out, N, dterms, nt);
+        k_pauli_sum<T, false><<<grid, kAT, 0, s>>>((const T*)psi, (T*)out, N, dterms, nt, partials);
     note_launches(1);
+    return grid;
 }
 
 int expval_pauli(const void* psi, int prec, int n, const qs_pauli_term* terms, size_t nt, cudaStream_t s, int sms,
@@ -419,21 +442,25 @@ int expval_pauli(const void* psi, int prec, int n, const qs_pauli_term* terms, s
     const size_t o_terms = 0, o_part = ((nt * sizeof(PauliDev) + 255) / 256) * 256, o_res = o_part + 4096 * 16,
                  o_lam = o_res + 256, total = o_lam + N * amp;
     std::vector<PauliDev> ht = pauli_table(terms, nt);
-    double res[2] = {0, 0};
+    double res = 0.0;
+    int blocks = 0;
     AJ_CHECK(device_alloc((void**)&blob, total, s), "expval buffers");
     if (nt) AJ_CHECK(cudaMemcpyAsync(blob + o_terms, ht.data(), nt * sizeof(PauliDev), cudaMemcpyHostToDevice, s),
                      "terms upload");
     if (prec == QS_PREC_C64)
-        launch_pauli_sum<float2>(psi, blob + o_lam, n, (const PauliDev*)(blob + o_terms), int(nt), pauli_df_ok(ht),
-                                 s, sms);
+        blocks = launch_pauli_sum<float2>(psi, blob + o_lam, n, (const PauliDev*)(blob + o_terms), int(nt),
+                                          pauli_df_ok(ht), (double*)(blob + o_part), s, sms);
     else
-        launch_pauli_sum<double2>(psi, blob + o_lam, n, (const PauliDev*)(blob + o_terms), int(nt), false, s, sms);
+        blocks = launch_pauli_sum<double2>(psi, blob + o_lam, n, (const PauliDev*)(blob + o_terms), int(nt), false,
+                                           (double*)(blob + o_part), s, sms);
     AJ_CHECK(cudaGetLastError(), "pauli sum");
-    if (inner_product(psi, prec, blob + o_lam, prec, n, s, sms, (double*)(blob + o_part), (double*)(blob + o_res)))
-        AJ_CHECK(cudaGetLastError(), "inner product");
-    AJ_CHECK(cudaMemcpyAsync(res, blob + o_res, 16, cudaMemcpyDeviceToHost, s), "expval readback");
+    k_grad_final<<<1, kAT, 0, s>>>((const double*)(blob + o_part), blocks, nullptr, 0, nullptr, nullptr,
+                                   (double*)(blob + o_res));
+    note_launches(1);
+    AJ_CHECK(cudaGetLastError(), "energy");
+    AJ_CHECK(cudaMemcpyAsync(&res, blob + o_res, sizeof(res), cudaMemcpyDeviceToHost, s), "expval readback");
     AJ_CHECK(cudaStreamSynchronize(s), "expval sync");
-    *value = res[0];
+    *value = res;
 done:
     if (blob) cudaFreeAsync(blob, s);
     return rc;
@@ -839,10 +866,9 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
     auto al = [](size_t x) { return ((x + 255) / 256) * 256; };
     const size_t o_terms = 0, o_part = o_terms + al(nt * sizeof(PauliDev) + 1),
                  o_res = o_part + al(size_t(std::max(nrot, 1)) * pgrid * 8 + 4096 * 16),
-                 o_err = o_res + al((2 + size_t(nrot)) * 8), o_lam = o_err + al(sizeof(int)),
-                 o_psi = o_lam + al(N * amp), total = o_psi + N * amp;
+                 o_lam = o_res + al((2 + size_t(nrot)) * 8), o_psi = o_lam + al(N * amp), total = o_psi + N * amp;
     unsigned char* blob = nullptr;
-    std::vector<double> res(2 + nrot, 0.0);
+    std::vector<double> res(2 + nrot, 0.0);  // the energy, the rotations' terms, the status: one readback
     std::vector<double2> angles(std::max<size_t>(m, 1), make_double2(1.0, 0.0));  // per gate: cos, sin of theta / 2
     for (size_t g = 0; g < m; g++)
         if (rot_slot[g] >= 0) {
@@ -861,11 +887,12 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
         if (nt)
             AJ_CHECK(cudaMemcpyAsync(blob + o_terms, ht.data(), nt * sizeof(PauliDev), cudaMemcpyHostToDevice, s),
                      "terms upload");
-        int* derr = reinterpret_cast<int*>(blob + o_err);  // raised by a forward tile kernel's bounded wait
-        AJ_CHECK(cudaMemsetAsync(derr, 0, sizeof(int), s), "status flag");
-        int herr = 0;
+        int* derr = reinterpret_cast<int*>(dres + 1 + nrot);  // raised by a forward tile kernel's bounded wait
+        int blocks = 0;  // of the energy's partials
+        double* epart = part + size_t(std::max(nrot, 1)) * pgrid;
         // forward
         if (df) {
+            AJ_CHECK(cudaMemsetAsync(derr, 0, sizeof(double), s), "status flag");
             AJ_CHECK(cudaMemcpyAsync(psi, state, N * amp, cudaMemcpyDeviceToDevice, s), "state copy");
             std::vector<OpDesc> fops(m);
             std::vector<double> rmat(8 * m);  // the rotations' matrices, in gate order
@@ -907,27 +934,27 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
         }
         // lambda = H psi, E = Re<psi|lambda>
         if (prec == QS_PREC_C64)
-            launch_pauli_sum<float2>(psi, lam, n, (const PauliDev*)(blob + o_terms), int(nt), pauli_df_ok(ht), s, sms);
+            blocks = launch_pauli_sum<float2>(psi, lam, n, (const PauliDev*)(blob + o_terms), int(nt), pauli_df_ok(ht),
+                                              epart, s, sms);
         else
-            launch_pauli_sum<double2>(psi, lam, n, (const PauliDev*)(blob + o_terms), int(nt), false, s, sms);
+            blocks = launch_pauli_sum<double2>(psi, lam, n, (const PauliDev*)(blob + o_terms), int(nt), false, epart, s,
+                                               sms);
         AJ_CHECK(cudaGetLastError(), "pauli sum");
-        if (inner_product(psi, prec, lam, prec, n, s, sms, part + size_t(std::max(nrot, 1)) * pgrid, dres))
-            AJ_CHECK(cudaGetLastError(), "energy");
         // reverse
         plan_sweep(gates, m, angles.data(), rot_slot, nrot, inv, n, tq, true, type, df, !unitary, &rplan);
         if ((rc = upload_sweep(rplan, angles, 1, s, &rtab, msg)) != QS_OK) goto done;
         if ((rc = run_sweep(rplan, rtab, nullptr, psi, lam, n, prec, arith, true, rot_slot, part, pgrid, s, sms, msg)) !=
             QS_OK)
             goto done;
-        if (nrot) {
-            k_grad_final<<<nrot, kAT, 0, s>>>(part, pgrid, rtab.weights, rtab.weight_at, dres + 2);
-            note_launches(1);
-            AJ_CHECK(cudaGetLastError(), "gradient reduction");
-        }
-        AJ_CHECK(cudaMemcpyAsync(res.data(), dres, res.size() * 8, cudaMemcpyDeviceToHost, s), "readback");
-        AJ_CHECK(cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, s), "status readback");
+        k_grad_final<<<1 + nrot, kAT, 0, s>>>(epart, blocks, part, pgrid, rtab.weights, rtab.weight_at, dres);
+        note_launches(1);
+        AJ_CHECK(cudaGetLastError(), "gradient reduction");
+        AJ_CHECK(cudaMemcpyAsync(res.data(), dres, (1 + size_t(nrot) + (df ? 1 : 0)) * 8, cudaMemcpyDeviceToHost, s),
+                 "readback");
         AJ_CHECK(cudaStreamSynchronize(s), "adjoint sync");
-        if (herr) {
+        int herr = 0;
+        std::memcpy(&herr, &res[1 + nrot], sizeof(herr));
+        if (df && herr) {
             *msg = "a tile kernel's bounded wait for its bulk copies gave up";
             rc = QS_TIMEOUT;
             goto done;
@@ -936,7 +963,7 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
         if (grad) {
             for (size_t p = 0; p < np; p++) grad[p] = 0.0;
             for (size_t g = 0; g < m; g++)
-                if (rot_slot[g] >= 0) grad[gates[g].param] += res[2 + rot_slot[g]];
+                if (rot_slot[g] >= 0) grad[gates[g].param] += res[1 + rot_slot[g]];
         }
     }
 done:
