@@ -823,10 +823,11 @@ __device__ __forceinline__ void fx_warp_norm(const double2* raw, uint32_t tsize,
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) box[threadIdx.x >> 5] = FxWarpNorm{int(e), s};
 }
-__device__ __forceinline__ bool fx_scale(const FxWarpNorm* box, int nwarps, int* k) {
+// Returns the tile's largest exponent field: 0 without a normal number, 0x7ff with an infinity or NaN.
+__device__ __forceinline__ int fx_scale(const FxWarpNorm* box, int nwarps, int* k) {
     int e = 0;
     for (int w = 0; w < nwarps; w++) e = max(e, box[w].e);
-    if (e == 0x7ff) return false;
+    if (e == 0x7ff) return e;
     float sum = 0.0f;
     for (int w = 0; w < nwarps; w++) {
         const int d = 2 * (e - box[w].e);
@@ -835,7 +836,7 @@ __device__ __forceinline__ bool fx_scale(const FxWarpNorm* box, int nwarps, int*
     // squares of truncated values: a margin of 2^-18; norm^2 < 2^(h + 1) 2^(2 (e - 1023))
     const int h = int(__float_as_uint(sum * 1.000004f) >> 23) - 127;
     *k = sum > 0.0f ? 60 - ((h + 2) >> 1) - (e - 1023) : 0;
-    return true;
+    return e;
 }
 
 // Shared memory of a program beside its tiles, in this order.
@@ -1038,24 +1039,35 @@ __device__ __forceinline__ void sw_tile(const typename Sw<T>::Glob* src, typenam
         *g = gp + (side.rowoff[i >> t.RL] + (i & rmask));
         *at = ap ^ S::at(i);
     };
+    // A tile of zeros goes through no program (from a basis state most tiles of a forward run's first stages are:
+    // 20 qubits, 12 stages). Fixed-point tiles know from their norm; complex64 tiles OR their bits, and a program
+    // with a dense fixed gate runs all the same: its entries may overflow a float.
+    uint32_t any = 0;
 #pragma unroll 8
     for (uint32_t i = 0; i + p < tsize; i += nt) {
         uint64_t g;
         uint32_t at;
         place(i, &g, &at);
-        rp[at] = CG ? __ldcg(src + g) : src[g];
-        if (REV) rl[at] = CG ? __ldcg(lam + g) : lam[g];
+        const G v = CG ? __ldcg(src + g) : src[g];
+        rp[at] = v;
+        if constexpr (sizeof(T) == 8) any |= (__float_as_uint(v.x) | __float_as_uint(v.y)) << 1;
+        if (REV) {
+            const G w = CG ? __ldcg(lam + g) : lam[g];
+            rl[at] = w;
+            if constexpr (sizeof(T) == 8) any |= (__float_as_uint(w.x) | __float_as_uint(w.y)) << 1;
+        }
     }
     int kp = 0, kl = 0;
     double unit = 1.0;
-    bool finite = true;
+    bool finite = true, live = true;
     if constexpr (FX) {  // each thread converts the elements it loaded
         const int nw = (nt + 31) / 32;
         fx_warp_norm(rp, tsize, nt, side.box);
         if (REV) fx_warp_norm(rl, tsize, nt, side.box + kSwWarps);
         __syncthreads();
-        finite = fx_scale(side.box, nw, &kp);
-        if (REV) finite = fx_scale(side.box + kSwWarps, nw, &kl) && finite;
+        const int ep = fx_scale(side.box, nw, &kp), el = REV ? fx_scale(side.box + kSwWarps, nw, &kl) : 0;
+        finite = ep != 0x7ff && el != 0x7ff;
+        live = finite && (ep | el) != 0;
         if (finite) {
             const int eu = 1023 + 60 - kp - kl;
             unit = eu > 0 && eu < 2047 ? __hiloint2double(eu << 20, 0) : fx_to_double_any(1, eu - 1023);
@@ -1070,8 +1082,13 @@ __device__ __forceinline__ void sw_tile(const typename Sw<T>::Glob* src, typenam
             }
         }
     }
-    __syncthreads();
-    if (!FX || finite) {
+    if constexpr (sizeof(T) == 8) {
+        live = __syncthreads_or(any != 0);
+        for (int k = 0; k < t.npass && !live; k++) live = side.passes[k].kind == SW_FIXED;
+    } else {
+        __syncthreads();
+    }
+    if (live) {
         sw_program<T, RB, REV>(sp, sl, t.T, base, side.passes, t.npass, fixed, side.coef, side.tables, side.sacc, nt);
     }
     if constexpr (FX && REV) {  // the tile's sums on its own scale (undefined with an infinity or NaN in it)
