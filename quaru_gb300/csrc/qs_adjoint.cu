@@ -474,9 +474,13 @@ static std::vector<double> rotation_matrix(int axis, double c, double s) {
 }
 
 // Tile qubits for an n-qubit state: `cap` for large states, fewer below n = cap + 7 so that 128
-// tiles (blocks) share the work of mid-size states, never fewer than 8 (16 tiles at 12 qubits),
-// and the whole state in one tile up to 8 qubits (one block runs every gate without a launch each).
-static int adj_tile_qubits(int n, int cap) { return std::min(n, std::max(8, std::min(cap, n - 7))); }
+// tiles (blocks) share the work of mid-size states, never fewer than `floor`: 8 (16 tiles at 12 qubits),
+// and the whole state in one tile up to 8 qubits (one block runs every gate without a launch each). Complex64
+// sweeps take 10: their tiles are cheap and the launches saved count for more (gradients of 10, 12, 14 qubits
+// 323, 423, 486 us at 8 and 285, 367, 444 us at 10; in complex128 the larger tiles lose).
+static int adj_tile_qubits(int n, int cap, int floor = 8) {
+    return std::min(n, std::max(floor, std::min(cap, n - 7)));
+}
 
 constexpr int kAdjDfMin = 6;  // from this many qubits QS_ARITH_DF64 runs double-float tiles
 
@@ -857,7 +861,7 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
     const size_t amp = prec == QS_PREC_C64 ? 8 : 16;
     const uint64_t N = 1ull << n;
     const bool df = prec == QS_PREC_C128 && arith == QS_ARITH_DF64 && n >= kAdjDfMin;
-    const int tq = adj_tile_qubits(n, kAdjT);
+    const int tq = adj_tile_qubits(n, kAdjT, prec == QS_PREC_C64 ? 10 : 8);
     bool unitary = true;
     for (size_t g = 0; g < m && unitary; g++)
         if (gates[g].kind == QS_GATE_FIXED) unitary = is_unitary(gates[g].matrix, gates[g].k);
