@@ -41,6 +41,7 @@ struct qs_register {
     uint64_t zval = 0;
     // The same knowledge for the gates, which also hold it from a basis state on: a superset of zmask.
     qs::LiveSpace known;
+    bool replayed = false;  // its gates were captured: a graph may change the state at any time
     // Scratch of the compact measurement sequences and of the squares of reference-order sums (half
     // the state), allocated by the first one and kept until the register is destroyed.
     void* mscratch = nullptr;
@@ -278,6 +279,24 @@ void touch_qubits(qs_register* reg, const double* matrix, const size_t* targets,
         }
 }
 
+// The gates' record of known qubits, or null where they go without: on states of fewer than 16 qubits, whose
+// gates are bound by their launch, and from the first gate call on that found the register's stream being
+// captured (the launches then have to serve any state, and replays pass the record by).
+constexpr int kLiveMinQubits = 16;
+
+qs::LiveSpace* live_space(qs_register* reg) {
+    if (reg->n < kLiveMinQubits) return nullptr;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (!reg->replayed && (cudaStreamIsCapturing(reg->stream, &status) != cudaSuccess ||
+                           status != cudaStreamCaptureStatusNone)) {
+        cudaGetLastError();
+        reg->replayed = true;
+    }
+    if (!reg->replayed) return &reg->known;
+    reg->known = qs::LiveSpace{};
+    return nullptr;
+}
+
 // Reference-order (sequential) probability sums for complex128 registers in the exact arithmetic
 // up to this size; larger registers and the other forms use the parallel tree reduction.
 constexpr int kSequentialMaxQubits = 20;
@@ -421,7 +440,7 @@ int qs_try_apply_fast(qs_register* reg, const double* matrix, size_t rows, size_
     qs::OpDesc op;
     qs::classify_gate(matrix, k, targets, &op);
     touch_qubits(reg, matrix, targets, k);
-    rc = qs::apply_op(reg->state, reg->n, reg->prec, reg->arith, op, reg->stream, reg->sms, &msg, &reg->known);
+    rc = qs::apply_op(reg->state, reg->n, reg->prec, reg->arith, op, reg->stream, reg->sms, &msg, live_space(reg));
     if (rc) reg->known = qs::LiveSpace{};
     return rc ? set_err(rc, msg) : QS_OK;
 }
@@ -475,7 +494,7 @@ int qs_apply_circuit(qs_register* reg, const qs_gate* gates, size_t m, const qs_
         o.fuse = 1;  // tuning switched off: stages at the automatic tile size
     }
     int rc = qs::run_circuit(reg->state, reg->n, reg->prec, reg->arith, ops, gates, o, reg->stream, reg->sms, &msg,
-                             nullptr, &reg->known);
+                             nullptr, live_space(reg));
     if (rc) reg->known = qs::LiveSpace{};  // part of it ran
     return rc ? set_err(rc, msg) : QS_OK;
 }

@@ -23,8 +23,8 @@ static int fail(cudaError_t e, const char* what, std::string* msg) {
     return QS_CUDA_ERROR;
 }
 
-// Gates on states of fewer qubits are bound by their launch, whatever they visit.
-constexpr int kLiveMinQubits = 16;
+static int apply_visited(void* state, int n, int reg_qubits, int prec, int arith, const OpDesc& op, cudaStream_t s,
+                         int sms, std::string* msg);
 
 int apply_op(void* state, int n, int prec, int arith, const OpDesc& op, cudaStream_t s, int sms, std::string* msg,
              LiveSpace* live) {
@@ -37,18 +37,24 @@ int apply_op(void* state, int n, int prec, int arith, const OpDesc& op, cudaStre
         const uint64_t targets = target_mask(op), known = live->mask & ~targets;
         const uint64_t val = live->val;
         live->release(targets);
-        if (n >= kLiveMinQubits && known) {
+        if (known) {
             if ((op.fixval ^ val) & op.fixmask & known) return QS_OK;  // a control that no amplitude meets
             OpDesc r = op;
             r.fixmask |= known;
             r.fixval |= val & known;
             int m = n;
             while (m > 1 && (r.fixmask & ~r.fixval) >> (m - 1) & 1ull) r.fixmask &= ~(1ull << --m);
-            return apply_op(state, m, prec, arith, r, s, sms, msg);
+            return apply_visited(state, m, n, prec, arith, r, s, sms, msg);
         }
     }
+    return apply_visited(state, n, n, prec, arith, op, s, sms, msg);
+}
+
+// On the register's first 2^n amplitudes.
+static int apply_visited(void* state, int n, int reg_qubits, int prec, int arith, const OpDesc& op, cudaStream_t s,
+                         int sms, std::string* msg) {
     if (op.k <= kMaxSmallK) {
-        cudaError_t e = launch_op(op, state, n, prec, arith, s, sms);
+        cudaError_t e = launch_op(op, state, n, prec, arith, s, sms, reg_qubits);
         return e == cudaSuccess ? QS_OK : fail(e, "gate kernel", msg);
     }
     if (op.k > kMaxBigK) {

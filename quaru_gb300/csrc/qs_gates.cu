@@ -225,6 +225,10 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? 4 : 5) k_dense1_im(doubl
 constexpr int kDotSpread = 17;
 constexpr uint32_t kDotLow = 300, kDotSpan = 1400;  // exponent fields of the largest component
 constexpr int32_t kLimb = (1 << 30) - 1;
+// Registers of up to 16 qubits keep the FMA chain: its launch bounds a gate there (16 qubits 5.0 us either way;
+// 17 qubits 7.1 us with the chain, 6.2 us so; 20 qubits 17.3 and 13.3, 22 qubits 52.2 and 40.2). The register's
+// size decides, not how much of it a gate visits: the values don't depend on what is known of the state.
+constexpr int kDotMinQubits = 17;
 
 struct DotVal {
     int32_t x0, x1, x2;  // each with the sign
@@ -727,7 +731,7 @@ static bool fill_fx(const OpDesc& op, Dense1FxArgs& a) {
 
 template <typename R>
 static cudaError_t launch_dense1(const OpDesc& op, void* state, int n, bool exact, cudaStream_t s, int sms,
-                                 bool df64 = false, bool fx64 = false) {
+                                 bool df64 = false, bool fx64 = false, int reg_qubits = 0) {
     using T = typename Cplx<R>::T;
     Dense1Args<R> a;
     std::memset(&a, 0, sizeof(a));
@@ -742,7 +746,7 @@ static cudaError_t launch_dense1(const OpDesc& op, void* state, int n, bool exac
     if constexpr (sizeof(R) == 8) {
         if (!df64 && !fx64) {
             Dense1DotArgs dot;
-            if (!exact && !real && fill_dot(op.m.data(), &dot)) {
+            if (!exact && !real && reg_qubits >= kDotMinQubits && fill_dot(op.m.data(), &dot)) {
                 dot.map = a.map;
                 dot.tbit = a.tbit;
                 const int g1 = grid_for(ntup, sms, 1);
@@ -952,7 +956,7 @@ static cudaError_t launch_mono(const OpDesc& op, void* state, int n, cudaStream_
 
 template <typename R>
 static cudaError_t launch_small(const OpDesc& op, void* state, int n, bool exact, cudaStream_t s, int sms,
-                                bool df64 = false, bool fx64 = false) {
+                                bool df64 = false, bool fx64 = false, int reg_qubits = 0) {
     if (op.kind == OP_MONO || op.kind == OP_MONO_PF) {
         switch (op.k) {
             case 0: return launch_mono<R, 0>(op, state, n, s, sms);
@@ -975,7 +979,7 @@ static cudaError_t launch_small(const OpDesc& op, void* state, int n, bool exact
                 z.pf[0] = 255;
                 return launch_mono<R, 0>(z, state, n, s, sms);
             }
-            case 1: return launch_dense1<R>(op, state, n, exact, s, sms, df64, fx64);
+            case 1: return launch_dense1<R>(op, state, n, exact, s, sms, df64, fx64, reg_qubits);
             case 2: return launch_denseK<R, 2>(op, state, n, exact, s, sms, df64);
             case 3: return launch_denseK<R, 3>(op, state, n, exact, s, sms, df64);
             case 4: return launch_denseK<R, 4>(op, state, n, exact, s, sms);
@@ -985,12 +989,14 @@ static cudaError_t launch_small(const OpDesc& op, void* state, int n, bool exact
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_op(const OpDesc& op, void* state, int n, int prec, int arith, cudaStream_t s, int sms) {
+cudaError_t launch_op(const OpDesc& op, void* state, int n, int prec, int arith, cudaStream_t s, int sms,
+                      int reg_qubits) {
     if (op.kind == OP_NOOP) return cudaSuccess;
     if (op.k > kMaxSmallK) return cudaErrorInvalidValue;
     const bool exact = (arith == QS_ARITH_EXACT);
     if (prec == QS_PREC_C64) return launch_small<float>(op, state, n, false, s, sms);
-    return launch_small<double>(op, state, n, exact, s, sms, arith == QS_ARITH_DF64, arith == QS_ARITH_FX64);
+    return launch_small<double>(op, state, n, exact, s, sms, arith == QS_ARITH_DF64, arith == QS_ARITH_FX64,
+                                reg_qubits);
 }
 
 cudaError_t launch_op_big(const OpDesc& op, void* state, const void* src, int n, int prec, int arith,

@@ -64,7 +64,9 @@ struct BigOpBuffers {
 };
 
 // One sweep applying `op` (op.k <= kMaxSmallK) in place.
-cudaError_t launch_op(const OpDesc& op, void* state, int n, int prec, int arith, cudaStream_t s, int sms);
+// reg_qubits: of the register whose first 2^n amplitudes these are.
+cudaError_t launch_op(const OpDesc& op, void* state, int n, int prec, int arith, cudaStream_t s, int sms,
+                      int reg_qubits);
 
 // One sweep applying a wide `op`, reading the pre-gate state from `src`.
 cudaError_t launch_op_big(const OpDesc& op, void* state, const void* src, int n, int prec, int arith,

@@ -1,4 +1,5 @@
-"""Dense complex one-qubit gates in FMA arithmetic: sums of four products as one integer.
+"""Dense complex one-qubit gates in FMA arithmetic on registers of 17 qubits and more: sums of four products as one
+integer.
 
 Bar: where the pair's non-zero components lie within 2^17 of the largest (exponent fields 300 to 1699),
 each output is within 2^-53 of itself plus 2^-54 of its largest product; any other pair, and any other
@@ -46,7 +47,7 @@ def _fits(m):
 
 @pytest.mark.parametrize("kind", ["haar", "rx", "small", "below", "cancel", "large"])
 @pytest.mark.parametrize("span,shift", [(0, 0), (4, 0), (17, 0), (18, 0), (60, 0), (3, 676), (3, 677), (0, -723), (0, -724)])
-@pytest.mark.parametrize("n,t,control", [(1, 0, None), (9, 3, None), (9, 8, 2), (6, 0, 5)])
+@pytest.mark.parametrize("n,t,control", [(17, 0, None), (17, 3, None), (17, 16, 2), (18, 0, 17)])
 def test_outputs_are_sums_rounded_once(n, t, control, span, shift, kind):
     import quaru_gb300 as q
     from quaru_gb300 import operation as O
@@ -70,6 +71,9 @@ def test_outputs_are_sums_rounded_once(n, t, control, span, shift, kind):
     i = i[(i >> t & 1) == 0]
     if control is not None:
         i = i[(i >> control & 1) == 1]
+    rest = np.setdiff1d(np.arange(1 << n), np.concatenate([i, i | 1 << t]))
+    np.testing.assert_array_equal(got[rest].view(np.float64), s[rest].view(np.float64))
+    i = np.concatenate([i[:64], i[-64:], rng.choice(i, 2000)])
     x = [s[i].real, s[i].imag, s[i | 1 << t].real, s[i | 1 << t].imag]
     expo = np.array([np.where(v == 0.0, -5000, np.frexp(v)[1] + 1022) for v in x])
     E = expo.max(axis=0)
@@ -87,5 +91,18 @@ def test_outputs_are_sums_rounded_once(n, t, control, span, shift, kind):
                             mags.sum(axis=0) * L(2.0 ** -51)) + mags.sum(axis=0) * L(2.0 ** -61)
             off = np.abs(getattr(out, part).astype(L) - want)
             assert np.all(off <= room), (part, r)
-    rest = np.setdiff1d(np.arange(1 << n), np.concatenate([i, i | 1 << t]))
-    np.testing.assert_array_equal(got[rest].view(np.float64), s[rest].view(np.float64))
+
+
+def test_values_do_not_depend_on_what_is_known_of_the_state():
+    """The register's size decides the form, not how much of it a gate has to visit."""
+    import quaru_gb300 as q
+
+    rng = np.random.default_rng(5)
+    for n in (16, 17, 19):
+        a, b = q.Register.from_int(n, 3), q.Register.from_int(n, 3)
+        b.state = a.state
+        ops = [q.Operation(_matrix(rng, "haar"), [int(t)]) for t in rng.permutation(n)[:6]] * 2
+        for r in (a, b):
+            r.set_arith(q.QS_ARITH_FMA)
+            r.apply_gates(ops, fuse=0)
+        np.testing.assert_array_equal(a.state, b.state)

@@ -98,3 +98,45 @@ def test_overflowing_entries_assume_nothing(fuse, precision, big):
         x, y = a.state, b.state
     np.testing.assert_array_equal(np.isnan(x), np.isnan(y))
     np.testing.assert_array_equal(x[~np.isnan(x)], y[~np.isnan(y)])
+
+
+@pytest.mark.parametrize("fuse", [0, None])
+def test_captured_gates_serve_any_state(fuse):
+    """Gates captured while the register is a basis state, replayed on what they made of it, on a state set later
+    and after a measurement."""
+    import quaru_gb300 as q
+    import torch
+    from quaru_gb300 import operation as O
+
+    n = 17
+    ops = [O.hadamard(3), O.cnot(3, 16), q.Operation(np.array([[0.6, 0.8], [-0.8, 0.6]]), [9]), O.cnot(9, 0)]
+
+    def run(r):
+        if fuse is None:
+            for g in ops:
+                r.try_apply_fast(g)
+        else:
+            r.apply_gates(ops, fuse=fuse)
+
+    a, b = q.Register.from_int(n, 0), q.Register.from_int(n, 0)
+    run(q.Register.from_int(n, 0))  # the kernels are loaded before the capture
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(a.stream), capture_error_mode="thread_local"):
+        run(a)
+    st = np.zeros(1 << n, dtype=np.complex128)
+    st[12345] = 1j
+    for step in ("first", "again", "measured", "set"):
+        if step == "measured":
+            assert a.measure(5, 0.5) == b.measure(5, 0.5)
+            assert a.measure(16, 0.3) == b.measure(16, 0.3)
+        if step == "set":
+            a.state, b.state = st, st
+        with torch.cuda.stream(torch.cuda.ExternalStream(a.stream)):
+            graph.replay()
+        torch.cuda.synchronize()
+        run(b)
+        np.testing.assert_array_equal(a.state, b.state)
+    a.try_apply_fast(O.hadamard(7))
+    b.try_apply_fast(O.hadamard(7))
+    np.testing.assert_array_equal(a.state, b.state)
