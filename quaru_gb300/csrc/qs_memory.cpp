@@ -1,7 +1,7 @@
 // qs_memory.cpp — device memory kept between calls.
 //
 // Working buffers of a call (and small register states) come from a stream-ordered pool of the library's
-// own instead of the device's default pool. The default pool gives every free byte back to the driver
+// own instead of the device's default pool. The default pool gives every free byte back to CUDA
 // at each synchronisation, so a call that allocates, works and waits pays for mapping its buffers anew:
 // about 95 us of an 8-qubit gradient's 225 us. This pool keeps up to kKeepBytes free while the library has
 // registers or batches, and one allocation unit once it has none; memory beyond that goes back as before,
