@@ -49,7 +49,10 @@ extern "C" {
 /* ---- arithmetic of gate application on a complex128 register ------------ */
 #define QS_ARITH_EXACT 0 /* the reference's operation order, no fused multiply-add:
                             bit-identical amplitudes (+0 and -0 compared as equal) */
-#define QS_ARITH_FMA 1   /* FP64 fused multiply-add; within 1e-15 relative per gate */
+#define QS_ARITH_FMA 1   /* FP64 fused multiply-add; within 1e-15 relative per gate. Dense complex
+                            1-qubit gates on 17 qubits and more sum their four products as one
+                            integer, rounded once (error <= 2^-53 of the output plus 2^-54 of its
+                            largest product, below the FMA chain's) */
 #define QS_ARITH_DF64 2  /* double-float arithmetic on the FP32 pipe for dense gates;
                             ~2^-47 relative per gate; permutation/diagonal gates stay exact */
 #define QS_ARITH_FX64 3  /* FP64-accurate fixed-point arithmetic on the integer pipes for dense
@@ -172,8 +175,8 @@ int qs_apply_circuit(qs_register* reg, const qs_gate* gates, size_t m,
  * does (:306-315), so sums, outcome and collapsed state are bit-identical to
  * it; larger registers and the other forms use a fixed-order parallel tree
  * (within 1e-14). The collapse divides by sqrt(prob) (:337): correctly rounded
- * on complex128 registers in QS_ARITH_EXACT, as Rust's `/`; the other forms
- * multiply by the rounded reciprocal (within one ulp of the quotient).
+ * on complex128 registers in every arithmetic, as Rust's `/`; complex64
+ * registers multiply by the reciprocal and round once to float.
  * Qubits measured since their last gate stay collapsed: later measurements
  * read only the amplitudes that can still be non-zero. */
 int qs_try_measure(qs_register* reg, size_t target, double draw, int* outcome,
@@ -290,7 +293,8 @@ typedef struct qs_batch_options {
     int chunk_log2;      /* amplitude pairs per work item = 2^chunk_log2; 0 = autotune */
     int ctas_per_sm;     /* persistent CTAs per SM; 0 = autotune */
     int arith;           /* QS_ARITH_DF64: complex128 stages of rotations and CNOTs in double-float
-                            tiles; any other value: FP64 arithmetic */
+                            tiles; any other value: FP64-accurate arithmetic
+                            (64-bit fixed point per tile, FP64 with a gate that is not unitary) */
 } qs_batch_options;
 
 typedef struct qs_batch qs_batch;
