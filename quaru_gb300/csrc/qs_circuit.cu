@@ -29,6 +29,10 @@ static int apply_visited(void* state, int n, int reg_qubits, int prec, int arith
 int apply_op(void* state, int n, int prec, int arith, const OpDesc& op, cudaStream_t s, int sms, std::string* msg,
              LiveSpace* live) {
     if (op.kind == OP_NOOP) return QS_OK;
+    if (op.k > kMaxBigK) {
+        if (msg) *msg = "dense or monomial sub-operation wider than " + std::to_string(kMaxBigK) + " qubits";
+        return QS_INVALID_ARGUMENT;
+    }
     if (live && live->mask) {
         // A circuit starts from a basis state and a gate frees its own qubits only: of the first layer on 28
         // qubits a gate on qubit q has 2^(q + 1) amplitudes to visit (28 qubits, 84 gates: 113.6 ms without
@@ -56,10 +60,6 @@ static int apply_visited(void* state, int n, int reg_qubits, int prec, int arith
     if (op.k <= kMaxSmallK) {
         cudaError_t e = launch_op(op, state, n, prec, arith, s, sms, reg_qubits);
         return e == cudaSuccess ? QS_OK : fail(e, "gate kernel", msg);
-    }
-    if (op.k > kMaxBigK) {
-        if (msg) *msg = "dense or monomial sub-operation wider than " + std::to_string(kMaxBigK) + " qubits";
-        return QS_INVALID_ARGUMENT;
     }
     // Wide gate: tables in device memory, read the pre-gate state from a copy.
     std::vector<uint64_t> off, off_src;
