@@ -269,6 +269,8 @@ typedef struct qs_param_gate {
  * sums on complex64 registers). No intermediate state is stored: memory is
  * three state vectors. The register's state is the initial state and is
  * unchanged on return. Gradients of rotations that share a parameter add up.
+ * A rotation by an infinity or NaN makes the energy and the derivative of every
+ * rotation NaN (batches: of its circuit).
  * Errors: InvalidTarget / InvalidDimensions as try_apply_fast with err[2] =
  * gate index; QS_INVALID_ARGUMENT for a bad kind or parameter index. */
 int qs_adjoint_gradient(qs_register* reg, const qs_param_gate* gates, size_t m, const double* params,

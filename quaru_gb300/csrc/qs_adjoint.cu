@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -874,11 +875,23 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
     unsigned char* blob = nullptr;
     std::vector<double> res(2 + nrot, 0.0);  // the energy, the rotations' terms, the status: one readback
     std::vector<double2> angles(std::max<size_t>(m, 1), make_double2(1.0, 0.0));  // per gate: cos, sin of theta / 2
+    bool finite = true;
     for (size_t g = 0; g < m; g++)
         if (rot_slot[g] >= 0) {
             const double th = params[gates[g].param];
             angles[g] = make_double2(std::cos(0.5 * th), std::sin(0.5 * th));
+            finite = finite && std::isfinite(angles[g].x) && std::isfinite(angles[g].y);
         }
+    if (!finite) {
+        // A rotation by an infinity or NaN leaves NaN in every amplitude, so the energy and every rotation's
+        // derivative are NaN. Said here: the tiles' fixed-point coefficients and phases have no NaN.
+        const double nan = std::numeric_limits<double>::quiet_NaN();
+        if (energy) *energy = nan;
+        for (size_t p = 0; grad && p < np; p++) grad[p] = 0.0;
+        for (size_t g = 0; grad && g < m; g++)
+            if (rot_slot[g] >= 0) grad[gates[g].param] = nan;
+        return QS_OK;
+    }
     SweepPlan fplan, rplan;
     SweepTables ftab, rtab;
     int rc = QS_OK;

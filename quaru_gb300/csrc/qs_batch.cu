@@ -26,6 +26,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <fstream>
+#include <limits>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -1026,10 +1027,17 @@ extern "C" int qs_batch_run(qs_batch* b, const double* params, double* energies,
         set_last_error_message("null argument");
         return QS_INVALID_ARGUMENT;
     }
-    for (int i = 0; i < b->ncs; i++) {
-        const double th = params[b->cs_param[i]];
-        b->hcs[i] = make_double2(std::cos(0.5 * th), std::sin(0.5 * th));
-    }
+    std::vector<char> undefined(size_t(b->count), 0);  // circuits with a rotation by an infinity or NaN
+    for (int c = 0, i = 0; c < b->count; c++)
+        for (size_t r = 0; r < b->rot_param[c].size(); r++, i++) {
+            const double th = params[b->cs_param[i]];
+            double2 cs = make_double2(std::cos(0.5 * th), std::sin(0.5 * th));
+            if (!(std::isfinite(cs.x) && std::isfinite(cs.y))) {  // fixed-point tiles have no NaN: the results get it below
+                undefined[c] = 1;
+                cs = make_double2(1.0, 0.0);
+            }
+            b->hcs[i] = cs;
+        }
     cudaError_t e = cudaGraphLaunch(b->exec, b->stream);
     if (e == cudaSuccess) note_launches(b->nprogs ? 4 : 3);  // the graph's coefficient, reset, persistent and reduction kernels
     if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
@@ -1043,6 +1051,8 @@ extern "C" int qs_batch_run(qs_batch* b, const double* params, double* energies,
     }
     for (int c = 0; c < b->count; c++) {
         const int base = b->res_circ_base[c];
+        if (undefined[c])
+            std::fill(b->hres + base, b->hres + base + 1 + b->rot_param[c].size(), std::numeric_limits<double>::quiet_NaN());
         if (energies) energies[c] = b->hres[base];
         if (grads) {
             const size_t po = b->param_off[c];
