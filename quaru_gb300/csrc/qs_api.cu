@@ -41,7 +41,8 @@ struct qs_register {
     uint64_t zval = 0;
     // The same knowledge for the gates, which also hold it from a basis state on: a superset of zmask.
     qs::LiveSpace known;
-    bool replayed = false;  // its gates were captured: a graph may change the state at any time
+    // Its gates were captured: a graph may change the state at any time, so neither record holds anything.
+    bool replayed = false;
     // Scratch of the compact measurement sequences and of the squares of reference-order sums (half
     // the state), allocated by the first one and kept until the register is destroyed.
     void* mscratch = nullptr;
@@ -261,6 +262,12 @@ void set_last_error_message(const std::string& msg) { g_last_error = msg; }
 
 namespace {
 
+// Nothing is known of the state any more.
+void forget(qs_register* reg) {
+    reg->zmask = reg->zval = 0;
+    reg->known = qs::LiveSpace{};
+}
+
 // A gate maps the live subspace of the qubits it does not act on into itself (zero amplitudes there
 // stay exact zeros), so only its own targets leave the collapsed set. A matrix with a non-finite
 // entry can turn zeros into NaNs: then nothing is assumed any more.
@@ -273,28 +280,26 @@ void touch_qubits(qs_register* reg, const double* matrix, const size_t* targets,
     const size_t entries = k < 32 ? (size_t(2) << (2 * k)) : 0;
     for (size_t i = 0; i < entries; i++)
         if (!std::isfinite(reg->prec == QS_PREC_C64 ? double(float(matrix[i])) : matrix[i])) {
-            reg->zmask = reg->zval = 0;
-            reg->known = qs::LiveSpace{};
+            forget(reg);
             break;
         }
 }
 
 // The gates' record of known qubits, or null where they go without: on states of fewer than 16 qubits, whose
 // gates are bound by their launch, and from the first gate call on that found the register's stream being
-// captured (the launches then have to serve any state, and replays pass the record by).
+// captured (the launches then have to serve any state, and replays pass the records by: from then on
+// measurements record nothing either).
 constexpr int kLiveMinQubits = 16;
 
 qs::LiveSpace* live_space(qs_register* reg) {
-    if (reg->n < kLiveMinQubits) return nullptr;
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     if (!reg->replayed && (cudaStreamIsCapturing(reg->stream, &status) != cudaSuccess ||
                            status != cudaStreamCaptureStatusNone)) {
         cudaGetLastError();
         reg->replayed = true;
+        forget(reg);
     }
-    if (!reg->replayed) return &reg->known;
-    reg->known = qs::LiveSpace{};
-    return nullptr;
+    return reg->replayed || reg->n < kLiveMinQubits ? nullptr : &reg->known;
 }
 
 // Reference-order (sequential) probability sums for complex128 registers in the exact arithmetic
@@ -321,10 +326,19 @@ double* seq_squares(qs_register* reg) {
     return sequential_sums(reg) && reg->n > 13 ? static_cast<double*>(measure_scratch(reg)) : nullptr;
 }
 
-void record_outcome(qs_register* reg, size_t target, int res) {
+// What a measurement call knows of the zeros: the register's record and the outcomes so far.
+struct Collapsed {
+    uint64_t mask, val;
+    explicit Collapsed(const qs_register* reg) : mask(reg->zmask), val(reg->zval) {}
+};
+
+void record_outcome(qs_register* reg, Collapsed* seen, size_t target, int res) {
     const uint64_t b = 1ull << target;
-    reg->zmask |= b;
-    reg->zval = (reg->zval & ~b) | (res ? b : 0ull);
+    seen->mask |= b;
+    seen->val = (seen->val & ~b) | (res ? b : 0ull);
+    if (reg->replayed) return;
+    reg->zmask = seen->mask;
+    reg->zval = seen->val;
     reg->known.mask |= b;
     reg->known.val = (reg->known.val & ~b) | (res ? b : 0ull);
 }
@@ -507,8 +521,9 @@ int qs_try_measure(qs_register* reg, size_t target, double draw, int* outcome, d
         if (err) err[0] = target;
         return set_err(QS_INVALID_TARGET, "InvalidTarget(" + std::to_string(target) + ")");
     }
+    Collapsed seen(reg);
     QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(target), reg->partials, kMaxPartials,
-                                     reg->hres, reg->stream, reg->sms, reg->zmask, reg->zval, sequential_sums(reg),
+                                     reg->hres, reg->stream, reg->sms, seen.mask, seen.val, sequential_sums(reg),
                                      seq_squares(reg)),
             "measure_probs");
     QS_CUDA(cudaStreamSynchronize(reg->stream), "measure sync");
@@ -518,9 +533,9 @@ int qs_try_measure(qs_register* reg, size_t target, double draw, int* outcome, d
     const double d = std::sqrt(total);
     const double rinv = 1.0 / d;
     QS_CUDA(qs::launch_collapse(reg->state, reg->n, reg->prec, int(target), res, d, rinv, reg->stream, reg->sms,
-                                reg->zmask, reg->zval),
+                                seen.mask, seen.val),
             "collapse");
-    record_outcome(reg, target, res);
+    record_outcome(reg, &seen, target, res);
     if (outcome) *outcome = res;
     if (prob0) *prob0 = p0;
     if (prob1) *prob1 = p1;
@@ -552,6 +567,7 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
     QS_CUDA(qs::launch_measure_probs(reg->state, n, reg->prec, int(targets[0]), reg->partials, kMaxPartials,
                                      reg->hres, reg->stream, reg->sms),
             "measure_probs");
+    Collapsed seen(reg);  // nothing yet
     std::vector<int> free_bits(n);  // the source buffer's index bits, as qubits, ascending
     for (int q = 0; q < n; q++) free_bits[q] = q;
     auto index_of = [&](size_t q) {
@@ -574,7 +590,7 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
         QS_CUDA(qs::launch_collapse_compact(src, dst, nfree, reg->prec, pos, res, d, rinv, next_pos, reg->partials,
                                             kMaxPartials, reg->hres, reg->stream, reg->sms),
                 "collapse_compact");
-        record_outcome(reg, targets[k], res);
+        record_outcome(reg, &seen, targets[k], res);
         src = dst;
         outcomes[k] = res;
         if (prob0s) prob0s[k] = p0;
@@ -585,7 +601,7 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
         QS_CUDA(cudaMemcpyAsync(scratch, reg->state, live * amp, cudaMemcpyDeviceToDevice, reg->stream),
                 "compact copy");
     QS_CUDA(cudaMemsetAsync(reg->state, 0, (size_t(1) << n) * amp, reg->stream), "state zero");
-    QS_CUDA(qs::launch_scatter_live(reg->state, scratch, n, reg->prec, reg->zmask, reg->zval, reg->stream, reg->sms),
+    QS_CUDA(qs::launch_scatter_live(reg->state, scratch, n, reg->prec, seen.mask, seen.val, reg->stream, reg->sms),
             "scatter live");
     return QS_OK;
 }
@@ -629,8 +645,9 @@ int qs_measure_sequence(qs_register* reg, const size_t* targets, size_t m, const
         const int rc = measure_sequence_compact(reg, targets, m, draws, outcomes, prob0s, prob1s);
         if (rc != 1) return rc;
     }
+    Collapsed seen(reg);
     QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(targets[0]), reg->partials, kMaxPartials,
-                                     reg->hres, reg->stream, reg->sms, reg->zmask, reg->zval, seq, seq_squares(reg)),
+                                     reg->hres, reg->stream, reg->sms, seen.mask, seen.val, seq, seq_squares(reg)),
             "measure_probs");
     for (size_t k = 0; k < m; k++) {
         QS_CUDA(cudaStreamSynchronize(reg->stream), "measure sync");
@@ -643,18 +660,18 @@ int qs_measure_sequence(qs_register* reg, const size_t* targets, size_t m, const
         if (k + 1 < m && !seq) {
             QS_CUDA(qs::launch_collapse_probs(reg->state, reg->n, reg->prec, t, res, d, rinv, int(targets[k + 1]),
                                               reg->partials, kMaxPartials, reg->hres, reg->stream, reg->sms,
-                                              reg->zmask, reg->zval),
+                                              seen.mask, seen.val),
                     "collapse_probs");
-            record_outcome(reg, targets[k], res);
+            record_outcome(reg, &seen, targets[k], res);
         } else {
             QS_CUDA(qs::launch_collapse(reg->state, reg->n, reg->prec, t, res, d, rinv, reg->stream, reg->sms,
-                                        reg->zmask, reg->zval),
+                                        seen.mask, seen.val),
                     "collapse");
-            record_outcome(reg, targets[k], res);
+            record_outcome(reg, &seen, targets[k], res);
             if (k + 1 < m)
                 QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(targets[k + 1]), reg->partials,
-                                                 kMaxPartials, reg->hres, reg->stream, reg->sms, reg->zmask,
-                                                 reg->zval, seq, seq_squares(reg)),
+                                                 kMaxPartials, reg->hres, reg->stream, reg->sms, seen.mask,
+                                                 seen.val, seq, seq_squares(reg)),
                         "measure_probs");
         }
         outcomes[k] = res;
@@ -719,8 +736,7 @@ int qs_adjoint_gradient(qs_register* reg, const qs_param_gate* gates, size_t m, 
     if (reg->n < 1) return set_err(QS_INVALID_ARGUMENT, "register has no qubits");
     if (!terms_fit(terms, nterms, reg->n)) return set_err(QS_INVALID_ARGUMENT, "Pauli term acts on a qubit >= n");
     std::string msg;
-    reg->zmask = reg->zval = 0;  // the state is restored on return, but not assumed collapsed any more
-    reg->known = qs::LiveSpace{};
+    forget(reg);  // the state is restored on return, but not assumed collapsed any more
     int rc = qs::adjoint_gradient(reg->state, reg->n, reg->prec, reg->arith, gates, m, params, nparams, terms, nterms,
                                   reg->stream, reg->sms, energy, grad, err, &msg);
     return rc ? set_err(rc, msg) : QS_OK;
@@ -782,8 +798,7 @@ int qs_get_state(const qs_register* reg, double* dst) {
 int qs_set_state(qs_register* reg, const double* src) {
     qs::TraceRange trace("qs_set_state");
     if (!reg || !src) return set_err(QS_INVALID_ARGUMENT, "null argument");
-    reg->zmask = reg->zval = 0;
-    reg->known = qs::LiveSpace{};
+    forget(reg);
     const uint64_t N = 1ull << reg->n;
     if (reg->prec == QS_PREC_C128) {
         QS_CUDA(cudaMemcpyAsync(reg->state, src, N * 16, cudaMemcpyHostToDevice, reg->stream), "set_state");

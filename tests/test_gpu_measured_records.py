@@ -1,0 +1,56 @@
+"""What a register records of its zeros behind measurements: registers whose gates were captured into a graph record
+nothing, as a replay changes the state behind the library's back."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("sequence", [False, True])
+@pytest.mark.parametrize("n", [5, 12, 15, 17])
+def test_replays_behind_a_measurement(n, sequence):
+    """Capture, measure, replay; then a clone's gates and measurements of other qubits, against a register that ran the
+    same gates itself. QS_ARITH_EXACT on registers of up to 20 qubits: sums in index order, so all bits agree."""
+    import quaru_gb300 as q
+    import torch
+    from quaru_gb300 import operation as O
+
+    ops = [O.hadamard(2), O.cnot(2, n - 1), O.hadamard(1)]
+
+    def run(r):
+        for g in ops:
+            r.try_apply_fast(g)
+
+    run(q.Register.from_int(n, 0))  # the kernels are loaded before the capture
+    a, b = q.Register.from_int(n, 0), q.Register.from_int(n, 0)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(a.stream), capture_error_mode="thread_local"):
+        run(a)
+
+    def replay():
+        with torch.cuda.stream(torch.cuda.ExternalStream(a.stream)):
+            graph.replay()
+        torch.cuda.synchronize()
+        run(b)
+
+    def measure(r, targets, draws):
+        if sequence:
+            return r.measure_sequence(targets, draws)
+        return [r.measure(t, d) for t, d in zip(targets, draws)]
+
+    replay()
+    assert measure(a, [2, n - 1], [0.3, 0.6]) == measure(b, [2, n - 1], [0.3, 0.6])
+    replay()
+    c = a.clone()
+    assert measure(a, [1, 0, 2, n - 1], [0.9, 0.5, 0.4, 0.7]) == measure(b, [1, 0, 2, n - 1], [0.9, 0.5, 0.4, 0.7])
+    np.testing.assert_array_equal(a.state, b.state)
+    # the clone: the state before those measurements
+    d = q.Register.from_int(n, 0)
+    d.state = c.state
+    for r in (c, d):
+        r.try_apply_fast(O.not_(2))
+        r.apply_gates([O.hadamard(0), O.cnot(n - 1, 0)], fuse=1)
+    np.testing.assert_array_equal(c.state, d.state)
+    assert measure(c, [0, 1], [0.2, 0.8]) == measure(d, [0, 1], [0.2, 0.8])
+    np.testing.assert_array_equal(c.state, d.state)
