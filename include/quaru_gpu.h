@@ -178,7 +178,8 @@ int qs_apply_circuit(qs_register* reg, const qs_gate* gates, size_t m,
  * on complex128 registers in every arithmetic, as Rust's `/`; complex64
  * registers multiply by the reciprocal and round once to float.
  * Qubits measured since their last gate stay collapsed: later measurements
- * read only the amplitudes that can still be non-zero. */
+ * read only the amplitudes that can still be non-zero. A collapse onto a sum
+ * that is zero or NaN divides the whole kept half, zeros included. */
 int qs_try_measure(qs_register* reg, size_t target, double draw, int* outcome,
                    double* prob0, double* prob1, size_t* err);
 

@@ -326,6 +326,10 @@ double* seq_squares(qs_register* reg) {
     return sequential_sums(reg) && reg->n > 13 ? static_cast<double*>(measure_scratch(reg)) : nullptr;
 }
 
+// Whether a collapse onto this probability sum leaves zeros zero. 0 / 0 and 0 / NaN are NaN: the collapse then visits
+// every amplitude, as the reference's does (src/register.rs:333-339), and nothing recorded before it holds.
+bool keeps_zeros(double total) { return total > 0.0; }
+
 // What a measurement call knows of the zeros: the register's record and the outcomes so far.
 struct Collapsed {
     uint64_t mask, val;
@@ -530,6 +534,10 @@ int qs_try_measure(qs_register* reg, size_t target, double draw, int* outcome, d
     const double p0 = reg->hres[0], p1 = reg->hres[1];
     const int res = draw > p0 ? 1 : 0;  // src/register.rs:321
     const double total = res ? p1 : p0;  // :323
+    if (!keeps_zeros(total)) {
+        forget(reg);
+        seen = Collapsed(reg);
+    }
     const double d = std::sqrt(total);
     const double rinv = 1.0 / d;
     QS_CUDA(qs::launch_collapse(reg->state, reg->n, reg->prec, int(target), res, d, rinv, reg->stream, reg->sms,
@@ -554,19 +562,21 @@ namespace {
 // and the front of the state buffer, and at the end the state is zeroed (the value the in-place
 // passes leave in every dropped amplitude) and the last live amplitudes are written back to their
 // places. Results are bit-identical to the in-place passes; a pass moves its live data instead of
-// whole DRAM sectors of a strided subspace. Returns 1 when the scratch buffer cannot be allocated,
-// and the caller then runs the in-place passes.
+// whole DRAM sectors of a strided subspace. The caller runs the in-place passes from target *done on: 0 when
+// the scratch buffer cannot be allocated, a target with nothing to collapse onto (its sums are in hres), or m.
+// *summed: target *done's sums are there.
 constexpr int kCompactMinQubits = 14;
 
 int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, const double* draws, int* outcomes,
-                             double* prob0s, double* prob1s) {
+                             double* prob0s, double* prob1s, size_t* done, bool* summed) {
     const int n = reg->n;
     const size_t amp = amp_bytes(reg->prec);
     void* scratch = measure_scratch(reg);
-    if (!scratch) return 1;
+    if (!scratch) return QS_OK;
     QS_CUDA(qs::launch_measure_probs(reg->state, n, reg->prec, int(targets[0]), reg->partials, kMaxPartials,
                                      reg->hres, reg->stream, reg->sms),
             "measure_probs");
+    *summed = true;
     Collapsed seen(reg);  // nothing yet
     std::vector<int> free_bits(n);  // the source buffer's index bits, as qubits, ascending
     for (int q = 0; q < n; q++) free_bits[q] = q;
@@ -574,19 +584,19 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
         return int(std::find(free_bits.begin(), free_bits.end(), int(q)) - free_bits.begin());
     };
     const void* src = reg->state;
-    void* dst = nullptr;
-    for (size_t k = 0; k < m; k++) {
+    for (size_t& k = *done; k < m; k++) {
         QS_CUDA(cudaStreamSynchronize(reg->stream), "measure sync");
         const double p0 = reg->hres[0], p1 = reg->hres[1];
         const int res = draws[k] > p0 ? 1 : 0;  // src/register.rs:321
         const double total = res ? p1 : p0;
+        if (!keeps_zeros(total)) break;
         const double d = std::sqrt(total);
         const double rinv = 1.0 / d;
         const int nfree = int(free_bits.size());
         const int pos = index_of(targets[k]);
         free_bits.erase(free_bits.begin() + pos);
         const int next_pos = k + 1 < m ? index_of(targets[k + 1]) : -1;
-        dst = (k % 2 == 0) ? scratch : reg->state;  // the first pass reads the whole state
+        void* dst = (k % 2 == 0) ? scratch : reg->state;  // the first pass reads the whole state
         QS_CUDA(qs::launch_collapse_compact(src, dst, nfree, reg->prec, pos, res, d, rinv, next_pos, reg->partials,
                                             kMaxPartials, reg->hres, reg->stream, reg->sms),
                 "collapse_compact");
@@ -596,8 +606,9 @@ int measure_sequence_compact(qs_register* reg, const size_t* targets, size_t m, 
         if (prob0s) prob0s[k] = p0;
         if (prob1s) prob1s[k] = p1;
     }
+    if (*done == 0) return QS_OK;  // the state is as it was
     const size_t live = size_t(1) << free_bits.size();
-    if (dst == reg->state)
+    if (src == reg->state)
         QS_CUDA(cudaMemcpyAsync(scratch, reg->state, live * amp, cudaMemcpyDeviceToDevice, reg->stream),
                 "compact copy");
     QS_CUDA(cudaMemsetAsync(reg->state, 0, (size_t(1) << n) * amp, reg->stream), "state zero");
@@ -640,20 +651,27 @@ int qs_measure_sequence(qs_register* reg, const size_t* targets, size_t m, const
         }
     if (m == 0) return QS_OK;
     const bool seq = sequential_sums(reg);
+    size_t done = 0;
+    bool summed = false;
     if (!seq && m >= 3 && reg->zmask == 0 && reg->n >= kCompactMinQubits && distinct_targets(targets, m) &&
         compact_measurement_enabled()) {
-        const int rc = measure_sequence_compact(reg, targets, m, draws, outcomes, prob0s, prob1s);
-        if (rc != 1) return rc;
+        const int rc = measure_sequence_compact(reg, targets, m, draws, outcomes, prob0s, prob1s, &done, &summed);
+        if (rc || done == m) return rc;
     }
     Collapsed seen(reg);
-    QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(targets[0]), reg->partials, kMaxPartials,
-                                     reg->hres, reg->stream, reg->sms, seen.mask, seen.val, seq, seq_squares(reg)),
-            "measure_probs");
-    for (size_t k = 0; k < m; k++) {
+    if (!summed)
+        QS_CUDA(qs::launch_measure_probs(reg->state, reg->n, reg->prec, int(targets[0]), reg->partials, kMaxPartials,
+                                         reg->hres, reg->stream, reg->sms, seen.mask, seen.val, seq, seq_squares(reg)),
+                "measure_probs");
+    for (size_t k = done; k < m; k++) {
         QS_CUDA(cudaStreamSynchronize(reg->stream), "measure sync");
         const double p0 = reg->hres[0], p1 = reg->hres[1];
         const int res = draws[k] > p0 ? 1 : 0;
         const double total = res ? p1 : p0;
+        if (!keeps_zeros(total)) {
+            forget(reg);
+            seen = Collapsed(reg);
+        }
         const double d = std::sqrt(total);
         const double rinv = 1.0 / d;
         const int t = int(targets[k]);

@@ -1,5 +1,6 @@
 """What a register records of its zeros behind measurements: registers whose gates were captured into a graph record
-nothing, as a replay changes the state behind the library's back."""
+nothing (a replay changes the state behind the library's back), and a collapse whose probability sum is zero or NaN
+fills the kept half with NaN, as the reference's division does, whatever was recorded before it."""
 import numpy as np
 import pytest
 
@@ -54,3 +55,41 @@ def test_replays_behind_a_measurement(n, sequence):
     np.testing.assert_array_equal(c.state, d.state)
     assert measure(c, [0, 1], [0.2, 0.8]) == measure(d, [0, 1], [0.2, 0.8])
     np.testing.assert_array_equal(c.state, d.state)
+
+
+@pytest.mark.parametrize("precision,arith", [(0, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("form", ["calls", "sequence", "in_place"])
+@pytest.mark.parametrize("n", [6, 15, 17])
+def test_collapse_onto_nothing(n, form, precision, arith, monkeypatch):
+    """Draws above 1 take outcome 1 of qubits that are 0: 0 / 0 on the whole kept half, then gates."""
+    import quaru_gb300 as q
+    from quaru_gb300 import operation as O
+
+    if form == "in_place":
+        monkeypatch.setenv("QS_MEASURE_COMPACT", "off")
+    targets = [n - 2, 3, 0, n - 1]
+    for bad in range(4):  # the measurement that has nothing to collapse onto
+        draws = [0.5] * 4
+        draws[bad] = 1.5
+        g = q.Register.from_int(n, 0, precision=precision)
+        g.set_arith(arith)
+        want = np.zeros(1 << n, dtype=complex)
+        want[0] = 1.0
+        i = np.arange(1 << n)
+        outcomes = []
+        for t, d in zip(targets, draws):  # src/register.rs:306-339
+            p0 = np.sum(np.abs(want[(i >> t & 1) == 0]) ** 2)
+            p1 = np.sum(np.abs(want[(i >> t & 1) == 1]) ** 2)
+            res = bool(d > p0)
+            with np.errstate(all="ignore"):
+                want = np.where((i >> t & 1) == res, want / np.sqrt(p1 if res else p0), 0.0)
+            outcomes.append(res)
+        got = g.measure_sequence(targets, draws) if form != "calls" else [g.measure(t, d) for t, d in zip(targets, draws)]
+        assert got == outcomes
+        for op, move in ((None, None), (O.not_(targets[bad]), 1 << targets[bad]), (O.not_(1), 2)):
+            if op is not None:
+                g.try_apply_fast(op)
+                want = want[i ^ move]
+            s = g.state
+            np.testing.assert_array_equal(np.isnan(s), np.isnan(want))
+            np.testing.assert_array_equal(s[~np.isnan(s)], want[~np.isnan(want)])
