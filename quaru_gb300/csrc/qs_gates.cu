@@ -217,8 +217,8 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? 4 : 5) k_dense1_im(doubl
 // A dense complex one-qubit gate in FMA arithmetic: each output component is a sum of four products, taken
 // as one integer and rounded once (the chain of FMAs rounds four times). The pair's four components go on the
 // scale of the largest, E: significands shifted left by 30 - (E - e), in limbs of 30 bits; a coefficient is two
-// limbs, exactly. Of the six limb products the lowest is dropped: below 2^-54 of any product whose component
-// is within 2^kDotSpread of the largest. Other pairs (1 in 2^17 of a random state's) take the FMA chain.
+// limbs, exactly. Of the six limb products the lowest is dropped, which leaves an output within 2^-54 of its largest
+// product while components lie within 2^kDotSpread of the largest and coefficients are as fill_dot wants them. Other pairs (1 in 2^17 of a random state's) take the FMA chain.
 // Bound: 220 ALU instructions and 80 wide multiply-adds per pair, in place of 12 FP64 instructions and 4
 // integer products (FP64: 64 cycles per warp instruction and sub-partition). 28 qubits, one gate on a
 // state without zeros: 3.07 ms before, 2.23 ms now; the state's traffic takes 1.26 ms.
@@ -310,7 +310,12 @@ __global__ void __launch_bounds__(kThreads, 4) k_dense1_dot(double2* __restrict_
 }
 
 // Coefficients of k_dense1_dot, if every part is an integer at 2^(e - 60), the largest below 2^e (parts of
-// 2^(e - 8) and more always are), and the scale leaves the results' exponents in range.
+// 2^(e - 8) and more always are), no part is so small that what is dropped shows, and the scale leaves the
+// results' exponents in range.
+// Dropped is less than 2^62.4 of an output (four lowest limb products of 2^60 each and the cut of C), and that has to
+// stay below 2^-54 of its largest product. Where a row's four parts are all non-zero, the pair's largest component (2^82
+// and more) is in that output: parts of 2^35 and more, 2^(e - 25), will do. Where one is zero, an output may be left with
+// a component 2^kDotSpread below (2^65), and no more than three of them: 2^52, 2^(e - 8).
 static bool fill_dot(const double* m, Dense1DotArgs* a) {
     double top = 0.0;
     for (int i = 0; i < 8; i++) top = std::max(top, std::fabs(m[i]));
@@ -326,6 +331,11 @@ static bool fill_dot(const double* m, Dense1DotArgs* a) {
         c->l = int32_t(i & kLimb);
         return true;
     };
+    for (int r = 0; r < 8; r += 4) {
+        const bool whole = m[r] != 0.0 && m[r + 1] != 0.0 && m[r + 2] != 0.0 && m[r + 3] != 0.0;
+        for (int i = r; i < r + 4; i++)
+            if (m[i] != 0.0 && std::fabs(m[i]) < std::ldexp(1.0, e - (whole ? 25 : 8))) return false;
+    }
     for (int i = 0; i < 4; i++) {
         a->m[2 * i] = m[2 * i];
         a->m[2 * i + 1] = m[2 * i + 1];

@@ -106,3 +106,38 @@ def test_values_do_not_depend_on_what_is_known_of_the_state():
             r.set_arith(q.QS_ARITH_FMA)
             r.apply_gates(ops, fuse=0)
         np.testing.assert_array_equal(a.state, b.state)
+
+
+@pytest.mark.parametrize("k", [7, 8, 9, 20, 24, 25, 30, 39, 40, 49, 58, 59])
+@pytest.mark.parametrize("full", [False, True])
+def test_small_parts_with_few_bits(full, k):
+    """Parts far below the largest that are integers at 2^-60 all the same: an output that only such parts feed keeps
+    the bound of the integer sums (see above). RX by 2^(1 - k) and a row of small parts, on pairs whose other
+    components are zero, or none of them."""
+    import quaru_gb300 as q
+
+    n, t, e = 17, 4, 2.0 ** -k
+    rng = np.random.default_rng([k, full])
+    for m in (np.array([[1.0, -1j * e], [-1j * e, 1.0]]), np.array([[1.0, 0.5], [e + e * 1j, e - 1j * e]])):
+        s = _state(rng, n, 17)
+        if not full:
+            s[rng.random(s.size) < 0.5] = 0.0
+        g = q.Register.from_int(n, 0)
+        g.set_arith(q.QS_ARITH_FMA)
+        g.state = s
+        g.try_apply_fast(q.Operation(m, [t]))
+        got = g.state
+        i = np.arange(1 << n)
+        i = i[(i >> t & 1) == 0]
+        a, b = s[i], s[i | 1 << t]
+        x = [v.astype(L) for v in (a.real, a.imag, b.real, b.imag)]
+        for r in (0, 1):
+            out = got[i | (r << t)]
+            ar, ai, br, bi = (L(v) for v in (m[r, 0].real, m[r, 0].imag, m[r, 1].real, m[r, 1].imag))
+            for part, c in (("real", (ar, -ai, br, -bi)), ("imag", (ai, ar, bi, br))):
+                terms = np.array([c[0] * x[0], c[1] * x[1], c[2] * x[2], c[3] * x[3]])
+                want = terms.sum(axis=0)
+                mags = np.abs(terms)
+                # four roundings of the chain, and the reference's own
+                room = mags.sum(axis=0) * L(2.0 ** -51 + 2.0 ** -61)
+                assert np.all(np.abs(getattr(out, part).astype(L) - want) <= room), (part, r)
