@@ -165,7 +165,7 @@ class Register:
         targets = op.targets if type(op.targets) is list else list(op.targets)
         k = len(targets)
         try:
-            if k and min(targets) < 0:  # ctypes would wrap it
+            if k and (min(targets) < 0 or max(targets) >> 64):  # ctypes would wrap it
                 raise ValueError
             t = (_TARGETS[k] if k < 9 else ctypes.c_size_t * k)(*targets)
         except (TypeError, ValueError):  # what else numpy takes as integers, or its error
