@@ -661,7 +661,9 @@ static Divisor make_divisor(double d, double rinv) {
     }
     v.rh = uint32_t(q >> 32);
     v.rl = uint32_t(q);
-    const int lo = std::max(1, e - 1020), hi = std::min(2046, e + 1020);
+    // from 2^-959 up: quotient_rare's remainder x - q d is a multiple of ulp(q) ulp(d) >= 2^-105 x, which has to be
+    // a double too (2^-1074 and more)
+    const int lo = std::max(64, e - 1020), hi = std::min(2046, e + 1020);
     v.low = uint32_t(lo) << 20;
     v.span = uint32_t(std::max(0, hi - lo + 1)) << 20;
     v.base = (1021 - e) * (1 << 20);

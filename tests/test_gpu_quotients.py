@@ -41,3 +41,25 @@ def test_kept_amplitudes_are_ieee_quotients(n, scale, arith):
                 want = s[live].view(np.float64) / math.sqrt(total)
             np.testing.assert_array_equal(out[live].view(np.uint64), want.view(np.uint64))
             assert not out[~live].view(np.uint64).any()
+
+
+@pytest.mark.parametrize("arith", [0, 1])
+@pytest.mark.parametrize("top", [-1010, -1000, -980, -960, -930, -905])
+def test_small_normal_amplitudes(top, arith):
+    """Amplitudes whose remainder x - q d has bits below the subnormal range (from about 2^-968 down), beside one large
+    amplitude that sets the divisor; enough of them to meet the quotients near the middle of two doubles."""
+    import quaru_gb300 as q
+
+    n = 18
+    rng = np.random.default_rng([-top, arith])
+    v = np.ldexp(rng.uniform(1.0, 2.0, 2 << n) * rng.choice([-1.0, 1.0], 2 << n), top - rng.integers(0, 12, 2 << n))
+    v[0], v[1] = 0.7390851332151607, 0.0
+    s = v.view(np.complex128)
+    g = q.Register.from_int(n, 0)
+    g.set_arith(arith)
+    g.state = s
+    assert not g.measure(n - 1, 0.0)
+    d = math.sqrt(g.last_probs[0])
+    assert 0.739 < d < 0.74
+    want = s[:1 << (n - 1)].view(np.float64) / d
+    np.testing.assert_array_equal(g.state[:1 << (n - 1)].view(np.float64).view(np.uint64), want.view(np.uint64))
