@@ -180,19 +180,20 @@ struct SweepArgs {
     int slot[kSwMaxRot];          // global slot of each program-local rotation
 };
 
-// src: psi as the launch finds it (the register's own state in the first launch, which is not written).
 template <int RB>
 constexpr int sweep_threads() {
     return RB == 3 ? 256 : 128;  // the largest tile that takes RB register bits
 }
+// src: psi as the launch finds it (the register's own state in the first launch, which is not written; psi itself in
+// the others, so neither is __restrict__).
 // Blocks per SM: two complex128 tile pairs fill the shared memory; complex64 tiles gain more from a third
 // block's warps (80 registers) than from free registers (20-qubit gradient 1.81 against 1.89 ms).
 template <typename T, int RB, bool REV>
 __global__ void __launch_bounds__(sweep_threads<RB>(), RB < 3 ? 4 : sizeof(T) == 16 ? 2 : REV ? 3 : 4)
-    k_sweep(const typename Sw<T>::Glob* __restrict__ src, typename Sw<T>::Glob* __restrict__ psi,
-            typename Sw<T>::Glob* __restrict__ lam, uint64_t ntiles, const __grid_constant__ SweepArgs a,
-            const SweepPass* __restrict__ passes, const TileOp* __restrict__ fixed,
-            const SweepCoef* __restrict__ coef, const double* __restrict__ sigmas, double* __restrict__ partials) {
+    k_sweep(const typename Sw<T>::Glob* src, typename Sw<T>::Glob* psi, typename Sw<T>::Glob* lam, uint64_t ntiles,
+            const __grid_constant__ SweepArgs a, const SweepPass* __restrict__ passes,
+            const TileOp* __restrict__ fixed, const SweepCoef* __restrict__ coef, const double* __restrict__ sigmas,
+            double* __restrict__ partials) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int nt = blockDim.x;
     SweepTile t = a.t;
