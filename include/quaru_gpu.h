@@ -268,8 +268,13 @@ typedef struct qs_param_gate {
  * each gate from psi and from lambda = H psi and reads each rotation's
  * derivative off Im<lambda|A|psi> (FP64 accumulation; FP32-pipe compensated
  * sums on complex64 registers). No intermediate state is stored: memory is
- * three state vectors. The register's state is the initial state and is
- * unchanged on return. Gradients of rotations that share a parameter add up.
+ * three state vectors. Complex128 registers hold the amplitudes in FP64 in
+ * QS_ARITH_EXACT; in QS_ARITH_FMA and QS_ARITH_FX64 as 64-bit fixed point per
+ * tile of up to 2^11 amplitudes (a gate's error is 2^-60 of the tile's norm on
+ * each: closer norm-wise and about twice as fast, but amplitudes below 2^-7 of
+ * that norm have fewer than 53 bits, and below 2^-61 none), or in FP64 with a
+ * fixed gate that is not unitary; in QS_ARITH_DF64 as double-float values. The
+ * register's state is the initial state and is unchanged on return. Gradients of rotations that share a parameter add up.
  * A rotation by an infinity or NaN makes the energy and the derivative of every
  * rotation NaN (batches: of its circuit).
  * Errors: InvalidTarget / InvalidDimensions as try_apply_fast with err[2] =
@@ -295,9 +300,10 @@ typedef struct qs_batch_options {
     int precision;       /* QS_PREC_C128 or QS_PREC_C64 */
     int chunk_log2;      /* amplitude pairs per work item = 2^chunk_log2; 0 = autotune */
     int ctas_per_sm;     /* persistent CTAs per SM; 0 = autotune */
-    int arith;           /* QS_ARITH_DF64: complex128 stages of rotations and CNOTs in double-float
-                            tiles; any other value: FP64-accurate arithmetic
-                            (64-bit fixed point per tile, FP64 with a gate that is not unitary) */
+    int arith;           /* complex128 tiles as in qs_adjoint_gradient: QS_ARITH_EXACT FP64; QS_ARITH_DF64
+                            double-float for stages of rotations and CNOTs; any other value 64-bit
+                            fixed point (FP64 where a circuit of the batch has a gate that is not
+                            unitary). Null options: QS_ARITH_FMA */
 } qs_batch_options;
 
 typedef struct qs_batch qs_batch;

@@ -867,7 +867,7 @@ int adjoint_gradient(void* state, int n, int prec, int arith, const qs_param_gat
     bool unitary = true;
     for (size_t g = 0; g < m && unitary; g++)
         if (gates[g].kind == QS_GATE_FIXED) unitary = is_unitary(gates[g].matrix, gates[g].k);
-    const SweepType type = prec == QS_PREC_C64 ? SW_C64 : unitary ? SW_FX : SW_F64;
+    const SweepType type = prec == QS_PREC_C64 ? SW_C64 : sweep_fixed_point(arith, unitary) ? SW_FX : SW_F64;
     const int pgrid = sweep_grid(n, tq, type, df, sms);
     auto al = [](size_t x) { return ((x + 255) / 256) * 256; };
     const size_t o_terms = 0, o_part = o_terms + al(nt * sizeof(PauliDev) + 1),

@@ -605,10 +605,9 @@ struct BTables {
 
 // Stages of one circuit (forward gates, then the reverse sweep) into the tables. Double-float stages hold
 // rotations and CNOTs; the others become programs.
-void plan_circuit(const qs_batch_circuit& q, int T, int prec, bool df_ok, bool unitary, BCirc* C,
+void plan_circuit(const qs_batch_circuit& q, int T, int prec, bool df_ok, bool unitary, bool fixed_point, BCirc* C,
                   const std::vector<int>& cs_of, const std::vector<int>& rslot_of, BTables* tb) {
     const int n = int(q.n);
-    const bool fixed_point = prec == QS_PREC_C128 && unitary;
     const int L = std::min(T, df_ok || !unitary ? 5 : prec == QS_PREC_C64 ? 4 : 3);  // rows of 128 bytes
     std::vector<char> cnot(q.m);
     for (size_t g = 0; g < q.m; g++) cnot[g] = q.gates[g].kind == QS_GATE_FIXED && q.gates[g].k == 2;
@@ -746,7 +745,7 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
             const qs_param_gate& G = circuits[c].gates[g];
             if (G.kind == QS_GATE_FIXED && G.k == 1 && G.matrix) unitary = is_unitary(G.matrix, 1);
         }
-    const bool fixed_point = b->prec == QS_PREC_C128 && unitary;
+    const bool fixed_point = b->prec == QS_PREC_C128 && sweep_fixed_point(b->arith, unitary);
     const size_t amp = b->prec == QS_PREC_C64 ? 8 : 16;
     size_t state_bytes = 0;
     int counters = 0;
@@ -802,7 +801,7 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
         }
         C.nrot = int(rp.size());
         tb.wtab.assign(rp.size(), -1);
-        plan_circuit(q, C.T, b->prec, df_ok, unitary, &C, cs_of, rslot_of, &tb);
+        plan_circuit(q, C.T, b->prec, df_ok, unitary, fixed_point, &C, cs_of, rslot_of, &tb);
         wtab.push_back(-1);  // the energy
         wtab.insert(wtab.end(), tb.wtab.begin(), tb.wtab.end());
         C.counter_off = counters;
@@ -947,7 +946,9 @@ extern "C" int qs_batch_create(const qs_batch_circuit* circuits, size_t count, c
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&max_per_sm, b->kernel, kBT, b->smem);
     max_per_sm = std::max(1, max_per_sm);
     std::ostringstream key;
-    key << "batch3:p" << b->prec << ":a" << (b->arith == QS_ARITH_DF64) << ":c" << count << ":items";
+    // the tile type: 0 fixed point or complex64, 1 with double-float stages, 2 FP64
+    const int form = df_ok ? 1 : b->prec == QS_PREC_C128 && !fixed_point ? 2 : 0;
+    key << "batch3:p" << b->prec << ":a" << form << ":c" << count << ":items";
     {
         uint64_t sig = 0;
         for (size_t c = 0; c < count; c++) sig = sig * 1315423911ull + uint64_t(circuits[c].n) * 131 + circuits[c].m;

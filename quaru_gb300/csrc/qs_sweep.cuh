@@ -1,7 +1,7 @@
 // qs_sweep.cuh — the passes of the gradient sweeps over a tile in shared memory (see qs_sweep.h).
 //
-// Tile types: float2 (complex64), FxC (complex128 as 64-bit fixed point), double2 (complex128 where a
-// fixed gate is not unitary, so that fixed point has no bound to scale by).
+// Tile types: float2 (complex64), FxC (complex128 as 64-bit fixed point), double2 (complex128 in
+// QS_ARITH_EXACT, or where a fixed gate is not unitary, so that fixed point has no bound to scale by).
 //
 // sm_103a issues about 2 FP64 operations per clock and SM, 64 integer and 128 FP32 ones, so double2
 // tiles are bound by the FP64 pipe and the others by instruction issue. Hence
