@@ -604,13 +604,12 @@ __device__ __forceinline__ void sw_moves(T* sp, T* sl, uint32_t tsize, int tq, u
             if (slot >= 0) S::gather(sacc[slot * kSwWarps + warp], mine);
         }
         const uint32_t tmask = (1u << (tq < 5 ? tq : 5)) - 1u;
-        if (P.phase_first) {
+        if (P.phase_first) {  // never in the reverse walk (without the branch its instances spill more: complex64 batches +1 %)
 #pragma unroll
             for (int r = 0; r < N; r++) {
                 const uint32_t y = from(r);
                 const typename S::Phase ph = sw_phase2(tab[y & tmask], tab[32 + (y >> 5)]);
                 x[r] = sw_phase(ph, x[r]);
-                if (REV) l[r] = sw_phase(ph, l[r]);
             }
         } else {
 #pragma unroll
@@ -919,7 +918,6 @@ static __global__ void __launch_bounds__(64) k_sweep_coefs(const SweepRange* __r
         const SweepRot rot = rots[R.coef0 + r];
         const double2 cs = angles[rot.angle];
         SweepCoef o{};
-        o.axis = rot.axis;
         o.c = cs.x;
         o.s = cs.y;
         fh[r] = 1.0;

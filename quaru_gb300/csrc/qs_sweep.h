@@ -90,8 +90,7 @@ struct alignas(16) SweepCoef {
     double c, s;
     int32_t ph, pl, sh, sl;  // limbs of -tan(a / 2) and sin(a); RZ: of cos and sin
     long long pk, sk;        // what rounds the limb products (FxLimb)
-    int32_t quarter, axis;
-    double pad;
+    int32_t quarter, pad[3];
 };
 
 }  // namespace qs
