@@ -10,6 +10,7 @@ used.
 from __future__ import annotations
 
 import ctypes
+import struct
 from typing import Callable, Iterable, Sequence
 
 import numpy as np
@@ -67,7 +68,7 @@ def _matrix(m) -> np.ndarray:
 
 
 _C128 = np.dtype(np.complex128)
-_TARGETS = [ctypes.c_size_t * k for k in range(9)]  # array types of the common arities
+_SIZES = [struct.Struct(f"{k}N") for k in range(9)]  # size_t arrays of the common arities
 
 
 class _Scratch(ctypes.Structure):
@@ -164,12 +165,11 @@ class Register:
             m = _matrix(m)
         targets = op.targets if type(op.targets) is list else list(op.targets)
         k = len(targets)
+        pack = _SIZES[k] if k < 9 else struct.Struct(f"{k}N")  # refuses what a size_t does not hold, as ctypes does not
         try:
-            if k and (min(targets) < 0 or max(targets) >> 64):  # ctypes would wrap it
-                raise ValueError
-            t = (_TARGETS[k] if k < 9 else ctypes.c_size_t * k)(*targets)
-        except (TypeError, ValueError):  # what else numpy takes as integers, or its error
-            t = (ctypes.c_size_t * k)(*np.array(targets, dtype=np.uintp).tolist())
+            t = pack.pack(*targets)
+        except (TypeError, struct.error):  # what else numpy takes as integers, or its error
+            t = pack.pack(*np.array(targets, dtype=np.uintp).tolist())
         rows = m.shape[0]
         cols = m.shape[1] if m.ndim == 2 else 1
         rc = _lib.apply_at(self._h, m.__array_interface__["data"][0], rows, cols, t, k, self._at)

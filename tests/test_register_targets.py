@@ -10,7 +10,7 @@ def calls(monkeypatch):
     got = []
 
     def apply(handle, matrix, rows, cols, targets, k, err):
-        got.append(list(targets))
+        got.append(np.frombuffer(targets, dtype=np.uintp, count=k).tolist())
         return 0
 
     monkeypatch.setattr(_lib, "apply_at", apply)
