@@ -717,7 +717,8 @@ __device__ __forceinline__ float2 collapse_value(float2 v, double d, double rinv
 
 // Complex64 collapse on the FP32 and integer pipes. 1/d = rh + rl to 48 bits, so p = x rh rounded, its
 // remainder x rh - p (exact) plus x rl, and p plus that sum is x / d within 2^-46 before its one rounding
-// to a float: the value of the FP64 product. That holds for 2^-100 <= |p| < inf (below, the remainder
+// to a float: the value of the FP64 product, but where x / d lies that near to the middle of two floats (1 in 2^21).
+// That holds for 2^-100 <= |p| < inf (below, the remainder
 // would not be exact) and reciprocals that the host found within 2^+-60; a chunk with any other
 // component but 0 takes the FP64 form of collapse_value. src(t) and dst(t) are the kept amplitude's places,
 // drop(t) clears the other one, one(t) is the next target's bit. 30 qubits, all 30 collapses: 16.5 ms with five
