@@ -26,6 +26,7 @@
 #include "qs_device.cuh"
 #include "qs_pass.cuh"
 #include "qs_reduce.cuh"
+#include "qs_rot.cuh"
 #include "qs_sweep.h"
 
 namespace qs {
@@ -144,9 +145,6 @@ struct Sw<float2> {
     using Coef = float2;
     using Phase = float2;
     static __device__ __forceinline__ Coef coef(const SweepCoef& c) { return make_float2(float(c.c), float(c.s)); }
-    static __device__ __forceinline__ Phase phase(const FxC& v) {
-        return make_float2(__ll2float_rn(v.x) * 0x1p-60f, __ll2float_rn(v.y) * 0x1p-60f);
-    }
     static __device__ __forceinline__ uint32_t at(uint32_t x) { return x ^ ((x >> 4) & 7u) ^ ((x >> 3) & 8u); }
     static __device__ __forceinline__ Acc zero() { return Acc(); }
     static __device__ __forceinline__ Acc add(Acc a, Acc b) {
@@ -705,8 +703,9 @@ __device__ __noinline__ void sw_fixed(T* s, const TileOp& op, uint32_t tsize, in
 // The factor tables of a program: entry i of the low part is the product of the phases of tile bits
 // 0..4 at i, entry j of the high part that of the bits from 5 on; sigma goes into the first table.
 // RZ(theta) multiplies bit 0 by c - i s and bit 1 by c + i s; the inverse the other way. Formed in fixed
-// point except for double2 tiles: an entry's error is common to every amplitude that it multiplies, and
-// FP64 products (2^-53 each) left three times the error on a gradient, in ten times the time.
+// point for fixed-point tiles: an entry's error is common to every amplitude that it multiplies, and
+// FP64 products (2^-53 each) left three times the error on a gradient, in ten times the time. Complex64 tables
+// are formed in float pairs, right to 2^-44 of each part however small it is, and rounded to floats once.
 template <typename T>
 __device__ __forceinline__ void sw_tables(typename Sw<T>::Phase* tables, const SweepPass* passes, int npass, int tq,
                                           bool rev, const SweepCoef* __restrict__ coef, double sigma, int nthreads) {
@@ -731,6 +730,22 @@ __device__ __forceinline__ void sw_tables(typename Sw<T>::Phase* tables, const S
                     re = r;
                 }
                 out = make_double2(re, im);
+            } else if constexpr (sizeof(T) == 8) {
+                float rh = 1.0f, rl = 0.0f, ih = 0.0f, il = 0.0f;
+                if (start != 1.0) df_split(start, rh, rl);
+                for (int b = lo; b < hi; b++) {
+                    if (P.zrot[b] < 0) continue;
+                    const SweepCoef& c = coef[P.zrot[b]];
+                    const bool plus = ((i >> (b - lo) & 1) != 0) != rev;
+                    const float ch = __int_as_float(c.ph), cl = __int_as_float(c.pl);
+                    float sh = __int_as_float(c.sh), sl = __int_as_float(c.sl);
+                    if (!plus) sh = -sh, sl = -sl;
+                    float th, tl;
+                    df_lin2(ch, cl, rh, rl, -sh, -sl, ih, il, th, tl);
+                    df_lin2(ch, cl, ih, il, sh, sl, rh, rl, ih, il);
+                    rh = th, rl = tl;
+                }
+                out = make_float2(__fadd_rn(rh, rl), __fadd_rn(ih, il));
             } else {
                 FxC v{start == 1.0 ? 1ll << 60 : __double2ll_rn(start * kFxOne), 0};
                 for (int b = lo; b < hi; b++) {
@@ -951,6 +966,13 @@ static __global__ void __launch_bounds__(64) k_sweep_coefs(const SweepRange* __r
             const FxLimb lc = fx_limb(__double2ll_rn(cs.x * kFxOne)), ls = fx_limb(__double2ll_rn(cs.y * kFxOne));
             o.ph = lc.h, o.pl = lc.l;
             o.sh = ls.h, o.sl = ls.l;
+            if (R.single) {
+                float h, l;
+                df_split(cs.x, h, l);
+                o.ph = __float_as_int(h), o.pl = __float_as_int(l);
+                df_split(cs.y, h, l);
+                o.sh = __float_as_int(h), o.sl = __float_as_int(l);
+            }
         }
         coefs[R.coef0 + r] = o;
         weights[R.coef0 + r] = 1.0;

@@ -83,7 +83,7 @@ inline bool sweep_fixed_point(int arith, bool unitary) { return unitary && arith
 //   floating tiles, RX and RY: the pair update without its common factor f (a' = a + t b and so on: two
 //     multiply-adds per real pair instead of four operations) in the form with |t| <= 1: c = t = tan
 //     (f = cos), s = 0; or behind an exchange of the pair c = t = -cot (f = sin), s = 1
-//   RZ: c = cos, s = sin of theta / 2, and the same as 2^60 ths in limbs
+//   RZ: c = cos, s = sin of theta / 2, and the same as 2^60 ths in limbs (complex64: as float pairs)
 //   fixed-point tiles, RX and RY: theta / 2 = a + k pi / 2 with |a| <= pi / 4, the rotation by a as three
 //     shears with tan(a / 2) and sin(a), as 2^60 ths in limbs; `quarter` for odd k
 struct alignas(16) SweepCoef {
