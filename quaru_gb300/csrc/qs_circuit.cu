@@ -125,10 +125,12 @@ static int run_blocks(void* state, int n, int prec, int arith, const qs_gate* ga
     std::vector<float> frags;
     std::vector<double> mats;
     for (FusedBlock& b : blocks) {
-        if (live && !all_finite(b.u, prec)) *live = LiveSpace{};
+        const bool finite = all_finite(b.u, prec);
+        if (live && !finite) *live = LiveSpace{};
         std::vector<size_t> tq(b.qubits.begin(), b.qubits.end());
         OpDesc op;
-        if (tensor && int(b.qubits.size()) <= 5) {
+        // digits of an infinity or NaN are digits of nothing: such a block is a dense sweep of its own
+        if (tensor && int(b.qubits.size()) <= 5 && (finite || !oz)) {
             pad_block(&b, 5, n);
             op.kind = OP_BLOCK;
             op.k = 5;
