@@ -513,9 +513,10 @@ int qs_apply_circuit(qs_register* reg, const qs_gate* gates, size_t m, const qs_
     } else if (o.fuse == 3) {
         o.fuse = 1;  // tuning switched off: stages at the automatic tile size
     }
+    bool overflow = false;
     int rc = qs::run_circuit(reg->state, reg->n, reg->prec, reg->arith, ops, gates, o, reg->stream, reg->sms, &msg,
-                             nullptr, live_space(reg));
-    if (rc) reg->known = qs::LiveSpace{};  // part of it ran
+                             nullptr, live_space(reg), &overflow);
+    if (rc || overflow) forget(reg);  // part of it ran, or zeros became NaN
     return rc ? set_err(rc, msg) : QS_OK;
 }
 

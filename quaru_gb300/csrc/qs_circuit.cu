@@ -105,7 +105,8 @@ static bool all_finite(const std::vector<double>& m, int prec) {
 // or complex128 in fixed-point arithmetic, the blocks run on the tensor cores inside 12-qubit
 // tiles; otherwise each block is one dense gate sweep.
 static int run_blocks(void* state, int n, int prec, int arith, const qs_gate* gates, size_t m,
-                      const qs_circuit_options& opts, cudaStream_t s, int sms, std::string* msg, LiveSpace* live) {
+                      const qs_circuit_options& opts, cudaStream_t s, int sms, std::string* msg, LiveSpace* live,
+                      bool* overflow) {
     // Tensor-core blocks inside 12-qubit tiles: 3xTF32 on complex64 registers; on complex128
     // registers in fixed-point arithmetic, the FP64-accurate split-integer product (k_tile_oz).
     const bool oz = (prec == QS_PREC_C128) && arith == QS_ARITH_FX64 && n >= 12;
@@ -127,6 +128,7 @@ static int run_blocks(void* state, int n, int prec, int arith, const qs_gate* ga
     for (FusedBlock& b : blocks) {
         const bool finite = all_finite(b.u, prec);
         if (live && !finite) *live = LiveSpace{};
+        if (overflow && !finite) *overflow = true;
         std::vector<size_t> tq(b.qubits.begin(), b.qubits.end());
         OpDesc op;
         // digits of an infinity or NaN are digits of nothing: such a block is a dense sweep of its own
@@ -167,8 +169,9 @@ static int run_blocks(void* state, int n, int prec, int arith, const qs_gate* ga
 
 int run_circuit(void* state, int n, int prec, int arith, const std::vector<OpDesc>& ops, const qs_gate* gates,
                 const qs_circuit_options& opts, cudaStream_t s, int sms, std::string* msg, int* derr_dev,
-                LiveSpace* live) {
-    if (opts.fuse == 2 && gates) return run_blocks(state, n, prec, arith, gates, ops.size(), opts, s, sms, msg, live);
+                LiveSpace* live, bool* overflow) {
+    if (opts.fuse == 2 && gates)
+        return run_blocks(state, n, prec, arith, gates, ops.size(), opts, s, sms, msg, live, overflow);
     if (opts.fuse >= 1) {
         // Tile qubits: 32 KiB of shared memory per tile by default; below 19 (complex64) or 18
         // (complex128) qubits smaller tiles, so that up to 128 blocks share the state (complex64

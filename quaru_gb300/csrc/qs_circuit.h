@@ -17,10 +17,11 @@ int apply_op(void* state, int n, int prec, int arith, const OpDesc& op, cudaStre
 
 // Apply a classified gate list with the fusion strategy in `opts` (gates are
 // the same list, unclassified, for dense-block fusion). derr_dev: see run_tiled. live: see
-// apply_op.
+// apply_op. overflow (nullable): set when a fused block's matrix is not finite, though the gates' may be: zeros on
+// qubits that no gate acts on are then zeros no more.
 int run_circuit(void* state, int n, int prec, int arith, const std::vector<OpDesc>& ops, const qs_gate* gates,
                 const qs_circuit_options& opts, cudaStream_t s, int sms, std::string* msg, int* derr_dev = nullptr,
-                LiveSpace* live = nullptr);
+                LiveSpace* live = nullptr, bool* overflow = nullptr);
 
 // ---- fusion autotuner (qs_autotune.cpp) ----
 struct TuneChoice {

@@ -93,3 +93,27 @@ def test_collapse_onto_nothing(n, form, precision, arith, monkeypatch):
             s = g.state
             np.testing.assert_array_equal(np.isnan(s), np.isnan(want))
             np.testing.assert_array_equal(s[~np.isnan(s)], want[~np.isnan(want)])
+
+
+@pytest.mark.parametrize("arith", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", [6, 13, 16])
+def test_fused_blocks_that_overflow(n, arith):
+    """Finite gates whose fused block is not: it makes NaN of zeros, those of measured qubits too."""
+    import quaru_gb300 as q
+
+    ops = [q.Operation(np.array([[2.0, 1.0], [1.0, -2.0]], dtype=complex), [1]),
+           q.Operation(np.array([[0.5, 1.0], [1e308, 1e308]], dtype=complex), [3])]
+    a, b = q.Register.from_int(n, 0), q.Register.from_int(n, 0)
+    for r in (a, b):
+        r.set_arith(arith)
+    a.measure_sequence([n - 1, 2], [0.5, 0.5])
+    st = np.zeros(1 << n, dtype=complex)
+    st[0] = 1.0
+    b.state = st
+    for r in (a, b):
+        r.apply_gates(ops, fuse=2, max_width=4)
+    x, y = a.state, b.state
+    np.testing.assert_array_equal(np.isnan(x), np.isnan(y))
+    assert np.isnan(x).any()
+    assert not a.measure(3, 0.25) and not b.measure(3, 0.25)  # the half without NaN
+    np.testing.assert_array_equal(np.isnan(a.state), np.isnan(b.state))
