@@ -58,9 +58,9 @@ extern "C" {
 #define QS_ARITH_FX64 3  /* FP64-accurate fixed-point arithmetic on the integer pipes for dense
                             1-qubit gates: each output is an exact-to-2^-55 integer dot product
                             rounded once to double (error <= ulp/2 + 2^-55 max|u| max|x|, below that
-                            of a chain of FP64 FMAs, which QS_ARITH_FMA is on up to 16 qubits); fused dense blocks (qs_apply_circuit, fuse = 2,
-                            12 qubits and more) run as FP64-accurate split-integer products on the
-                            BF16 tensor cores; other gates and cache-blocked stages use FP64 FMA */
+                            of a chain of FP64 FMAs, which QS_ARITH_FMA is on up to 16 qubits);
+                            fused dense blocks (qs_apply_circuit, fuse = 2, 12 qubits and more)
+                            run as FP64-accurate split-integer products on the BF16 tensor cores; other gates and cache-blocked stages use FP64 FMA */
 
 typedef struct qs_register qs_register;
 

@@ -218,7 +218,8 @@ __global__ void __launch_bounds__(kThreads, MODE == 0 ? 4 : 5) k_dense1_im(doubl
 // as one integer and rounded once (the chain of FMAs rounds four times). The pair's four components go on the
 // scale of the largest, E: significands shifted left by 30 - (E - e), in limbs of 30 bits; a coefficient is two
 // limbs, exactly. Of the six limb products the lowest is dropped, which leaves an output within 2^-54 of its largest
-// product while components lie within 2^kDotSpread of the largest and coefficients are as fill_dot wants them. Other pairs (1 in 2^17 of a random state's) take the FMA chain.
+// product while components lie within 2^kDotSpread of the largest and coefficients are as fill_dot wants them. Other
+// pairs (1 in 2^17 of a random state's) take the FMA chain.
 // Bound: 220 ALU instructions and 80 wide multiply-adds per pair, in place of 12 FP64 instructions and 4
 // integer products (FP64: 64 cycles per warp instruction and sub-partition). 28 qubits, one gate on a
 // state without zeros: 3.07 ms before, 2.23 ms now; the state's traffic takes 1.26 ms.

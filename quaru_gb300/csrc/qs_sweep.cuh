@@ -602,7 +602,7 @@ __device__ __forceinline__ void sw_moves(T* sp, T* sl, uint32_t tsize, int tq, u
             if (slot >= 0) S::gather(sacc[slot * kSwWarps + warp], mine);
         }
         const uint32_t tmask = (1u << (tq < 5 ? tq : 5)) - 1u;
-        if (P.phase_first) {  // never in the reverse walk (without the branch its instances spill more: complex64 batches +1 %)
+        if (P.phase_first) {  // never in the reverse walk; without the branch there it spills more (complex64 batches +1 %)
 #pragma unroll
             for (int r = 0; r < N; r++) {
                 const uint32_t y = from(r);
