@@ -60,7 +60,8 @@ extern "C" {
                             rounded once to double (error <= ulp/2 + 2^-55 max|u| max|x|, below that
                             of a chain of FP64 FMAs, which QS_ARITH_FMA is on up to 16 qubits);
                             fused dense blocks (qs_apply_circuit, fuse = 2, 12 qubits and more)
-                            run as FP64-accurate split-integer products on the BF16 tensor cores; other gates and cache-blocked stages use FP64 FMA */
+                            run as FP64-accurate split-integer products on the BF16 tensor cores;
+                            other gates and cache-blocked stages use FP64 FMA */
 
 typedef struct qs_register qs_register;
 
